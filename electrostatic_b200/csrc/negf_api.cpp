@@ -139,7 +139,31 @@ struct DevBuf {
     }
 };
 
+// FP64 chains of a tube for its current energy paths, on the device: the energy
+// table and the codes (energy, mode) of the contour and pole chains, then of
+// the real-axis ones.  Made once per version of the tube's paths, shared by
+// every call and plan that uses that version and freed with the last of them.
+struct ChainSet {
+    std::vector<negf::EnergyRec> h_items;
+    std::vector<int> h_codes;
+    DevBuf items, codes;
+    int contour = 0, realaxis = 0;  // chains of each kind
+};
+
+// FP64 part of a launch (negf_sweep.cu): groups with K = kSweepSeg and with K = 2.
+struct SweepPart {
+    std::vector<std::shared_ptr<const ChainSet>> sets;
+    std::vector<negf::GroupDev> groups[2];
+    std::vector<int> pass_of[2];  // pass of each group
+    negf::SweepShape shape[2] = {};
+    long long ck_doubles = 0, cc_doubles = 0, tm_doubles = 0;
+    int chains = 0, warps = 0;  // chains, and warps of 32 of them
+    bool scan = false;
+    bool any() const { return !groups[0].empty() || !groups[1].empty(); }
+};
+
 struct ChainTable {
+    SweepPart fp64;  // empty when every chain is in `warps` (an explicit fused request)
     std::vector<negf::ChainRec> chains;
     std::vector<negf::WarpRec> warps;
     std::vector<negf::ReduceTube> rts;
@@ -177,6 +201,8 @@ struct negf_tube {
     std::vector<Pt> eq_pts, noneq_pts, rho0_pts;
     std::vector<cplx> poles;
     int version = 0;
+    std::shared_ptr<const ChainSet> set;  // FP64 chains of version set_version
+    int set_version = -1;
     long long serial = 0;  // unique per tube of the process (keys the cached launch tables)
     int shard_rank = 0, shard_world = 1;
     // adaptive non-equilibrium limits (NEGF_Common.H:453-457)
@@ -208,6 +234,9 @@ struct negf_charge_plan {
     std::vector<negf_tube*> tubes;
     std::vector<int> versions;
     DevBuf d_tubes, d_chains, d_warps, d_units, d_rts, d_partial, d_scratch, d_order, d_pieces;
+    DevBuf d_ck, d_cc, d_tm, d_groups;
+    SweepPart fp64;
+    negf::ReduceTube rt0{};  // the reduction record of a one-tube plan
     int num_warps = 0, num_units = 0, max_N = 0;
     int pieces = 1;  // pass-1 pieces of the two-pass schedule (parallel in length)
     int n64 = 0, n32 = 0;  // fused schedule: FP64 / FP32 warps in d_order
@@ -239,6 +268,7 @@ struct Workspace {
     int device = 0;
     cudaStream_t stream = nullptr;
     DevBuf tubes, chains, warps, rts, units, partial, scratch, qbuf, pieces, order;
+    DevBuf ck, cc, tm, groups;  // FP64 part: boundary states, chain constants, scan matrices, group table
     cudaStream_t side = nullptr;                 // the FP32 warps of the fused schedule
     cudaEvent_t fork = nullptr, join = nullptr;  // around them
     // real-space pass (negf_rs_compute_charge)
@@ -248,6 +278,7 @@ struct Workspace {
     std::vector<int> key_versions;
     ChainTable table;
     bool table_valid = false;
+    int key_pieces = 0, key_schedule = 0;  // settings the table was built with
     cudaEvent_t ev[4] = {nullptr, nullptr, nullptr, nullptr};  // timing of the last call
     cudaEvent_t done = nullptr;                                 // end of the last call's kernels
     bool used = false;
@@ -262,7 +293,7 @@ struct Workspace {
         if (join) cudaEventDestroy(join);
         if (side) cudaStreamDestroy(side);
         DevBuf* bufs[] = {&tubes, &chains, &warps, &rts,  &units, &partial,   &scratch, &qbuf,   &pieces,
-                          &order, &rsE,    &rsFlags, &rsU0, &rsUa, &rsCorners, &rsGL,    &rsGLn,  &rsRows,
+                          &ck,    &cc,   &tm,    &groups, &order, &rsE,    &rsFlags, &rsU0, &rsUa, &rsCorners, &rsGL,    &rsGLn,  &rsRows,
                           &rsStatus};
         for (DevBuf* b : bufs) {
             if (b->p) cudaFree(b->p);
@@ -621,7 +652,9 @@ bool near_lead_band_edge(const negf_tube& t, int m, cplx E, double band) {
 
 // Chains of one tube, grouped by (kind, precision) with each group padded
 // to whole warps (padding lanes: mode -1, zero coefficients).
-void build_tube_chains(Out<negf::ChainRec>& chains, Out<negf::WarpRec>& warps, TableCounts& cnt, const TubePass& tp) {
+// only32: the FP32 chains alone (the FP64 ones run as groups).
+void build_tube_chains(Out<negf::ChainRec>& chains, Out<negf::WarpRec>& warps, TableCounts& cnt, const TubePass& tp,
+                       bool only32) {
     const negf_tube& t = *tp.t;
     const int M = t.d.num_modes;
     const int total = pass_items(t, tp.rho0_pass);
@@ -631,7 +664,7 @@ void build_tube_chains(Out<negf::ChainRec>& chains, Out<negf::WarpRec>& warps, T
     const double band = t.d.mixed_fp64_band;
     for (int kind = 0; kind < 2; ++kind)
         for (int fp32 = 0; fp32 < 2; ++fp32) {
-            if (fp32 && !mixed) continue;
+            if (fp32 ? !mixed : only32) continue;
             const size_t first = chains.size();
             for (int idx = lo; idx < hi; ++idx) {
                 const Item it = pass_item(t, tp.rho0_pass, idx);
@@ -709,6 +742,16 @@ int auto_pieces(int nw, int max_N) {
     return nw >= target / 2 ? 1 : std::min(maxp, (target + nw - 1) / std::max(nw, 1));
 }
 
+// Boundary states of the FP64 chains by the scan over segments (parallel in
+// length) rather than by sweeps.  A sweep of few chains takes its N dependent
+// steps, 17 ns a site; the scan takes 3 us more to start and then works at 8.4
+// ps per site and chain (measured: 4000 sites and 512 chains 27 us against 73
+// us by sweeps, 4096 chains 138 us against 78 us, 400 sites and 228 chains 14
+// us against 17 us).
+bool scan_better(long long site_chains, int max_N) {
+    return 3.0 + 8.4e-6 * double(site_chains) < 0.017 * max_N;
+}
+
 int choose_schedule(int setting, int nw, int pieces) {
     if (pieces > 1) return negf::kScheduleTwoPass;
     if (setting == NEGF_SCHEDULE_FUSED) return negf::kScheduleFused;
@@ -731,14 +774,10 @@ long long checkpoint_traffic(const std::vector<negf::WarpRec>& warps, const std:
     return 2 * b;
 }
 
-// Launch tables of a set of tube passes.  Launch order: longest tubes first
-// (order[] is caller scratch of passes.size() ints); rts[i] describes pass i.
-void build_table_generic(const TubePass* passes, int num_passes, int* order, Out<negf::ChainRec>& chains,
-                         Out<negf::WarpRec>& warps, Out<negf::SegUnit>& units, negf::ReduceTube* rts,
-                         TableCounts& cnt, int segs_per_unit = negf::kSegsPerUnit) {
-    cnt = TableCounts();
+// Indices of the passes by descending N (stable).
+void longest_first(const TubePass* passes, int num_passes, int* order) {
     for (int i = 0; i < num_passes; ++i) order[i] = i;
-    for (int i = 1; i < num_passes; ++i) {  // stable insertion sort by descending N
+    for (int i = 1; i < num_passes; ++i) {
         const int v = order[i];
         int j = i - 1;
         while (j >= 0 && passes[order[j]].t->N < passes[v].t->N) {
@@ -747,18 +786,248 @@ void build_table_generic(const TubePass* passes, int num_passes, int* order, Out
         }
         order[j + 1] = v;
     }
+}
+
+// Device copy of an FP64 chain list on `stream`, finished on return (other
+// streams may use it next).  An unchanged list keeps the set it has.
+int upload_chain_set(std::vector<negf::EnergyRec>& items, std::vector<int> (&codes)[2], cudaStream_t stream,
+                     std::shared_ptr<const ChainSet>* set) {
+    std::shared_ptr<ChainSet> cs = std::make_shared<ChainSet>();
+    cs->contour = (int)codes[negf::kContour].size();
+    cs->realaxis = (int)codes[negf::kRealAxis].size();
+    cs->h_codes = std::move(codes[negf::kContour]);
+    cs->h_codes.insert(cs->h_codes.end(), codes[negf::kRealAxis].begin(), codes[negf::kRealAxis].end());
+    cs->h_items = std::move(items);
+    const size_t ib = cs->h_items.size() * sizeof(negf::EnergyRec), cb = cs->h_codes.size() * sizeof(int);
+    if (*set && (*set)->contour == cs->contour && (*set)->h_codes == cs->h_codes &&
+        (*set)->h_items.size() == cs->h_items.size() &&
+        (ib == 0 || std::memcmp((*set)->h_items.data(), cs->h_items.data(), ib) == 0))
+        return NEGF_OK;
+    if (cb) {
+        // another thread may be capturing a graph: these allocations are not part of it
+        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+        NEGF_CUDA(cudaThreadExchangeStreamCaptureMode(&mode));
+        cudaError_t e = cs->items.reserve(ib);
+        if (e == cudaSuccess) e = cs->codes.reserve(cb);
+        if (e == cudaSuccess) e = cudaMemcpyAsync(cs->items.p, cs->h_items.data(), ib, cudaMemcpyHostToDevice, stream);
+        if (e == cudaSuccess) e = cudaMemcpyAsync(cs->codes.p, cs->h_codes.data(), cb, cudaMemcpyHostToDevice, stream);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
+        cudaThreadExchangeStreamCaptureMode(&mode);
+        NEGF_CUDA(e);
+    }
+    *set = std::move(cs);
+    return NEGF_OK;
+}
+
+// FP64 chains of one pass of a tube (see ChainSet); fp64_all: every chain,
+// whatever the tube's precision mode.
+int make_chain_set(const negf_tube& t, bool rho0_pass, bool fp64_all, cudaStream_t stream,
+                   std::shared_ptr<const ChainSet>* set) {
+    const int M = t.d.num_modes, total = pass_items(t, rho0_pass);
+    int lo = 0, hi = total;
+    if (!rho0_pass) negf_shard_range(total, t.shard_rank, t.shard_world, &lo, &hi);
+    const bool mixed = t.d.precision == NEGF_PREC_MIXED && !rho0_pass && !fp64_all;
+    const double band = t.d.mixed_fp64_band;
+    std::vector<negf::EnergyRec> items;
+    std::vector<int> codes[2];
+    items.reserve(hi - lo);
+    for (int idx = lo; idx < hi; ++idx) {
+        const Item it = pass_item(t, rho0_pass, idx);
+        const bool kind_ok = it.kind == negf::kContour || t.d.mixed_realaxis_fp32;
+        const bool axis_ok = mixed && kind_ok && std::fabs(it.E.imag()) >= band;
+        bool used = false;
+        for (int m = 0; m < M; ++m) {
+            // the complement of the FP32 rule of build_tube_chains
+            if (axis_ok && !(it.kind == negf::kRealAxis && near_lead_band_edge(t, m, it.E, band))) continue;
+            codes[it.kind].push_back((int)items.size() << negf::kModeBits | m);
+            used = true;
+        }
+        if (used) items.push_back({it.E.real(), it.E.imag(), it.c.real(), it.c.imag(), it.b0, it.b1});
+    }
+    if (items.size() >= (size_t(1) << (31 - negf::kModeBits))) return fail(NEGF_ERR_ARG, "too many energy points");
+    return upload_chain_set(items, codes, stream, set);
+}
+
+// Whether the FP64 chains of a batch run as groups (negf_sweep.cu) beside the
+// FP32 ones.  Not on an explicit fused request, and not when most of the work
+// is FP32: the few FP64 chains left (near the axis or a band edge) then ride
+// along in the launches of the FP32 warps (a 16-tube batch with the real axis
+// in FP32: 2.364 ms so, 2.382 ms with groups; a small mixed tube 44 us against
+// 47 us).  Counted by energies; the band-edge rule moves single chains only.
+bool use_groups(negf_tube* const* tubes, int num_tubes, bool fp64_all) {
+    if (settings().schedule == NEGF_SCHEDULE_FUSED) return false;
+    long long all = 0, low = 0;
+    for (int i = 0; i < num_tubes; ++i) {
+        const negf_tube& t = *tubes[i];
+        const long long w = (long long)t.N * t.d.num_modes;
+        all += w * (long long)(t.eq_pts.size() + t.poles.size() + t.noneq_pts.size());
+        if (t.d.precision != NEGF_PREC_MIXED || fp64_all) continue;
+        const double band = t.d.mixed_fp64_band;
+        for (const Pt& p : t.eq_pts) low += std::fabs(p.E.imag()) >= band ? w : 0;
+        for (const cplx& p : t.poles) low += std::fabs(p.imag()) >= band ? w : 0;
+        if (t.d.mixed_realaxis_fp32)
+            for (const Pt& p : t.noneq_pts) low += std::fabs(p.E.imag()) >= band ? w : 0;
+    }
+    return 2 * low <= all;
+}
+
+// The tube's FP64 chains for the current paths, made on first use of a version.
+int chain_set(negf_tube& t, cudaStream_t stream, std::shared_ptr<const ChainSet>* out) {
+    if (!t.set || t.set_version != t.version) {
+        if (int rc = make_chain_set(t, false, false, stream, &t.set)) return rc;
+        t.set_version = t.version;
+    }
+    *out = t.set;
+    return NEGF_OK;
+}
+
+// One group's constant fields and its place in the launch.
+negf::GroupDev make_group(const negf::TubeDev& d, const ChainSet& cs, int kind, int K) {
+    negf::GroupDev g{};
+    g.U = d.U;
+    g.items = cs.items.as<negf::EnergyRec>();
+    g.chains = cs.codes.as<int>() + (kind == negf::kRealAxis ? cs.contour : 0);
+    g.N = d.N;
+    g.nseg = (d.N + K - 1) / K;
+    g.nblk = (g.nseg + 7) / 8;
+    g.kind = kind;
+    g.nch = kind == negf::kRealAxis ? cs.realaxis : cs.contour;
+    g.use_decimation = d.use_decimation;
+    g.dec_iters = d.dec_iters;
+    g.dec_layers = d.dec_layers;
+    g.uc_from_U = d.uc_from_U;
+    g.gamma = d.gamma;
+    g.Uc0 = d.Uc0;
+    g.Uc1 = d.Uc1;
+    g.lanes = 1;
+    while (g.lanes < 32 && g.lanes < g.nseg) g.lanes *= 2;
+    g.nsb = (g.nseg + g.lanes - 1) / g.lanes;
+    std::copy(d.beta, d.beta + negf::kMaxModes, g.beta);
+    std::copy(d.degen, d.degen + negf::kMaxModes, g.degen);
+    return g;
+}
+
+// Groups of the FP64 chains of a launch, longest tubes first.  pieces: the
+// setting (0 automatic, 1 sweeps, more: parallel in length).
+void plan_groups(SweepPart& sp, const TubePass* passes, const negf::TubeDev* tdev, int num_passes, int pieces) {
+    std::vector<int> order(num_passes);
+    longest_first(passes, num_passes, order.data());
+    long long work = 0, site_chains = 0;  // chain x segment-block iterations of seg_kernel
+    int max_N = 0;
+    for (int o : order) {
+        const ChainSet& cs = *sp.sets[o];
+        const int k = tdev[o].N < negf::kSweepSeg ? 1 : 0;
+        for (int kind : {negf::kRealAxis, negf::kContour}) {
+            if ((kind == negf::kRealAxis ? cs.realaxis : cs.contour) == 0) continue;
+            sp.groups[k].push_back(make_group(tdev[o], cs, kind, k ? 2 : negf::kSweepSeg));
+            sp.pass_of[k].push_back(o);
+            const negf::GroupDev& g = sp.groups[k].back();
+            const int cpw = 32 / g.lanes;
+            work += (long long)g.nsb * ((g.nch + cpw - 1) / cpw);
+            sp.chains += g.nch;
+            site_chains += (long long)g.nch * g.N;
+            sp.warps += (g.nch + 31) / 32;
+            max_N = std::max(max_N, g.N);
+        }
+    }
+    sp.scan = pieces > 1 || (pieces == 0 && scan_better(site_chains, max_N));
+    // Units of seg_kernel: whole waves of the 11 warps an SM holds, of at most
+    // 32 chain iterations each (a unit costs about 3 us to start and 0.6 us
+    // per iteration; fewer and longer units also mean fewer partial rows).
+    const long long slots = 11LL * device_sm_count();
+    const long long waves = std::max(1LL, (work + 32 * slots - 1) / (32 * slots));
+    const int iters = (int)std::max(1LL, (work + waves * slots - 1) / (waves * slots));
+    for (int k = 0; k < 2; ++k) {
+        negf::SweepShape& sh = sp.shape[k];
+        sh.K = k ? 2 : negf::kSweepSeg;
+        sh.scan = sp.scan;
+        int max_nseg = 1;
+        for (negf::GroupDev& g : sp.groups[k]) {
+            g.chains_per_unit = iters * (32 / g.lanes);
+            g.sweep_base = sh.sweep_blocks;
+            g.chain_base = sh.chains;
+            g.seg_base = sh.seg_blocks;
+            sh.sweep_blocks += 2 * ((g.nch + 31) / 32);
+            sh.chains += g.nch;
+            sh.seg_blocks += g.nsb * ((g.nch + g.chains_per_unit - 1) / g.chains_per_unit);
+            const int comps = g.kind == negf::kRealAxis ? 6 : 4;
+            g.ck_off = sp.ck_doubles;
+            sp.ck_doubles += (long long)((g.nch + 31) / 32) * g.nblk * comps * 256;
+            g.cc_off = sp.cc_doubles;
+            sp.cc_doubles += (long long)g.nch * negf::kConst;
+            max_nseg = std::max(max_nseg, g.nseg);
+        }
+        sh.scan_threads = std::min(512, (max_nseg + 31) / 32 * 32);
+        const bool keep = max_nseg > sh.scan_threads;  // more segments than threads: their matrices go to scratch
+        for (negf::GroupDev& g : sp.groups[k]) g.tm_segs = keep ? max_nseg : 0;
+        if (sp.scan && keep) sp.tm_doubles = std::max(sp.tm_doubles, 9LL * sh.chains * max_nseg);
+    }
+}
+
+// Partial rows of pass `pass`'s groups from row (in doubles) on; returns their number.
+int place_rows(SweepPart& sp, int pass, int N, long long& row, TableCounts& cnt) {
+    int rows = 0;
+    for (int k = 0; k < 2; ++k)
+        for (size_t i = 0; i < sp.groups[k].size(); ++i) {
+            if (sp.pass_of[k][i] != pass) continue;
+            negf::GroupDev& g = sp.groups[k][i];
+            g.row_base = row;
+            const int n = (g.nch + g.chains_per_unit - 1) / g.chains_per_unit;
+            rows += n;
+            row += (long long)n * N;
+            cnt.updates += (long long)g.nch * N;
+            (g.kind == negf::kRealAxis ? cnt.realaxis_updates : cnt.contour_updates) += (long long)g.nch * N;
+        }
+    return rows;
+}
+
+// Pieces a chain runs in: its segments when parallel in length, else one sweep.
+int reported_pieces(const SweepPart& sp) {
+    int n = 1;
+    if (sp.scan)
+        for (const std::vector<negf::GroupDev>& v : sp.groups)
+            for (const negf::GroupDev& g : v) n = std::max(n, g.nseg);
+    return n;
+}
+
+// The kernels' argument for the groups of one segment length: up to two in the
+// parameters, more from `dev` (their device copy).
+negf::GroupSet group_set(const std::vector<negf::GroupDev>& v, const negf::GroupDev* dev) {
+    negf::GroupSet gs{};
+    gs.ng = (int)v.size();
+    for (int i = 0; i < std::min(gs.ng, negf::kMaxBases); ++i) {
+        gs.sweep_base[i] = v[i].sweep_base;
+        gs.chain_base[i] = v[i].chain_base;
+        gs.seg_base[i] = v[i].seg_base;
+    }
+    if (gs.ng > 2)
+        gs.ext = dev;
+    else
+        for (int i = 0; i < gs.ng; ++i) gs.g[i] = v[i];
+    return gs;
+}
+
+// Launch tables of a set of tube passes.  Launch order: longest tubes first
+// (order[] is caller scratch of passes.size() ints); rts[i] describes pass i.
+void build_table_generic(const TubePass* passes, int num_passes, int* order, Out<negf::ChainRec>& chains,
+                         Out<negf::WarpRec>& warps, Out<negf::SegUnit>& units, negf::ReduceTube* rts,
+                         TableCounts& cnt, int segs_per_unit = negf::kSegsPerUnit, SweepPart* fp64 = nullptr) {
+    cnt = TableCounts();
+    longest_first(passes, num_passes, order);
     long long row = 0, ck = 0;
     for (int k = 0; k < num_passes; ++k) {
         const int oi = order[k];
         const TubePass& tp = passes[oi];
         const size_t w0 = warps.size();
-        build_tube_chains(chains, warps, cnt, tp);
+        build_tube_chains(chains, warps, cnt, tp, fp64 != nullptr);
         const int N = tp.t->N;
         negf::ReduceTube rt{};
         rt.row_base = row;
+        int rows64 = 0;
+        if (fp64) rows64 = place_rows(*fp64, oi, N, row, cnt);
         rt.q_off = tp.q_off;
         rt.N = N;
-        rt.num_rows = int(warps.size() - w0);
+        rt.num_rows = rows64 + int(warps.size() - w0);
         rt.rho0 = (!tp.rho0_pass && tp.t->shard_rank == 0) ? tp.t->d_rho0 : nullptr;
         const int nseg = (N + negf::kSeg - 1) / negf::kSeg;
         for (size_t w = w0; w < warps.size() && !warps.overflow; ++w) {
@@ -787,8 +1056,18 @@ void fused_order(ChainTable& ct) {
     ct.n64 = (int)ct.warps.size() - ct.n32;
 }
 
-void build_table(ChainTable& ct, const std::vector<TubePass>& passes) {
+// Launch table of a set of passes.  sets: the FP64 chains of each pass, which
+// then run as groups (negf_sweep.cu) and only the FP32 chains fill the warp
+// tables; empty: every chain in the warp tables.
+void build_table(ChainTable& ct, const std::vector<TubePass>& passes, const std::vector<negf::TubeDev>& tdev,
+                 std::vector<std::shared_ptr<const ChainSet>> sets, int pieces,
+                 int segs_per_unit = negf::kSegsPerUnit) {
     ct = ChainTable();
+    const bool split = !sets.empty();
+    if (split) {
+        ct.fp64.sets = std::move(sets);
+        plan_groups(ct.fp64, passes.data(), tdev.data(), (int)passes.size(), pieces);
+    }
     Out<negf::ChainRec> oc;
     oc.vec = &ct.chains;
     Out<negf::WarpRec> ow;
@@ -798,7 +1077,8 @@ void build_table(ChainTable& ct, const std::vector<TubePass>& passes) {
     ct.rts.resize(passes.size());
     std::vector<int> order(passes.size());
     TableCounts cnt;
-    build_table_generic(passes.data(), (int)passes.size(), order.data(), oc, ow, ou, ct.rts.data(), cnt);
+    build_table_generic(passes.data(), (int)passes.size(), order.data(), oc, ow, ou, ct.rts.data(), cnt, segs_per_unit,
+                        split ? &ct.fp64 : nullptr);
     ct.updates = cnt.updates;
     ct.updates_fp32 = cnt.updates_fp32;
     ct.contour_updates = cnt.contour_updates;
@@ -809,18 +1089,70 @@ void build_table(ChainTable& ct, const std::vector<TubePass>& passes) {
     fused_order(ct);
 }
 
+// Device copies of the groups that do not fit the kernels' parameters: K =
+// kSweepSeg first, then K = 2.
+int upload_groups(const SweepPart& sp, DevBuf& buf, cudaStream_t stream) {
+    const size_t n0 = sp.groups[0].size(), n1 = sp.groups[1].size();
+    if (n0 <= 2 && n1 <= 2) return NEGF_OK;
+    NEGF_CUDA(buf.reserve((n0 + n1) * sizeof(negf::GroupDev)));
+    for (int k = 0; k < 2; ++k)
+        if (sp.groups[k].size() > 2)
+            NEGF_CUDA(cudaMemcpyAsync(buf.as<negf::GroupDev>() + (k ? n0 : 0), sp.groups[k].data(),
+                                      sp.groups[k].size() * sizeof(negf::GroupDev), cudaMemcpyHostToDevice, stream));
+    return NEGF_OK;
+}
+
+cudaError_t launch_fp64(const SweepPart& sp, const DevBuf& groups, const DevBuf& ck, const DevBuf& cc, const DevBuf& tm,
+                        double* d_partial, const int* skip, cudaStream_t stream, cudaEvent_t mid) {
+    for (int k = 0; k < 2; ++k) {
+        const negf::GroupDev* dev = groups.as<negf::GroupDev>();
+        const cudaError_t e =
+            negf::launch_sweep(group_set(sp.groups[k], dev ? dev + (k ? sp.groups[0].size() : 0) : nullptr), sp.shape[k],
+                               ck.as<double>(), cc.as<double>(), tm.as<double>(), d_partial, skip, stream, mid);
+        if (e != cudaSuccess) return e;
+    }
+    return cudaSuccess;
+}
+
+// The two precisions of a launch side by side: the FP32 warps on `side`
+// between the events fork and join, the FP64 groups on `stream`.  run32
+// launches the FP32 warps on the stream it is given.
+template <class F64, class F32>
+cudaError_t launch_split(bool any64, bool any32, cudaStream_t stream, cudaStream_t side, cudaEvent_t fork,
+                         cudaEvent_t join, F64&& run64, F32&& run32) {
+    cudaError_t e = cudaSuccess;
+    const bool both = any64 && any32;
+    if (both) {
+        e = cudaEventRecord(fork, stream);
+        if (e == cudaSuccess) e = cudaStreamWaitEvent(side, fork, 0);
+    }
+    if (e == cudaSuccess && any64) e = run64();
+    if (e == cudaSuccess && any32) e = run32(both ? side : stream);
+    if (both) {
+        // the side stream joins also after a failed launch, so that a capture ends whole
+        cudaError_t j = cudaEventRecord(join, side);
+        if (j == cudaSuccess) j = cudaStreamWaitEvent(stream, join, 0);
+        if (e == cudaSuccess) e = j;
+    }
+    return e;
+}
+
 int upload_and_launch(Workspace& W, const std::vector<TubePass>& passes, const std::vector<negf::TubeDev>& tdev,
-                      bool rebuild, double* d_Q, cudaStream_t stream) {
+                      const std::vector<std::shared_ptr<const ChainSet>>& sets, bool rebuild, double* d_Q,
+                      cudaStream_t stream) {
     Settings& G = settings();
     ChainTable& ct = W.table;
     if (rebuild) {
-        build_table(ct, passes);
+        build_table(ct, passes, tdev, sets, G.pass1_pieces);
         NEGF_CUDA(W.chains.reserve(std::max<size_t>(1, ct.chains.size()) * sizeof(negf::ChainRec)));
         NEGF_CUDA(W.warps.reserve(std::max<size_t>(1, ct.warps.size()) * sizeof(negf::WarpRec)));
         NEGF_CUDA(W.rts.reserve(std::max<size_t>(1, ct.rts.size()) * sizeof(negf::ReduceTube)));
         NEGF_CUDA(W.units.reserve(std::max<size_t>(1, ct.units.size()) * sizeof(negf::SegUnit)));
         NEGF_CUDA(W.partial.reserve(std::max<long long>(1, ct.partial_doubles) * sizeof(double)));
         NEGF_CUDA(W.scratch.reserve(std::max<long long>(1, ct.scratch_doubles) * sizeof(double)));
+        NEGF_CUDA(W.ck.reserve(std::max<long long>(1, ct.fp64.ck_doubles) * sizeof(double)));
+        NEGF_CUDA(W.cc.reserve(std::max<long long>(1, ct.fp64.cc_doubles) * sizeof(double)));
+        NEGF_CUDA(W.tm.reserve(std::max<long long>(1, ct.fp64.tm_doubles) * sizeof(double)));
         if (!ct.chains.empty())
             NEGF_CUDA(cudaMemcpyAsync(W.chains.p, ct.chains.data(), ct.chains.size() * sizeof(negf::ChainRec),
                                       cudaMemcpyHostToDevice, stream));
@@ -838,12 +1170,29 @@ int upload_and_launch(Workspace& W, const std::vector<TubePass>& passes, const s
     // the reduce table carries device pointers that can change (rho0 of a rebuilt tube)
     for (size_t i = 0; i < passes.size(); ++i)
         ct.rts[i].rho0 = (!passes[i].rho0_pass && passes[i].t->shard_rank == 0) ? passes[i].t->d_rho0 : nullptr;
-    NEGF_CUDA(cudaMemcpyAsync(W.rts.p, ct.rts.data(), ct.rts.size() * sizeof(negf::ReduceTube), cudaMemcpyHostToDevice,
-                              stream));
-    NEGF_CUDA(W.tubes.reserve(tdev.size() * sizeof(negf::TubeDev)));
-    NEGF_CUDA(cudaMemcpyAsync(W.tubes.p, tdev.data(), tdev.size() * sizeof(negf::TubeDev), cudaMemcpyHostToDevice,
-                              stream));
-    const int nw = (int)ct.warps.size();
+    negf::ReduceSet rs{};
+    if (passes.size() == 1) {
+        rs.one = ct.rts[0];
+    } else {
+        rs.ext = W.rts.as<negf::ReduceTube>();
+        NEGF_CUDA(cudaMemcpyAsync(W.rts.p, ct.rts.data(), ct.rts.size() * sizeof(negf::ReduceTube),
+                                  cudaMemcpyHostToDevice, stream));
+    }
+    const int nw = (int)ct.warps.size(), nw_all = nw + ct.fp64.warps;
+    if (nw > 0) {
+        NEGF_CUDA(W.tubes.reserve(tdev.size() * sizeof(negf::TubeDev)));
+        NEGF_CUDA(cudaMemcpyAsync(W.tubes.p, tdev.data(), tdev.size() * sizeof(negf::TubeDev), cudaMemcpyHostToDevice,
+                                  stream));
+    }
+    // potentials and contacts of this call
+    for (int k = 0; k < 2; ++k)
+        for (size_t i = 0; i < ct.fp64.groups[k].size(); ++i) {
+            const negf::TubeDev& d = tdev[ct.fp64.pass_of[k][i]];
+            ct.fp64.groups[k][i].U = d.U;
+            ct.fp64.groups[k][i].Uc0 = d.Uc0;
+            ct.fp64.groups[k][i].Uc1 = d.Uc1;
+        }
+    if (int rc = upload_groups(ct.fp64, W.groups, stream)) return rc;
     if (G.timing) {
         for (auto& e : W.ev)
             if (!e) NEGF_CUDA(cudaEventCreate(&e));
@@ -851,19 +1200,31 @@ int upload_and_launch(Workspace& W, const std::vector<TubePass>& passes, const s
     }
     int pieces = G.pass1_pieces;
     if (pieces == 0 && G.schedule == NEGF_SCHEDULE_FUSED) pieces = 1;  // an explicit fused request wins
-    if (pieces == 0) pieces = auto_pieces(nw, ct.max_N);
+    if (pieces == 0) pieces = auto_pieces(nw_all, ct.max_N);
     pieces = std::max(1, pieces);
-    const int schedule = choose_schedule(G.schedule, nw, pieces);
+    // schedule of the warp tables (the FP32 chains, or every chain of an explicit fused request)
+    const int schedule = nw > 0 ? choose_schedule(G.schedule, nw_all, pieces) : negf::kScheduleTwoPass;
     if (schedule == negf::kScheduleFused) pieces = 1;
-    if (pieces > 1) NEGF_CUDA(W.pieces.reserve(sizeof(double) * (size_t)nw * pieces * 24 * negf::kWarp));
-    const negf::FusedOrder fo{W.order.as<int>(), ct.n64, ct.n32, W.side, W.fork, W.join};
-    NEGF_CUDA(negf::launch_rgf(W.tubes.as<negf::TubeDev>(), W.chains.as<negf::ChainRec>(), W.warps.as<negf::WarpRec>(),
-                               nw, W.units.as<negf::SegUnit>(), (int)ct.units.size(), W.partial.as<double>(),
-                               W.scratch.p, G.warps_per_block, stream, G.timing ? W.ev[3] : nullptr, nullptr, pieces,
-                               W.pieces.as<double>(), schedule, &fo));
+    if (nw > 0 && pieces > 1) NEGF_CUDA(W.pieces.reserve(sizeof(double) * (size_t)nw * pieces * 24 * negf::kWarp));
+    const bool any64 = ct.fp64.any();
+    if (G.timing && !any64) NEGF_CUDA(cudaEventRecord(W.ev[3], stream));
+    NEGF_CUDA(launch_split(
+        any64, nw > 0, stream, W.side, W.fork, W.join,
+        [&] {
+            return launch_fp64(ct.fp64, W.groups, W.ck, W.cc, W.tm, W.partial.as<double>(), nullptr, stream,
+                               G.timing ? W.ev[3] : nullptr);
+        },
+        [&](cudaStream_t s32) {
+            // the launch forks by itself when both precisions are in the warp tables
+            const negf::FusedOrder fo{W.order.as<int>(), ct.n64, ct.n32, W.side, W.fork, W.join};
+            return negf::launch_rgf(W.tubes.as<negf::TubeDev>(), W.chains.as<negf::ChainRec>(),
+                                    W.warps.as<negf::WarpRec>(), nw, W.units.as<negf::SegUnit>(), (int)ct.units.size(),
+                                    W.partial.as<double>(), W.scratch.p, G.warps_per_block, s32,
+                                    G.timing && !any64 ? W.ev[3] : nullptr, nullptr, pieces, W.pieces.as<double>(),
+                                    schedule, &fo);
+        }));
     if (G.timing) NEGF_CUDA(cudaEventRecord(W.ev[1], stream));
-    NEGF_CUDA(negf::launch_reduce(W.rts.as<negf::ReduceTube>(), (int)ct.rts.size(), ct.max_N, W.partial.as<double>(),
-                                  d_Q, stream));
+    NEGF_CUDA(negf::launch_reduce(rs, (int)ct.rts.size(), ct.max_N, W.partial.as<double>(), d_Q, stream));
     if (G.timing) NEGF_CUDA(cudaEventRecord(W.ev[2], stream));
     NEGF_CUDA(cudaEventRecord(W.done, stream));
     W.used = true;
@@ -873,15 +1234,17 @@ int upload_and_launch(Workspace& W, const std::vector<TubePass>& passes, const s
     st.updates_fp32 = ct.updates_fp32;
     st.contour_updates = ct.contour_updates;
     st.realaxis_updates = ct.realaxis_updates;
-    st.chains = (int)ct.chains.size();
-    st.warps = nw;
+    st.chains = (int)ct.chains.size() + 32 * ct.fp64.warps;
+    st.warps = nw_all;
     const bool fused = schedule == negf::kScheduleFused;
     const int fused_kernels = (ct.n64 > 0 ? 1 : 0) + (ct.n32 > 0 ? 1 : 0);
     st.kernel_launches =
         (nw > 0 ? (fused ? fused_kernels : pieces > 1 ? 4 : 2) : 0) + (ct.max_N > 0 && !ct.rts.empty() ? 1 : 0);
-    st.pieces = pieces;
-    st.units = fused ? 0 : (int)ct.units.size();
-    st.checkpoint_bytes = checkpoint_traffic(ct.warps, tdev, ct.scratch_doubles, schedule);
+    for (int k = 0; k < 2; ++k) st.kernel_launches += ct.fp64.groups[k].empty() ? 0 : 2;
+    st.pieces = G.pass1_pieces > 0 || nw > 0 ? pieces : reported_pieces(ct.fp64);
+    st.units = (fused ? 0 : (int)ct.units.size()) + ct.fp64.shape[0].seg_blocks + ct.fp64.shape[1].seg_blocks;
+    st.checkpoint_bytes = (nw > 0 ? checkpoint_traffic(ct.warps, tdev, ct.scratch_doubles, schedule) : 0) +
+                          2 * 8 * ct.fp64.ck_doubles;
     st.schedule = fused ? NEGF_SCHEDULE_FUSED : NEGF_SCHEDULE_TWO_PASS;
     G.stats_ws = G.timing ? &W : nullptr;
     return NEGF_OK;
@@ -919,8 +1282,10 @@ int compute_rho0(negf_tube* t) {
     rho0_paths(*t);
     std::vector<TubePass> passes{{t, 0, 0, true}};
     std::vector<negf::TubeDev> tdev{make_tubedev(*t, true)};
+    std::vector<std::shared_ptr<const ChainSet>> sets(1);
+    if (int rc = make_chain_set(*t, true, true, nullptr, &sets[0])) return rc;
     W->table_valid = false;
-    int rc = upload_and_launch(*W, passes, tdev, true, t->d_rho0, nullptr);
+    int rc = upload_and_launch(*W, passes, tdev, sets, true, t->d_rho0, nullptr);
     W->table_valid = false;
     if (rc != NEGF_OK) return rc;
     NEGF_CUDA(cudaStreamSynchronize(nullptr));
@@ -1401,10 +1766,18 @@ int negf_compute_charge(negf_tube* const* tubes, int num_tubes, double* Q, int q
     std::vector<TubePass> passes;
     std::vector<negf::TubeDev> tdev;
     long long off = 0;
-    bool same = W.table_valid && W.key_serials.size() == (size_t)num_tubes;
+    Settings& G = settings();
+    std::vector<std::shared_ptr<const ChainSet>> sets;
+    for (int i = 0; i < num_tubes; ++i) update_paths(*tubes[i]);
+    const bool split = use_groups(tubes, num_tubes, false);
+    bool same = W.table_valid && W.key_serials.size() == (size_t)num_tubes && W.key_pieces == G.pass1_pieces &&
+                W.key_schedule == G.schedule;
     for (int i = 0; i < num_tubes; ++i) {
         negf_tube* t = tubes[i];
-        update_paths(*t);
+        if (split) {
+            sets.emplace_back();
+            if (int rc = chain_set(*t, s, &sets.back())) return rc;
+        }
         passes.push_back({t, i, off, false});
         tdev.push_back(make_tubedev(*t, false));
         off += t->N;
@@ -1415,11 +1788,13 @@ int negf_compute_charge(negf_tube* const* tubes, int num_tubes, double* Q, int q
         NEGF_CUDA(W.qbuf.reserve(sizeof(double) * off));
         dQ = W.qbuf.as<double>();
     }
-    int rc = upload_and_launch(W, passes, tdev, !same, dQ, s);
+    int rc = upload_and_launch(W, passes, tdev, sets, !same, dQ, s);
     if (rc) {
         W.table_valid = false;
         return rc;
     }
+    W.key_pieces = G.pass1_pieces;
+    W.key_schedule = G.schedule;
     W.key_serials.clear();
     W.key_versions.clear();
     for (int i = 0; i < num_tubes; ++i) {
@@ -1457,24 +1832,29 @@ int plan_tables(negf_charge_plan& p, int spu, bool upload_all) {
         off += p.tubes[i]->N;
     }
     ChainTable ct;
-    Out<negf::ChainRec> oc;
-    oc.vec = &ct.chains;
-    Out<negf::WarpRec> ow;
-    ow.vec = &ct.warps;
-    Out<negf::SegUnit> ou;
-    ou.vec = &ct.units;
-    ct.rts.resize(n);
-    std::vector<int> order(n);
-    TableCounts cnt;
-    build_table_generic(passes.data(), n, order.data(), oc, ow, ou, ct.rts.data(), cnt, spu);
+    std::vector<std::shared_ptr<const ChainSet>> sets;
+    int rc = NEGF_OK;
+    if (use_groups(p.tubes.data(), n, p.force_fp64)) {
+        if (!p.fp64.sets.empty()) {
+            sets = p.fp64.sets;
+        } else {
+            for (int i = 0; i < n && rc == NEGF_OK; ++i) {
+                sets.emplace_back();
+                rc = p.force_fp64 ? make_chain_set(*p.tubes[i], false, true, nullptr, &sets.back())
+                                  : chain_set(*p.tubes[i], nullptr, &sets.back());
+            }
+        }
+    }
+    if (rc == NEGF_OK) build_table(ct, passes, tdev, sets, settings().pass1_pieces, spu);
     for (int i = 0; i < n; ++i) p.tubes[i]->d.precision = saved[i];
-    fused_order(ct);
+    if (rc) return rc;
+    p.fp64 = ct.fp64;
     p.n64 = ct.n64;
     p.n32 = ct.n32;
     p.num_warps = (int)ct.warps.size();
     p.num_units = (int)ct.units.size();
-    p.max_N = cnt.max_N;
-    p.updates = cnt.updates;
+    p.max_N = ct.max_N;
+    p.updates = ct.updates;
     p.spu = spu;
     NEGF_CUDA(p.d_units.reserve(std::max<size_t>(1, ct.units.size()) * sizeof(negf::SegUnit)));
     if (!ct.units.empty())
@@ -1488,8 +1868,12 @@ int plan_tables(negf_charge_plan& p, int spu, bool upload_all) {
     NEGF_CUDA(p.d_chains.reserve(std::max<size_t>(1, ct.chains.size()) * sizeof(negf::ChainRec)));
     NEGF_CUDA(p.d_warps.reserve(std::max<size_t>(1, ct.warps.size()) * sizeof(negf::WarpRec)));
     NEGF_CUDA(p.d_rts.reserve(ct.rts.size() * sizeof(negf::ReduceTube)));
-    NEGF_CUDA(p.d_partial.reserve(std::max<long long>(1, cnt.partial_doubles) * sizeof(double)));
-    NEGF_CUDA(p.d_scratch.reserve(std::max<long long>(1, cnt.scratch_doubles) * sizeof(double)));
+    NEGF_CUDA(p.d_partial.reserve(std::max<long long>(1, ct.partial_doubles) * sizeof(double)));
+    NEGF_CUDA(p.d_scratch.reserve(std::max<long long>(1, ct.scratch_doubles) * sizeof(double)));
+    NEGF_CUDA(p.d_ck.reserve(std::max<long long>(1, ct.fp64.ck_doubles) * sizeof(double)));
+    NEGF_CUDA(p.d_cc.reserve(std::max<long long>(1, ct.fp64.cc_doubles) * sizeof(double)));
+    NEGF_CUDA(p.d_tm.reserve(std::max<long long>(1, ct.fp64.tm_doubles) * sizeof(double)));
+    if (int rc2 = upload_groups(ct.fp64, p.d_groups, nullptr)) return rc2;
     NEGF_CUDA(cudaMemcpy(p.d_tubes.p, tdev.data(), tdev.size() * sizeof(negf::TubeDev), cudaMemcpyHostToDevice));
     if (!ct.chains.empty())
         NEGF_CUDA(cudaMemcpy(p.d_chains.p, ct.chains.data(), ct.chains.size() * sizeof(negf::ChainRec),
@@ -1499,19 +1883,33 @@ int plan_tables(negf_charge_plan& p, int spu, bool upload_all) {
                              cudaMemcpyHostToDevice));
     for (int i = 0; i < n; ++i) ct.rts[i].rho0 = p.tubes[i]->shard_rank == 0 ? p.tubes[i]->d_rho0 : nullptr;
     NEGF_CUDA(cudaMemcpy(p.d_rts.p, ct.rts.data(), ct.rts.size() * sizeof(negf::ReduceTube), cudaMemcpyHostToDevice));
+    p.rt0 = ct.rts[0];
+    // pageable copies may still be in flight, and the plan's streams may not wait for the legacy one
+    NEGF_CUDA(cudaStreamSynchronize(nullptr));
     return NEGF_OK;
 }
 
 cudaError_t plan_launch(const negf_charge_plan& p, const int* skip, cudaStream_t s, cudaStream_t side) {
-    const negf::FusedOrder fo{p.d_order.as<int>(), p.n64, p.n32, side, p.fork, p.join};
-    cudaError_t e = negf::launch_rgf(p.d_tubes.as<negf::TubeDev>(), p.d_chains.as<negf::ChainRec>(),
-                                     p.d_warps.as<negf::WarpRec>(), p.num_warps, p.d_units.as<negf::SegUnit>(),
-                                     p.num_units, p.d_partial.as<double>(), p.d_scratch.p, p.wpb, s, nullptr, skip,
-                                     p.schedule == negf::kScheduleFused ? 1 : p.pieces, p.d_pieces.as<double>(),
-                                     p.schedule, &fo);
+    const cudaError_t e = launch_split(
+        p.fp64.any(), p.num_warps > 0, s, side, p.fork, p.join,
+        [&] {
+            return launch_fp64(p.fp64, p.d_groups, p.d_ck, p.d_cc, p.d_tm, p.d_partial.as<double>(), skip, s, nullptr);
+        },
+        [&](cudaStream_t s32) {
+            const negf::FusedOrder fo{p.d_order.as<int>(), p.n64, p.n32, side, p.fork, p.join};
+            return negf::launch_rgf(p.d_tubes.as<negf::TubeDev>(), p.d_chains.as<negf::ChainRec>(),
+                                    p.d_warps.as<negf::WarpRec>(), p.num_warps, p.d_units.as<negf::SegUnit>(),
+                                    p.num_units, p.d_partial.as<double>(), p.d_scratch.p, p.wpb, s32, nullptr, skip,
+                                    p.schedule == negf::kScheduleFused ? 1 : p.pieces, p.d_pieces.as<double>(),
+                                    p.schedule, &fo);
+        });
     if (e != cudaSuccess) return e;
-    return negf::launch_reduce(p.d_rts.as<negf::ReduceTube>(), (int)p.tubes.size(), p.max_N,
-                               p.d_partial.as<double>(), p.d_Q, s, skip);
+    negf::ReduceSet rs{};
+    if (p.tubes.size() == 1)
+        rs.one = p.rt0;
+    else
+        rs.ext = p.d_rts.as<negf::ReduceTube>();
+    return negf::launch_reduce(rs, (int)p.tubes.size(), p.max_N, p.d_partial.as<double>(), p.d_Q, s, skip);
 }
 }  // namespace
 
@@ -1543,23 +1941,25 @@ int negf_charge_plan_create(negf_tube* const* tubes, int num_tubes, double* d_Q,
         // pass-1 pieces as negf_compute_charge chooses them (the setting, else the automatic rule)
         int pc = settings().pass1_pieces;
         if (pc == 0 && settings().schedule == NEGF_SCHEDULE_FUSED) pc = 1;
-        if (pc == 0) pc = auto_pieces(p->num_warps, p->max_N);
+        if (pc == 0) pc = auto_pieces(p->num_warps + p->fp64.warps, p->max_N);
         p->pieces = std::max(1, pc);
     }
-    p->schedule = choose_schedule(settings().schedule, p->num_warps, p->pieces);
+    p->schedule = p->num_warps > 0 ? choose_schedule(settings().schedule, p->num_warps + p->fp64.warps, p->pieces)
+                                   : negf::kScheduleTwoPass;
     if (p->schedule == negf::kScheduleFused) p->pieces = 1;
+    if (p->num_warps == 0 && settings().pass1_pieces == 0) p->pieces = reported_pieces(p->fp64);
     // piece candidates of the autotuner: only when the chains cannot fill the GPU
     std::vector<int> piece_cands = {1};
-    if ((flags & NEGF_PLAN_AUTOTUNE) && p->num_warps < 4 * device_sm_count()) {
+    if ((flags & NEGF_PLAN_AUTOTUNE) && p->num_warps > 0 && p->num_warps + p->fp64.warps < 4 * device_sm_count()) {
         const int maxp = std::min(128, std::max(1, ((p->max_N + negf::kSeg - 1) / negf::kSeg) / 32));
-        for (int q : {2, 4, 8, auto_pieces(p->num_warps, p->max_N)})
+        for (int q : {2, 4, 8, auto_pieces(p->num_warps + p->fp64.warps, p->max_N)})
             if (q > 1 && q <= maxp && std::find(piece_cands.begin(), piece_cands.end(), q) == piece_cands.end())
                 piece_cands.push_back(q);
     }
     {
         int maxpc = p->pieces;
         for (int q : piece_cands) maxpc = std::max(maxpc, q);
-        if (maxpc > 1)
+        if (maxpc > 1 && p->num_warps > 0)
             NEGF_CUDA(p->d_pieces.reserve(sizeof(double) * (size_t)std::max(1, p->num_warps) * maxpc * 24 *
                                           negf::kWarp));
     }
@@ -1571,16 +1971,24 @@ int negf_charge_plan_create(negf_tube* const* tubes, int num_tubes, double* d_Q,
         NEGF_CUDA(cudaEventCreate(&e1));
         double best = 1e300;
         int best_spu = negf::kSegsPerUnit, best_wpb = p->wpb, best_pc = 1;
+        // no warp tables: the FP64 groups have nothing to choose (their shape
+        // follows the rules of plan_groups), one shape is timed
+        const bool choose = p->num_warps > 0;
+        if (!choose) best_pc = p->pieces;
         for (int spu : {16, 32, 64}) {
+            if (!choose && spu != negf::kSegsPerUnit) continue;
             rc = plan_tables(*p, spu, false);
             if (rc) break;
             for (int wpb : {0, 1, 2, 4}) {
+                if (!choose && wpb != p->wpb) continue;
                 if (wpb == 0 && spu != 16) continue;  // the fused schedule has no segment units
                 for (int pc : piece_cands) {
                     if (wpb == 0 && pc != 1) continue;  // the fused schedule runs whole chains
-                    p->wpb = wpb == 0 ? 4 : wpb;
-                    p->schedule = wpb == 0 ? negf::kScheduleFused : negf::kScheduleTwoPass;
-                    p->pieces = pc;
+                    if (choose) {
+                        p->wpb = wpb == 0 ? 4 : wpb;
+                        p->schedule = wpb == 0 ? negf::kScheduleFused : negf::kScheduleTwoPass;
+                        p->pieces = pc;
+                    }
                     cudaError_t e = plan_launch(*p, nullptr, 0, side0);
                     for (int r = 0; r < 3 && e == cudaSuccess; ++r) {
                         if (r == 1) e = cudaEventRecord(e0, 0);
@@ -1599,7 +2007,7 @@ int negf_charge_plan_create(negf_tube* const* tubes, int num_tubes, double* d_Q,
                         best = ms / 2;
                         best_spu = spu;
                         best_wpb = wpb;
-                        best_pc = pc;
+                        best_pc = choose ? pc : p->pieces;
                     }
                 }
             }

@@ -61,6 +61,13 @@ struct __align__(16) ReduceTube {
     int num_rows;        // warps of the tube
 };
 
+// Reduction table of a launch: one tube in the kernel's parameters, more in
+// device memory.
+struct ReduceSet {
+    const ReduceTube* ext;
+    ReduceTube one;
+};
+
 // Pass-2 work unit: segments [seg0, seg1) of the chains of one warp.
 struct __align__(16) SegUnit {
     int warp;
@@ -68,6 +75,53 @@ struct __align__(16) SegUnit {
     int pad;
 };
 constexpr int kSegsPerUnit = 32;  // segments per pass-2 unit (256 sites)
+
+// ---- FP64 passes (negf_sweep.cu): chains grouped by (tube, kind).
+constexpr int kSweepSeg = 16;  // sites per segment (2 for tubes of fewer sites)
+constexpr int kConst = 8;      // doubles of constants per chain
+constexpr int kModeBits = 6;   // chain code = energy index << kModeBits | mode
+static_assert(kMaxModes <= (1 << kModeBits), "mode does not fit its bits");
+
+struct EnergyRec {  // one energy point (device table of a tube)
+    double Er, Ei;  // energy
+    double cr, ci;  // contour coefficient of G_nn
+    double b0, b1;  // real-axis coefficients of the two contacts
+};
+struct __align__(16) GroupDev {
+    const double* U;         // potential, kPadLo / kPadHi zeros around it
+    const EnergyRec* items;  // the tube's energies
+    const int* chains;       // codes of the group's chains
+    int N, nseg, nblk;       // sites, segments, blocks of 8 segments
+    int kind, nch;           // WarpKind, chains
+    int use_decimation, dec_iters, dec_layers, uc_from_U;
+    double gamma, Uc0, Uc1;
+    long long ck_off;    // boundary states (layout in negf_sweep.cu)
+    long long cc_off;    // constants [chain][kConst]
+    long long row_base;  // first partial row (one per unit of chains)
+    int sweep_base, chain_base, seg_base;    // first block of the group in each kernel
+    int chains_per_unit, nsb, lanes;         // seg_kernel: chains of a unit, segment blocks, segments side by side in a warp
+    int tm_segs;                             // scan_kernel: matrices per chain in its scratch
+    int pad;
+    double beta[kMaxModes], degen[kMaxModes];
+};
+// Groups of a launch: up to two in the kernel's parameters (one tube: no
+// table upload), more in device memory.  The first blocks of up to
+// kMaxBases groups stand in the parameters in either case, so that a block
+// finds its group without a chain of global loads.
+constexpr int kMaxBases = 64;
+struct GroupSet {
+    const GroupDev* ext;
+    int ng;
+    int sweep_base[kMaxBases], chain_base[kMaxBases], seg_base[kMaxBases];
+    GroupDev g[2];
+};
+struct SweepShape {
+    int K;                  // kSweepSeg or 2
+    int scan;               // boundary states by scan_kernel (parallel in length) instead of sweep_kernel
+    int chains, scan_threads, sweep_blocks, seg_blocks;
+};
+cudaError_t launch_sweep(const GroupSet& gs, const SweepShape& sh, double* ck, double* cc, double* tm, double* partial,
+                         const int* skip, cudaStream_t s, cudaEvent_t mid);
 
 // RGF launch: pass 1 (one warp per WarpRec, lane = chain: concurrent forward
 // and backward sweeps storing boundary checkpoints) then pass 2 (one warp per
@@ -161,7 +215,7 @@ cudaError_t launch_rgf(const TubeDev* d_tubes, const ChainRec* d_chains, const W
 // 1 FP32 reciprocal (input/output as doubles), n values, device pointers.
 cudaError_t selftest(int which, int n, const double* d_in, double* d_out, cudaStream_t stream);
 // Per-site reduction (Kahan) of warp rows, minus Rho0 when rho0 != null.
-cudaError_t launch_reduce(const ReduceTube* d_rt, int num_tubes, int max_N, const double* d_partial, double* d_Q,
+cudaError_t launch_reduce(const ReduceSet& rs, int num_tubes, int max_N, const double* d_partial, double* d_Q,
                           cudaStream_t stream,
                           const int* skip = nullptr);
 // Scratch elements (doubles, rounded up) needed per warp for a tube of N sites.

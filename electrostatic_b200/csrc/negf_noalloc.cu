@@ -134,7 +134,9 @@ extern "C" int negf_compute_charge_noalloc(negf_tube* const* tubes, int num_tube
                    reinterpret_cast<const SegUnit*>(base + o_units), (int)fp.num_units,
                    reinterpret_cast<double*>(base + o_partial), base + o_ck, 4, s, nullptr);
     if (e != cudaSuccess) return report(NEGF_ERR_CUDA, cudaGetErrorString(e));
-    e = launch_reduce(reinterpret_cast<const ReduceTube*>(base + o_rts), fp.num_tubes, fp.max_N,
+    ReduceSet rs{};
+    rs.ext = reinterpret_cast<const ReduceTube*>(base + o_rts);
+    e = launch_reduce(rs, fp.num_tubes, fp.max_N,
                       reinterpret_cast<const double*>(base + o_partial), d_Q, s);
     if (e != cudaSuccess) return report(NEGF_ERR_CUDA, cudaGetErrorString(e));
     return NEGF_OK;

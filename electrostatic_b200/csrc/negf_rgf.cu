@@ -1449,56 +1449,68 @@ __global__ void selftest_kernel(int which, int n, const double* __restrict__ in,
 }
 
 // Q[q_off + n] = sum_w partial[row_base + w N + n] - rho0[n].
-// Block = 32 sites x kRowGroups row groups; each thread sums rows
-// g, g + kRowGroups, ... with Kahan compensation, then the row groups are
-// combined in a fixed order (deterministic).  32 row groups: a 4000-site tube
-// gives 125 blocks of 32 warps, enough loads in flight to stream the rows
-// at HBM rate.
-constexpr int kRowGroups = 32;
-__global__ void __launch_bounds__(32 * kRowGroups) reduce_kernel(const ReduceTube* __restrict__ rts,
-                                                                 const double* __restrict__ partial,
-                                                                 double* __restrict__ Q, const int* __restrict__ skip) {
+// Block = 32 sites x RG row groups; each thread sums rows g, g + RG, ... with
+// Kahan compensation and eight loads in flight, then RG lanes per site combine
+// the groups in a fixed tree of error-free additions (deterministic).  Bound
+// by the latency of its rounds of loads: 32 groups when there are too few
+// blocks to fill the GPU (short tubes), 8 groups and small blocks otherwise.
+// (A serial combination of 32 groups by 32 threads kept a block of 1024
+// threads resident for another 1.2 us.)
+constexpr int kRowLoads = 8;
+template <int RG>
+__global__ void __launch_bounds__(32 * RG) reduce_kernel(const __grid_constant__ ReduceSet rs,
+                                                         const double* __restrict__ partial, double* __restrict__ Q,
+                                                         const int* __restrict__ skip) {
     if (skip && *skip) return;  // uniform over the block
-    __shared__ double sh_s[kRowGroups][32], sh_c[kRowGroups][32];
-    const ReduceTube r = rts[blockIdx.y];
-    const int n = blockIdx.x * 32 + threadIdx.x;
+    __shared__ double sh_s[RG][33], sh_c[RG][33];
+    const ReduceTube r = rs.ext ? rs.ext[blockIdx.y] : rs.one;
+    const int n0 = blockIdx.x * 32, n = n0 + threadIdx.x;
+    if (n0 >= r.N) return;  // the grid covers the longest tube
     const int g = threadIdx.y;
     double s = 0.0, comp = 0.0;
     if (n < r.N) {
         const double* p = partial + r.row_base + n;
-        int w = g;
-        for (; w + 3 * kRowGroups < r.num_rows; w += 4 * kRowGroups) {
-            double v[4];
-#pragma unroll
-            for (int k = 0; k < 4; ++k) v[k] = p[(size_t)(w + k * kRowGroups) * r.N];
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                const double y = v[k] - comp;
-                const double t = s + y;
-                comp = (t - s) - y;
-                s = t;
-            }
-        }
-        for (; w < r.num_rows; w += kRowGroups) {
-            const double y = p[(size_t)w * r.N] - comp;
+        auto add = [&](double v) {
+            const double y = v - comp;
             const double t = s + y;
             comp = (t - s) - y;
             s = t;
+        };
+        int w = g;
+        for (; w + (kRowLoads - 1) * RG < r.num_rows; w += kRowLoads * RG) {
+            double v[kRowLoads];
+#pragma unroll
+            for (int k = 0; k < kRowLoads; ++k) v[k] = p[(size_t)(w + k * RG) * r.N];
+#pragma unroll
+            for (int k = 0; k < kRowLoads; ++k) add(v[k]);
+        }
+        if (w < r.num_rows) {  // the last round: rows past the end repeat the last one and add 0
+            double v[kRowLoads];
+#pragma unroll
+            for (int k = 0; k < kRowLoads; ++k) v[k] = p[(size_t)min(w + k * RG, r.num_rows - 1) * r.N];
+#pragma unroll
+            for (int k = 0; k < kRowLoads; ++k) add(w + k * RG < r.num_rows ? v[k] : 0.0);
         }
     }
     sh_s[g][threadIdx.x] = s;
     sh_c[g][threadIdx.x] = comp;
     __syncthreads();
-    if (g == 0 && n < r.N) {
-        double tot = 0.0, cc = 0.0;
-        for (int k = 0; k < kRowGroups; ++k) {
-            const double y = (sh_s[k][threadIdx.x] - sh_c[k][threadIdx.x]) - cc;
-            const double t = tot + y;
-            cc = (t - tot) - y;
-            tot = t;
-        }
-        if (r.rho0) tot -= r.rho0[n];
-        Q[r.q_off + n] = tot;
+    const int site = g * (32 / RG) + threadIdx.x / RG, grp = threadIdx.x % RG;
+    s = sh_s[grp][site];
+    comp = -sh_c[grp][site];  // the sum is s + comp
+#pragma unroll
+    for (int o = RG / 2; o >= 1; o >>= 1) {
+        const double s2 = __shfl_xor_sync(kFull, s, o), c2 = __shfl_xor_sync(kFull, comp, o);
+        // error-free s + s2 (the same in both lanes: the larger lane's operands swapped)
+        const double a = threadIdx.x & o ? s2 : s, b = threadIdx.x & o ? s : s2;
+        const double t = a + b, bb = t - a;
+        comp = (comp + c2) + ((a - (t - bb)) + (b - bb));
+        s = t;
+    }
+    if (grp == 0 && n0 + site < r.N) {
+        double tot = s + comp;
+        if (r.rho0) tot -= r.rho0[n0 + site];
+        Q[r.q_off + n0 + site] = tot;
     }
 }
 
@@ -1751,12 +1763,14 @@ cudaError_t selftest(int which, int n, const double* d_in, double* d_out, cudaSt
     return cudaGetLastError();
 }
 
-cudaError_t launch_reduce(const ReduceTube* d_rt, int num_tubes, int max_N, const double* d_partial, double* d_Q,
+cudaError_t launch_reduce(const ReduceSet& rs, int num_tubes, int max_N, const double* d_partial, double* d_Q,
                           cudaStream_t stream, const int* skip) {
     if (num_tubes <= 0 || max_N <= 0) return cudaSuccess;
-    dim3 grid((max_N + 31) / 32, num_tubes);
-    dim3 block(32, kRowGroups);
-    reduce_kernel<<<grid, block, 0, stream>>>(d_rt, d_partial, d_Q, skip);
+    const dim3 grid((max_N + 31) / 32, num_tubes);
+    if ((long long)grid.x * grid.y < 296)  // two blocks of 1024 threads per SM
+        reduce_kernel<32><<<grid, dim3(32, 32), 0, stream>>>(rs, d_partial, d_Q, skip);
+    else
+        reduce_kernel<8><<<grid, dim3(32, 8), 0, stream>>>(rs, d_partial, d_Q, skip);
     return cudaGetLastError();
 }
 

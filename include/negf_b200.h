@@ -207,7 +207,7 @@ typedef struct negf_stats {
     int warps;                 /* pass-1 warps launched */
     int units;                 /* pass-2 warps (segment groups) launched */
     int kernel_launches;       /* kernels launched by the call */
-    int pieces;                /* pass-1 pieces per chain (parallel in length) */
+    int pieces;                /* pass-1 pieces per chain (parallel in length; automatic: segments) */
     long long checkpoint_bytes;/* scratch bytes written+read by the kernel */
     int schedule;              /* NEGF_SCHEDULE_TWO_PASS or NEGF_SCHEDULE_FUSED */
 } negf_stats;
@@ -219,21 +219,26 @@ int negf_last_stats(negf_stats* s);
  *   backward sweeps of every chain run as P pieces of the tube in parallel
  *   ("parallel in length", for long tubes with few energies): 2 x 2 transfer
  *   matrices of each piece, a prefix over the pieces for their boundary
- *   states, then the pieces' sweeps.  Automatic: when the chains fill
- *   fewer than 4 warps per SM, enough pieces for about 8 warps per SM, each
- *   of >= 32 segments (256 sites), at most 128.  Results agree with P = 1 to
- *   rounding (relative 1e-10 in the tests, about 1e-12 measured).
+ *   states, then the pieces' sweeps.  Automatic for FP32 chains: when the
+ *   chains fill fewer than 4 warps per SM, enough pieces for about 8 warps
+ *   per SM, each of >= 32 segments (256 sites), at most 128.  FP64 chains of
+ *   the two-pass schedule are parallel in length by whole 16-site segments
+ *   for any P > 1 (one scan per chain) and automatically when few long
+ *   chains would leave the sweeps waiting on their steps.  Results agree with
+ *   P = 1 to rounding (relative 1e-10 in the tests, about 1e-12 measured).
  * NEGF_TUNE_SCHEDULE: 0 (default, automatic), NEGF_SCHEDULE_TWO_PASS or
  *   NEGF_SCHEDULE_FUSED.  Two-pass: pass 1 runs both sweeps of every chain
- *   and checkpoints them at every 8-site segment, pass 2 integrates the
- *   segments in parallel tiles (parallelism for few chains).  Fused: one
+ *   and stores their states at every segment boundary (16 sites in FP64, 8 in
+ *   FP32), pass 2 integrates the segments in parallel.  Fused: one
  *   kernel; the forward sweep crosses the first half of the tube and the
  *   backward sweep the second, each storing its own checkpoints, then each
  *   continues into the other half and integrates the segments it crosses
  *   (every site crossed twice instead of three times, half the checkpoint
- *   bytes; needs enough chains to fill the GPU).  Automatic: fused when the
- *   chains fill at least one warp per SM sub-partition and the sweeps run as
- *   one piece.  Results agree to rounding. */
+ *   bytes; needs enough chains to fill the GPU).  Automatic: two-pass for
+ *   batches whose work is mostly FP64; for mostly FP32 batches (and the FP32
+ *   chains of the others) fused when the chains fill at least one warp per
+ *   SM sub-partition and the sweeps run as one piece.  Results agree to
+ *   rounding. */
 #define NEGF_TUNE_PASS2_WARPS_PER_BLOCK 2
 #define NEGF_TUNE_PASS1_PIECES 4
 #define NEGF_TUNE_SCHEDULE 6
