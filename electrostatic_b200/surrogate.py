@@ -150,7 +150,8 @@ class FourierOperator:
         h = self._buf("h0", (R, W))
         hb = self._buf("h0b", (R, W), t.bfloat16)
         self._gemm(0, 0, R, W, self.feat, 1, xb, self.feat, 0, self.bf["W_lift"], W, 0, h, W, 0)
-        check(L.negf_nn_gelu_fwd(R, W, _p(h), None, _p(self.params["b_lift"]), None, _p(h), _p(hb), 0, self._s()),
+        # only the BF16 copy of a hidden state is read again (the last layer's FP32 one by the projection)
+        check(L.negf_nn_gelu_fwd(R, W, _p(h), None, _p(self.params["b_lift"]), None, None, _p(hb), 0, self._s()),
               "lift")
         for l in range(LAYERS):
             s1 = self._buf(f"s1_{l}", (R, W))
@@ -167,7 +168,7 @@ class FourierOperator:
                        z, 2 * M * W, 2 * W, zb)
             self._gemm(0, 0, S, W, 2 * M, B, Ga, 2 * M, sG, zb, W, 2 * M * W, s2, W, S * W)
             pre = self._buf(f"pre{l}", (R, W)) if keep else None
-            hn = self._buf(f"h{l + 1}", (R, W))
+            hn = self._buf(f"h{l + 1}", (R, W)) if l == LAYERS - 1 else None
             hnb = self._buf(f"h{l + 1}b", (R, W), t.bfloat16)
             check(L.negf_nn_gelu_fwd(R, W, _p(s1), _p(s2), _p(self.params[f"b{l}"]), _p(pre), _p(hn), _p(hnb), 1,
                                      self._s()), "gelu")

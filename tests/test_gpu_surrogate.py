@@ -164,3 +164,54 @@ def test_fixed_point_surrogate_set_sweep():
         assert np.max(np.abs(a.Q - b.Q)) <= 2e-6
     for t in tubes + mixed:
         t.close()
+
+
+@pytest.mark.parametrize("rows,cols,off", [(1, 1, 0), (7, 3, 0), (64, 8, 0), (513, 9, 0), (4097, 12, 0), (4097, 12, 1),
+                                           (60001, 128, 0)])
+def test_elementwise_kernels_and_column_sums(rows, cols, off):
+    """Column sums over the blocks of a cluster, and the elementwise kernels by
+    four and one by one (odd counts; operands off the 16-byte boundary) give
+    the same values."""
+    import ctypes as C
+    import torch
+    from electrostatic_b200 import _lib
+    L = _lib.load()
+    g = torch.Generator(device="cuda").manual_seed(rows + cols)
+    n = rows * cols
+
+    def dev(k=n):
+        return torch.randn(k + off, generator=g, device="cuda")[off:]
+
+    def p(t):
+        return C.c_void_p(t.data_ptr())
+    x, b, bias, dy, dq, w = dev(), dev(), dev(cols), dev(), dev(rows), dev(cols)
+    out = torch.empty(cols, device="cuda")
+    assert L.negf_nn_colsum(rows, cols, p(x), p(out), 0, None) == 0
+    ref = x.double().reshape(rows, cols).sum(0)
+    # sequential runs of at most rows / 64 additions, then 16 + 8: eps times the sum of magnitudes times that depth
+    bound = 6e-8 * (rows / 64 + 30) * x.double().abs().reshape(rows, cols).sum(0)
+    assert bool(((out.double() - ref).abs() <= bound).all())
+    first = out.clone()
+    assert L.negf_nn_colsum(rows, cols, p(x), p(out), 1, None) == 0
+    assert torch.equal(out, first + first)
+
+    def gelu(x, b, bias, dy, dq, w):
+        pre, y, d, dh = (torch.zeros(n + off, device="cuda")[off:] for _ in range(4))
+        yb, db, dhb, xb = (torch.zeros(n + off, device="cuda", dtype=torch.bfloat16)[off:] for _ in range(4))
+        assert L.negf_nn_gelu_fwd(rows, cols, p(x), p(b), p(bias), p(pre), p(y), p(yb), 1, None) == 0
+        assert L.negf_nn_gelu_bwd(n, p(dy), p(x), p(d), p(db), None) == 0
+        assert L.negf_nn_outer(rows, cols, p(dq), p(w), p(dh), p(dhb), None) == 0
+        assert L.negf_nn_cast_bf16(n, p(x), p(xb), None) == 0
+        return pre, y, yb, d, db, dh, dhb, xb
+    pre, y, yb, d, db, dh, dhb, xb = gelu(x, b, bias, dy, dq, w)
+    X = x.reshape(rows, cols)
+    assert torch.equal(pre.reshape(rows, cols), (X + b.reshape(rows, cols)) + bias)
+    t = pre.double().requires_grad_()
+    ref = torch.nn.functional.gelu(t, approximate="tanh")
+    assert float((y.double() - ref.detach()).abs().max()) <= 4e-6  # a few roundings of values of order 4
+    xr = x.double().requires_grad_()
+    torch.nn.functional.gelu(xr, approximate="tanh").backward(dy.double())
+    assert float((d.double() - xr.grad).abs().max()) <= 2e-5
+    assert torch.equal(dh.reshape(rows, cols), dq[:, None] * w[None, :])
+    for full, half in ((y, yb), (d, db), (dh, dhb), (x, xb)):
+        assert torch.equal(full.to(torch.bfloat16), half)
