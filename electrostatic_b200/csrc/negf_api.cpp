@@ -268,6 +268,7 @@ struct Workspace {
     int device = 0;
     cudaStream_t stream = nullptr;
     DevBuf tubes, chains, warps, rts, units, partial, scratch, qbuf, pieces, order;
+    DevBuf trTable, trOut, trLdos;  // transport characteristics
     DevBuf ck, cc, tm, groups;  // FP64 part: boundary states, chain constants, scan matrices, group table
     cudaStream_t side = nullptr;                 // the FP32 warps of the fused schedule
     cudaEvent_t fork = nullptr, join = nullptr;  // around them
@@ -293,7 +294,7 @@ struct Workspace {
         if (join) cudaEventDestroy(join);
         if (side) cudaStreamDestroy(side);
         DevBuf* bufs[] = {&tubes, &chains, &warps, &rts,  &units, &partial,   &scratch, &qbuf,   &pieces,
-                          &ck,    &cc,   &tm,    &groups, &order, &rsE,    &rsFlags, &rsU0, &rsUa, &rsCorners, &rsGL,    &rsGLn,  &rsRows,
+                          &ck,    &cc,   &tm,    &groups, &trTable, &trOut, &trLdos, &order, &rsE,    &rsFlags, &rsU0, &rsUa, &rsCorners, &rsGL,    &rsGLn,  &rsRows,
                           &rsStatus};
         for (DevBuf* b : bufs) {
             if (b->p) cudaFree(b->p);
@@ -881,17 +882,18 @@ int chain_set(negf_tube& t, cudaStream_t stream, std::shared_ptr<const ChainSet>
     return NEGF_OK;
 }
 
-// One group's constant fields and its place in the launch.
-negf::GroupDev make_group(const negf::TubeDev& d, const ChainSet& cs, int kind, int K) {
+// A group's fields but its places in the launch's buffers and grids.
+negf::GroupDev make_group(const negf::TubeDev& d, const negf::EnergyRec* items, const int* codes, int kind, int nch,
+                          int K) {
     negf::GroupDev g{};
     g.U = d.U;
-    g.items = cs.items.as<negf::EnergyRec>();
-    g.chains = cs.codes.as<int>() + (kind == negf::kRealAxis ? cs.contour : 0);
+    g.items = items;
+    g.chains = codes;
     g.N = d.N;
     g.nseg = (d.N + K - 1) / K;
     g.nblk = (g.nseg + 7) / 8;
     g.kind = kind;
-    g.nch = kind == negf::kRealAxis ? cs.realaxis : cs.contour;
+    g.nch = nch;
     g.use_decimation = d.use_decimation;
     g.dec_iters = d.dec_iters;
     g.dec_layers = d.dec_layers;
@@ -907,6 +909,11 @@ negf::GroupDev make_group(const negf::TubeDev& d, const ChainSet& cs, int kind, 
     return g;
 }
 
+// Doubles of a group's boundary states (the layout of negf_sweep.cu).
+long long group_state_doubles(const negf::GroupDev& g) {
+    return (long long)((g.nch + 31) / 32) * g.nblk * (g.kind == negf::kRealAxis ? 6 : 4) * 256;
+}
+
 // Groups of the FP64 chains of a launch, longest tubes first.  pieces: the
 // setting (0 automatic, 1 sweeps, more: parallel in length).
 void plan_groups(SweepPart& sp, const TubePass* passes, const negf::TubeDev* tdev, int num_passes, int pieces) {
@@ -918,8 +925,11 @@ void plan_groups(SweepPart& sp, const TubePass* passes, const negf::TubeDev* tde
         const ChainSet& cs = *sp.sets[o];
         const int k = tdev[o].N < negf::kSweepSeg ? 1 : 0;
         for (int kind : {negf::kRealAxis, negf::kContour}) {
-            if ((kind == negf::kRealAxis ? cs.realaxis : cs.contour) == 0) continue;
-            sp.groups[k].push_back(make_group(tdev[o], cs, kind, k ? 2 : negf::kSweepSeg));
+            const int nch = kind == negf::kRealAxis ? cs.realaxis : cs.contour;
+            if (nch == 0) continue;
+            sp.groups[k].push_back(make_group(tdev[o], cs.items.as<negf::EnergyRec>(),
+                                              cs.codes.as<int>() + (kind == negf::kRealAxis ? cs.contour : 0), kind,
+                                              nch, k ? 2 : negf::kSweepSeg));
             sp.pass_of[k].push_back(o);
             const negf::GroupDev& g = sp.groups[k].back();
             const int cpw = 32 / g.lanes;
@@ -950,9 +960,8 @@ void plan_groups(SweepPart& sp, const TubePass* passes, const negf::TubeDev* tde
             sh.sweep_blocks += 2 * ((g.nch + 31) / 32);
             sh.chains += g.nch;
             sh.seg_blocks += g.nsb * ((g.nch + g.chains_per_unit - 1) / g.chains_per_unit);
-            const int comps = g.kind == negf::kRealAxis ? 6 : 4;
             g.ck_off = sp.ck_doubles;
-            sp.ck_doubles += (long long)((g.nch + 31) / 32) * g.nblk * comps * 256;
+            sp.ck_doubles += group_state_doubles(g);
             g.cc_off = sp.cc_doubles;
             sp.cc_doubles += (long long)g.nch * negf::kConst;
             max_nseg = std::max(max_nseg, g.nseg);
@@ -1303,82 +1312,70 @@ std::vector<Pt> dos_points(const negf_tube& t) {
 }
 
 // One transport run of a tube over energies pts: red[e][8] (see
-// negf::launch_transport) and, when ldos != null, LDOS [e][N].  Every buffer
-// is local to the call (this runs once per bias step, not per SCF iteration).
+// transport_kernel in negf_sweep.cu; [0] the sum of deg A_nn over the sites)
+// and, when ldos != null, LDOS [e][N].  The buffers are the stream's workspace
+// (allocating and freeing eleven of them per call took 3 to 10 ms).
 int transport_run(negf_tube& t, const std::vector<Pt>& pts, std::vector<double>& red, double* ldos,
                   cudaStream_t s) {
     const int P = (int)pts.size(), M = t.d.num_modes, N = t.N;
     red.assign((size_t)P * 8, 0.0);
     if (P == 0) return NEGF_OK;
-    std::vector<negf::ChainRec> chains;
-    chains.reserve((size_t)P * M + negf::kWarp);
+    negf_tube* one = &t;
+    if (int rc = check_batch_device(&one, 1)) return rc;
+    Workspace* Wp = nullptr;
+    if (int rc = get_workspace(s, &Wp)) return rc;
+    Workspace& W = *Wp;
+    // energy table, then the chains' codes
+    const size_t ib = sizeof(negf::EnergyRec) * P, cb = sizeof(int) * (size_t)P * M;
+    std::vector<char> host(ib + cb);
+    negf::EnergyRec* items = reinterpret_cast<negf::EnergyRec*>(host.data());
+    int* codes = reinterpret_cast<int*>(host.data() + ib);
     for (int e = 0; e < P; ++e) {
-        const double f0 = fermi(pts[e].E - t.mu[0], t.kT[0]).real();
-        const double f1 = fermi(pts[e].E - t.mu[1], t.kT[1]).real();
-        for (int m = 0; m < M; ++m) {
-            negf::ChainRec c{};
-            c.Er = pts[e].E.real();
-            c.Ei = pts[e].E.imag();
-            c.cr = f0;
-            c.ci = f1;
-            c.b0 = c.b1 = 1.0;
-            c.mode = m;
-            chains.push_back(c);
-        }
+        items[e] = {pts[e].E.real(), pts[e].E.imag(), fermi(pts[e].E - t.mu[0], t.kT[0]).real(),
+                    fermi(pts[e].E - t.mu[1], t.kT[1]).real(), 1.0, 1.0};
+        for (int m = 0; m < M; ++m) codes[(size_t)e * M + m] = e << negf::kModeBits | m;
     }
-    while (chains.size() % negf::kWarp) {
-        negf::ChainRec p = chains.back();
-        p.mode = -1;
-        p.cr = p.ci = p.b0 = p.b1 = 0.0;
-        chains.push_back(p);
-    }
-    const int nw = (int)(chains.size() / negf::kWarp);
-    const int nseg = (N + negf::kSeg - 1) / negf::kSeg;
-    const int upw = (nseg + negf::kSegsPerUnit - 1) / negf::kSegsPerUnit;
-    const long long per_warp = negf::rgf_scratch_doubles(N, negf::kRealAxis, 0);
-    std::vector<negf::WarpRec> warps(nw);
-    std::vector<negf::SegUnit> units;
-    for (int w = 0; w < nw; ++w) {
-        warps[w] = negf::WarpRec{};
-        warps[w].tube = 0;
-        warps[w].kind = negf::kRealAxis;
-        warps[w].fp32 = 0;
-        warps[w].ck_off = w * per_warp;
-        for (int s0 = 0; s0 < nseg; s0 += negf::kSegsPerUnit)
-            units.push_back({w, s0, std::min(nseg, s0 + negf::kSegsPerUnit), 0});
-    }
-    const negf::TubeDev td = make_tubedev(t, false);
-    const size_t C = chains.size();
-    DevBuf b_tube, b_chains, b_warps, b_units, b_scratch, b_part, b_cout, b_red, b_site, b_ldos;
-    NEGF_CUDA(b_tube.reserve(sizeof(td)));
-    NEGF_CUDA(b_chains.reserve(C * sizeof(negf::ChainRec)));
-    NEGF_CUDA(b_warps.reserve(warps.size() * sizeof(negf::WarpRec)));
-    NEGF_CUDA(b_units.reserve(units.size() * sizeof(negf::SegUnit)));
-    NEGF_CUDA(b_scratch.reserve((size_t)nw * per_warp * sizeof(double)));
-    NEGF_CUDA(b_part.reserve(units.size() * negf::kWarp * sizeof(double)));
-    NEGF_CUDA(b_cout.reserve(C * 7 * sizeof(double)));
-    NEGF_CUDA(b_red.reserve(red.size() * sizeof(double)));
-    if (ldos) {
-        NEGF_CUDA(b_site.reserve((size_t)N * C * sizeof(double)));
-        NEGF_CUDA(b_ldos.reserve((size_t)P * N * sizeof(double)));
-    }
-    NEGF_CUDA(cudaMemcpyAsync(b_tube.p, &td, sizeof(td), cudaMemcpyHostToDevice, s));
-    NEGF_CUDA(cudaMemcpyAsync(b_chains.p, chains.data(), C * sizeof(negf::ChainRec), cudaMemcpyHostToDevice, s));
-    NEGF_CUDA(cudaMemcpyAsync(b_warps.p, warps.data(), warps.size() * sizeof(negf::WarpRec), cudaMemcpyHostToDevice,
-                              s));
-    NEGF_CUDA(cudaMemcpyAsync(b_units.p, units.data(), units.size() * sizeof(negf::SegUnit),
-                              cudaMemcpyHostToDevice, s));
-    // sites that a chain never reaches keep these zeros (N = 1, 2 probe rules)
-    NEGF_CUDA(cudaMemsetAsync(b_cout.p, 0, C * 7 * sizeof(double), s));
-    NEGF_CUDA(negf::launch_transport(b_tube.as<negf::TubeDev>(), b_chains.as<negf::ChainRec>(),
-                                     b_warps.as<negf::WarpRec>(), nw, b_units.as<negf::SegUnit>(), (int)units.size(),
-                                     b_scratch.p, b_part.as<double>(), b_cout.as<double>(),
-                                     ldos ? b_site.as<double>() : nullptr, (long long)C, P, M, upw,
-                                     b_red.as<double>(), ldos ? b_ldos.as<double>() : nullptr, N, s));
-    NEGF_CUDA(cudaMemcpyAsync(red.data(), b_red.p, red.size() * sizeof(double), cudaMemcpyDeviceToHost, s));
+    NEGF_CUDA(W.trTable.reserve(host.size()));
+    NEGF_CUDA(cudaMemcpyAsync(W.trTable.p, host.data(), host.size(), cudaMemcpyHostToDevice, s));
+    const int K = N < negf::kSweepSeg ? 2 : negf::kSweepSeg;
+    negf::GroupSet gs{};
+    gs.ng = 1;
+    negf::GroupDev& g = gs.g[0];
+    g = make_group(make_tubedev(t, false), W.trTable.as<negf::EnergyRec>(),
+                   reinterpret_cast<const int*>(W.trTable.as<char>() + ib), negf::kRealAxis, P * M, K);
+    g.lanes = 32;
+    g.nsb = (g.nseg + 31) / 32;
+    negf::SweepShape sh{};
+    sh.K = K;
+    sh.scan = scan_better((long long)g.nch * N, N);
+    sh.chains = g.nch;
+    sh.sweep_blocks = 2 * ((g.nch + 31) / 32);
+    sh.scan_threads = std::min(512, (g.nseg + 31) / 32 * 32);
+    if (g.nseg > sh.scan_threads) g.tm_segs = g.nseg;
+    NEGF_CUDA(W.ck.reserve(sizeof(double) * group_state_doubles(g)));
+    NEGF_CUDA(W.cc.reserve(sizeof(double) * (size_t)g.nch * negf::kConst));
+    if (sh.scan) NEGF_CUDA(W.tm.reserve(std::max<size_t>(1, sizeof(double) * 9 * (size_t)g.nch * g.tm_segs)));
+    const size_t nred = (size_t)P * 8, npart = (size_t)P * g.nsb;
+    NEGF_CUDA(W.trOut.reserve(sizeof(double) * (nred + npart)));
+    if (ldos) NEGF_CUDA(W.trLdos.reserve(sizeof(double) * (size_t)P * N));
+    double* d_red = W.trOut.as<double>();
+    // sites that no probe rule reaches keep these zeros
+    NEGF_CUDA(cudaMemsetAsync(d_red, 0, sizeof(double) * nred, s));
+    NEGF_CUDA(negf::launch_transport(gs, sh, M, W.ck.as<double>(), W.cc.as<double>(), W.tm.as<double>(), d_red + nred,
+                                     d_red, ldos ? W.trLdos.as<double>() : nullptr, s));
+    std::vector<double> out(nred + npart);
+    NEGF_CUDA(cudaMemcpyAsync(out.data(), d_red, sizeof(double) * out.size(), cudaMemcpyDeviceToHost, s));
     if (ldos)
-        NEGF_CUDA(cudaMemcpyAsync(ldos, b_ldos.p, (size_t)P * N * sizeof(double), cudaMemcpyDeviceToHost, s));
+        NEGF_CUDA(cudaMemcpyAsync(ldos, W.trLdos.p, sizeof(double) * (size_t)P * N, cudaMemcpyDeviceToHost, s));
+    NEGF_CUDA(cudaEventRecord(W.done, s));
+    W.used = true;
     NEGF_CUDA(cudaStreamSynchronize(s));
+    std::copy(out.begin(), out.begin() + nred, red.begin());
+    for (int e = 0; e < P; ++e) {
+        double sum = 0.0;
+        for (int b = 0; b < g.nsb; ++b) sum += out[nred + (size_t)e * g.nsb + b];
+        red[(size_t)e * 8] = sum;
+    }
     return NEGF_OK;
 }
 

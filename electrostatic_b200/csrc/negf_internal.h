@@ -122,19 +122,12 @@ struct SweepShape {
 };
 cudaError_t launch_sweep(const GroupSet& gs, const SweepShape& sh, double* ck, double* cc, double* tm, double* partial,
                          const int* skip, cudaStream_t s, cudaEvent_t mid);
+// Transport characteristics of one tube (one group of real-axis chains, M per
+// energy in order, lanes = 32): boundary states, then part[e][nsb], red[e][8]
+// and, when not null, ldos[e][N] as described at transport_kernel.
+cudaError_t launch_transport(const GroupSet& gs, const SweepShape& sh, int M, double* ck, double* cc, double* tm,
+                             double* part, double* red, double* ldos, cudaStream_t s);
 
-// RGF launch: pass 1 (one warp per WarpRec, lane = chain: concurrent forward
-// and backward sweeps storing boundary checkpoints) then pass 2 (one warp per
-// SegUnit: independent segments, per-site contributions into partial rows).
-// Transport characteristics of one tube (DOS, transmission, current
-// integrand probes, optional LDOS): pass 1 on real-axis FP64 chains with
-// b0 = b1 = 1 and (cr, ci) = (Re f_0, Re f_1), then the spectral kernel and
-// the per-energy reductions.  d_red: [num_e][8]; d_ldos: [num_e][N] when
-// d_site (scratch of N x chains doubles, stride site_stride) is given.
-cudaError_t launch_transport(const TubeDev* d_tubes, const ChainRec* d_chains, const WarpRec* d_warps, int num_warps,
-                             const SegUnit* d_units, int num_units, void* d_scratch, double* d_part,
-                             double* d_chain_out, double* d_site, long long site_stride, int num_e, int M, int upw,
-                             double* d_red, double* d_ldos, int N, cudaStream_t stream);
 // Real-space ring-block RGF (negf_realspace.cu): leads, chain and reduction
 // for num_e >= 0 energies with coefficients c, Q[r] = sum_e Im(c sum_atoms
 // G_jj) - d_sub[r] (d_sub may be null).  The last num_neq energies are
@@ -205,6 +198,9 @@ struct FusedOrder {
     cudaStream_t side;
     cudaEvent_t fork, join;
 };
+// RGF launch: pass 1 (one warp per WarpRec, lane = chain: concurrent forward
+// and backward sweeps storing boundary checkpoints) then pass 2 (one warp per
+// SegUnit: independent segments, per-site contributions into partial rows).
 cudaError_t launch_rgf(const TubeDev* d_tubes, const ChainRec* d_chains, const WarpRec* d_warps, int num_warps,
                        const SegUnit* d_units, int num_units, double* d_partial, void* d_scratch,
                        int warps_per_block, cudaStream_t stream, cudaEvent_t mid_event,

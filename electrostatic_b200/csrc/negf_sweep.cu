@@ -665,10 +665,12 @@ __device__ __forceinline__ void segment(const SegIn& v, P&& u, F&& site) {
     }
 }
 
-template <int K, bool RA, class P, class F>
+// Chains c0 .. c1 - 1 of one unit: each(v) before a chain's segment, then its
+// site terms.
+template <int K, bool RA, class P, class E, class F>
 __device__ __forceinline__ void seg_loop(const GroupDev& g, SegStage* __restrict__ ring, const double* __restrict__ ck,
                                          const double* __restrict__ cc, int c0, int c1, int sub, int seg,
-                                         P&& u, F&& site) {
+                                         P&& u, E&& each, F&& site) {
     constexpr int NC = RA ? 6 : 4;
     const int lane = threadIdx.x, cpw = 32 / g.lanes;
     const double* __restrict__ con0 = cc + g.cc_off;
@@ -711,6 +713,7 @@ __device__ __forceinline__ void seg_loop(const GroupDev& g, SegStage* __restrict
         // the slot read in the previous iteration is free: every lane has passed the __syncwarp above
         fetch(slot == 0 ? kStages - 1 : slot - 1, c + (kStages - 1) * cpw);
         slot = slot == kStages - 1 ? 0 : slot + 1;
+        each(v);
         segment<K, RA>(v, u, site);
     }
 }
@@ -745,10 +748,11 @@ __global__ void __launch_bounds__(32, 11) seg_kernel(const __grid_constant__ Gro
     }
     auto u = [&](int p) { return usm[p][lane]; };
     auto add = [&](int j, double a, double x, double b, double y) { acc[j] = fma(a, x, fma(b, y, acc[j])); };
+    auto none = [](const SegIn&) {};
     if (g.kind == kRealAxis)
-        seg_loop<K, true>(g, ring, ck, cc, c0, c1, sub, seg, u, add);
+        seg_loop<K, true>(g, ring, ck, cc, c0, c1, sub, seg, u, none, add);
     else
-        seg_loop<K, false>(g, ring, ck, cc, c0, c1, sub, seg, u, add);
+        seg_loop<K, false>(g, ring, ck, cc, c0, c1, sub, seg, u, none, add);
     for (int o = G; o < 32; o <<= 1) {
 #pragma unroll
         for (int j = 0; j < K; ++j) acc[j] += __shfl_xor_sync(kFull, acc[j], o);
@@ -761,17 +765,105 @@ __global__ void __launch_bounds__(32, 11) seg_kernel(const __grid_constant__ Gro
     }
 }
 
+// Transport characteristics (Compute_DensityOfStates, NEGF_Common.cpp:2390-2847;
+// Compute_Current's integrand, :4321-4816) of one tube: block = (energy, block
+// of 32 segments), the warp loops over the energy's M modes (real-axis chains
+// with b0 = b1 = 1, in order; the energy record's cr, ci are Re f_0, Re f_1)
+// and keeps the mode sums of a_n = deg Gamma_0 |G_n0|^2 and b_n = deg Gamma_1
+// |G_n,N-1|^2 of its sites in registers: deg A_nn = a_n + b_n needs no scratch
+// per site and chain.  red[e][8] (zeroed by the caller): [1] Gamma_0 b_0 and [2]
+// Gamma_1 a_{N-1} summed over the modes (transmission from either end), then
+// a_n f_0 + b_n f_1 at n = N/2, else 0, else N-1 (the current's probes,
+// :4684-4714), and at n = N/4, else 3N/4 after N/2 (the charge integrand's,
+// :3467-3496).  part[e][segment block]: sum of a_n + b_n; ldos[e][n] (may be
+// null): (a_n + b_n) / 2 pi.
 template <int K>
-cudaError_t launch_k(const GroupSet& gs, const SweepShape& sh, double* ck, double* cc, double* tm, double* partial,
-                     const int* skip, cudaStream_t s, cudaEvent_t mid) {
+__global__ void __launch_bounds__(32, 8) transport_kernel(const __grid_constant__ GroupSet gs, int M,
+                                                          const double* __restrict__ ck,
+                                                          const double* __restrict__ cc, double* __restrict__ part,
+                                                          double* __restrict__ red, double* __restrict__ ldos) {
+    __shared__ __align__(16) SegStage ring[kStages];
+    __shared__ double2 usm[K / 2][32];
+    const GroupDev& g = group(gs, 0);
+    const int e = blockIdx.x / g.nsb, sb = blockIdx.x % g.nsb;
+    const int lane = threadIdx.x, N = g.N, nseg = g.nseg;
+    const int seg = min(sb * 32 + lane, nseg - 1), n0 = min(seg * K, N - K);
+    const double ig = 1.0 / g.gamma;
+    double A[K], B[K];
+#pragma unroll
+    for (int j = 0; j < K; j += 2) {
+        const double2 v = __ldg(reinterpret_cast<const double2*>(g.U + n0 + j));
+        usm[j / 2][lane] = make_double2(v.x * ig, v.y * ig);
+        A[j] = A[j + 1] = B[j] = B[j + 1] = 0.0;
+    }
+    double g0 = 0.0, g1 = 0.0, t0 = 0.0, t1 = 0.0;
+    seg_loop<K, true>(
+        g, ring, ck, cc, e * M, (e + 1) * M, 0, seg, [&](int p) { return usm[p][lane]; },
+        [&](const SegIn& v) {
+            g0 = v.c0;
+            g1 = v.c1;
+        },
+        [&](int j, double a, double x, double b, double y) {
+            A[j] = fma(a, x, A[j]);
+            B[j] = fma(b, y, B[j]);
+            if (j == 0) t0 = fma(g0, b * y, t0);
+            if (j == K - 1) t1 = fma(g1, a * x, t1);
+        });
+    const bool real = sb * 32 + lane < nseg;
+    const double f0 = g.items[e].cr, f1 = g.items[e].ci;
+    double* __restrict__ out = red + (long long)e * 8;
+    double sum = 0.0;
+#pragma unroll
+    for (int j = 0; j < K; ++j) {
+        const int n = n0 + j;
+        if (!real || n < seg * K) continue;  // the overlapping last segment leaves its neighbour's sites alone
+        const double ab = A[j] + B[j], v = fma(A[j], f0, B[j] * f1);
+        sum += ab;
+        if (ldos) ldos[(long long)e * N + n] = ab / (2.0 * 3.14159265358979323846);
+        if (n == N / 2)
+            out[3] = v;
+        else if (n == 0)
+            out[4] = v;
+        else if (n == N - 1)
+            out[5] = v;
+        if (n != N / 2) {
+            if (n == N / 4)
+                out[6] = v;
+            else if (n == (N * 3) / 4)
+                out[7] = v;
+        }
+    }
+    if (real && seg == 0) out[1] = t0;
+    if (real && seg == nseg - 1) out[2] = t1;
+#pragma unroll
+    for (int o = 16; o >= 1; o >>= 1) sum += __shfl_xor_sync(kFull, sum, o);
+    if (lane == 0) part[blockIdx.x] = sum;
+}
+
+template <int K>
+cudaError_t launch_states(const GroupSet& gs, const SweepShape& sh, double* ck, double* cc, double* tm,
+                          const int* skip, cudaStream_t s) {
     if (sh.scan)
         scan_kernel<K><<<sh.chains, sh.scan_threads, 0, s>>>(gs, ck, cc, tm, skip);
     else
         sweep_kernel<K><<<sh.sweep_blocks, 32, 0, s>>>(gs, ck, cc, skip);
-    cudaError_t e = cudaGetLastError();
+    return cudaGetLastError();
+}
+template <int K>
+cudaError_t launch_k(const GroupSet& gs, const SweepShape& sh, double* ck, double* cc, double* tm, double* partial,
+                     const int* skip, cudaStream_t s, cudaEvent_t mid) {
+    const cudaError_t e = launch_states<K>(gs, sh, ck, cc, tm, skip, s);
     if (e != cudaSuccess) return e;
     if (mid) cudaEventRecord(mid, s);
     seg_kernel<K><<<sh.seg_blocks, 32, 0, s>>>(gs, ck, cc, partial, skip);
+    return cudaGetLastError();
+}
+template <int K>
+cudaError_t launch_transport_k(const GroupSet& gs, const SweepShape& sh, int M, double* ck, double* cc, double* tm,
+                               double* part, double* red, double* ldos, cudaStream_t s) {
+    const cudaError_t e = launch_states<K>(gs, sh, ck, cc, tm, nullptr, s);
+    if (e != cudaSuccess) return e;
+    transport_kernel<K><<<gs.g[0].nch / M * gs.g[0].nsb, 32, 0, s>>>(gs, M, ck, cc, part, red, ldos);
     return cudaGetLastError();
 }
 
@@ -782,6 +874,13 @@ cudaError_t launch_sweep(const GroupSet& gs, const SweepShape& sh, double* ck, d
     if (gs.ng <= 0) return cudaSuccess;
     return sh.K == kSweepSeg ? launch_k<kSweepSeg>(gs, sh, ck, cc, tm, partial, skip, s, mid)
                              : launch_k<2>(gs, sh, ck, cc, tm, partial, skip, s, mid);
+}
+
+cudaError_t launch_transport(const GroupSet& gs, const SweepShape& sh, int M, double* ck, double* cc, double* tm,
+                             double* part, double* red, double* ldos, cudaStream_t s) {
+    if (gs.ng != 1 || M < 1 || gs.g[0].lanes != 32) return cudaErrorInvalidValue;
+    return sh.K == kSweepSeg ? launch_transport_k<kSweepSeg>(gs, sh, M, ck, cc, tm, part, red, ldos, s)
+                             : launch_transport_k<2>(gs, sh, M, ck, cc, tm, part, red, ldos, s);
 }
 
 }  // namespace negf

@@ -111,3 +111,24 @@ def test_many_tubes_read_their_groups_from_memory(oracle):
     for r in refs:
         assert _rel(Q[off:off + len(r)], r) <= FP64_TOL
         off += len(r)
+
+
+# N = 4, 6 (2-site segments), 16, 18, 34 and 516 (33 segments: two blocks of them); on two sites the
+# oracle counts the drain site, which is also N/2, twice
+@pytest.mark.parametrize("tid,cells", [((17, 0), 1), ((13, 2), 3), ((17, 0), 4), ((13, 2), 9), ((13, 2), 17), ((17, 0), 129)])
+def test_transport_segments_match_oracle(oracle, tid, cells):
+    """Density of states, transmission, LDOS, current and its probes at the edges of the segment tiling."""
+    from electrostatic_b200.negf import CNT
+    from electrostatic_b200.workloads import site_potential
+    kw = dict(type_id=tid, num_unitcells=cells, num_modes=3, contact_mu=(0.0, -0.3), contact_T=(300.0, 300.0),
+              noneq_integration_pts=(17, 24), noneq_percent_intercuts=(40.0,), E_zPlus_imag=1e-4)
+    g, o = CNT(**kw), oracle.OracleTube(**kw)
+    U = site_potential(g.site_positions(), 900 + cells, amp=0.2, ramp=0.2)
+    for t in (g, o):
+        t.set_potential(U, (U[0], U[-1]))
+    d, od = g.Compute_DensityOfStates(ldos=True), o.dos(faithful=True, nthreads=8, ldos=True)
+    for key in ("dos", "T", "conductance", "ldos"):
+        assert _rel(d[key], od[key]) <= FP64_TOL, (key, _rel(d[key], od[key]))
+    I, probes, _ = g.Compute_Current(integrand=True)
+    oI, oprobes = o.current(nthreads=8, probes=True)
+    assert _rel(I, oI) <= FP64_TOL and _rel(probes, oprobes) <= FP64_TOL
