@@ -403,13 +403,24 @@ def config3_measure(torch, passes=2, small=False):
     U = site_potential(t.site_positions(), SEED_BASE + 3)
     t.set_potential(U, (U[0], U[-1]))
     Q = torch.zeros(t.num_field_sites, dtype=torch.float64, device="cuda")
-    t.realspace_charge(out=Q)  # warm-up (buffers, lazy loading)
+    # the ring potential given per atom: the ring-block kernels (without it an FP64
+    # tube runs the ring's Fourier modes, timed on its own below)
+    Ua = torch.tensor(np.repeat(U, 13).reshape(-1, 13), device="cuda")
+    t.realspace_charge(out=Q, U_atoms=Ua)  # warm-up (buffers, lazy loading)
     torch.cuda.synchronize()
     t0 = time.perf_counter()
     for _ in range(passes):
-        t.realspace_charge(out=Q)
+        t.realspace_charge(out=Q, U_atoms=Ua)
     torch.cuda.synchronize()
     sec = (time.perf_counter() - t0) / passes
+    Qu = torch.zeros_like(Q)
+    t.realspace_charge(out=Qu)
+    torch.cuda.synchronize()
+    t0 = time.perf_counter()
+    for _ in range(passes):
+        t.realspace_charge(out=Qu)
+    torch.cuda.synchronize()
+    sec_uniform = (time.perf_counter() - t0) / passes
     Qm = t.Solve_NEGF()
     # mixed precision: FP32 chains with tensor-core products away from the real axis
     tm = CNT(**kw, precision="mixed")
@@ -446,7 +457,12 @@ def config3_measure(torch, passes=2, small=False):
                                  "note": "the dense 2m x 2m block algorithm's count (56 n^3 per block update, n = 26: "
                                          "forward inverse + 2 GEMM, backward the same, G_nn inverse), which the "
                                          "ring-corner algebra replaces with 1/14 of the operations (32 m^3 per update)"},
-            "path": "negf_rs_compute_charge (FP64 CUDA cores, one warp per energy, Schur complements on ring corners)",
+            "path": "negf_rs_compute_charge with per-atom potentials (FP64, one warp per energy, Schur complements "
+                    "on ring corners)",
+            "ring_uniform": {"seconds_per_pass": sec_uniform,
+                             "path": "the same call without per-atom potentials: the ring's Fourier modes decouple "
+                                     "the blocks exactly (FP64)",
+                             "max_rel_vs_blocks": float(np.max(np.abs(Qu.cpu().numpy() - Qr)) / np.max(np.abs(Qr)))},
             "max_rel_vs_mode_space_all_modes": float(np.max(np.abs(Qr - Qm)) / np.max(np.abs(Qm))),
             "mixed": {"seconds_per_pass": sec_mixed, "block_updates_per_s": E * K / sec_mixed,
                       "fp32_energies": n32, "fp64_energies": E - n32,
@@ -467,11 +483,12 @@ def config3_biased(torch, kw, U, passes):
         t = CNT(**kb)
         t.set_potential(U, (U[0], U[-1]))
         Q = torch.zeros(t.num_field_sites, dtype=torch.float64, device="cuda")
-        t.realspace_charge(out=Q)
+        Ua = torch.tensor(np.repeat(U, 13).reshape(-1, 13), device="cuda")  # per atom: the ring-block kernels
+        t.realspace_charge(out=Q, U_atoms=Ua)
         torch.cuda.synchronize()
         t0 = time.perf_counter()
         for _ in range(passes):
-            t.realspace_charge(out=Q)
+            t.realspace_charge(out=Q, U_atoms=Ua)
         torch.cuda.synchronize()
         sec = (time.perf_counter() - t0) / passes
         Qm = t.Solve_NEGF()

@@ -134,9 +134,8 @@ cudaError_t launch_transport(const GroupSet& gs, const SweepShape& sh, int M, do
 // real-axis points whose coefficients (b0, b1) = (c_re, c_im) weight the
 // source and drain spectral functions: they add b0 A^L + b1 A^R per ring
 // (FP64).
-// d_flags[e]: 1 = chain in FP32 (tensor-core products), 2 = U = 0 pass
-// (d_Uzero on the atoms and 0 at the contacts; with negated c it subtracts
-// Rho0); otherwise the atom potentials d_Uatoms ([2K][m]) and Uc0, Uc1.
+// d_flags[e]: 1 = chain in FP32 (tensor-core products).  Atom potentials
+// d_Uatoms ([2K][m]), contact potentials Uc0, Uc1.
 // d_corners: num_e * 2 * m^2 complex, d_gL: (num_e - num_neq) * K * m^2
 // complex, d_gLn: num_neq * (2K + 1) * m^2 complex, d_rows: num_e * 2K
 // doubles; *d_status set to 1 on a zero pivot.
@@ -148,8 +147,8 @@ struct RsLeads {
 };
 cudaError_t launch_realspace(int m, int K, double gamma, const double* d_Ere, const double* d_Eim,
                              const double* d_cre, const double* d_cim, int num_e, int num_neq, const int* d_flags,
-                             const double* d_Uatoms, const double* d_Uzero, double Uc0, double Uc1,
-                             const RsLeads& leads, void* d_corners, void* d_gL, void* d_gLn, double* d_rows,
+                             const double* d_Uatoms, double Uc0, double Uc1, const RsLeads& leads, void* d_corners,
+                             void* d_gL, void* d_gLn, double* d_rows,
                              double* d_Q, const double* d_sub, int* d_status, cudaStream_t stream);
 cudaError_t rs_expand(const double* d_U, int N, int m, double* d_Ua, cudaStream_t stream);
 // Self-test of the real-space tile primitives for m in {4, 13, 16}: which 2 / 3

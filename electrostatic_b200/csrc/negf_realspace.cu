@@ -42,8 +42,9 @@
 //                    ring corners: ring sums of the contact spectral
 //                    functions (the non-equilibrium term, FP64);
 //   rs_reduce_kernel sum over energies per ring in a fixed order (Kahan).
-// The energies of the U = 0 pass (Rho0) run in the same launches with
-// negated coefficients, so one reduction gives the induced charge.
+// The U = 0 pass (Rho0) and, in FP64, ring-uniform potentials do not come
+// here: the ring's Fourier modes decouple them (ring_modes_charge in
+// negf_api.cpp).
 // Inversions: Gauss-Jordan on [S | I] (lane = column), on the diagonal
 // pivots with a fall-back to partial pivoting when a pivot is small.
 //
@@ -456,9 +457,8 @@ __device__ __forceinline__ void cp_async(T* smem_dst, const T* gsrc) {
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
-// Energy flags: kRsFP32 runs the chain in FP32, kRsZeroU takes U = 0 on the
-// atoms and the contacts (the Rho0 pass).
-constexpr int kRsFP32 = 1, kRsZeroU = 2;
+// Energy flags: kRsFP32 runs the chain in FP32.
+constexpr int kRsFP32 = 1;
 
 // Lead kernel: block e -> energy e, lanes 0-15 the left lead, 16-31 the
 // right one.  A lead is uniform (the contact potential u on every atom), so
@@ -480,8 +480,8 @@ constexpr int kRsFP32 = 1, kRsZeroU = 2;
 // corners[e][side] = g_surface[s][s] (m x m, row-major).
 template <int m>
 __global__ void __launch_bounds__(32) rs_lead_kernel(double gamma, const double* __restrict__ Ere,
-                                                     const double* __restrict__ Eim, int num_e,
-                                                     const int* __restrict__ flags, double Uc0, double Uc1,
+                                                     const double* __restrict__ Eim, int num_e, double Uc0,
+                                                     double Uc1,
                                                      int use_decimation, int dec_layers, int dec_iters,
                                                      cplxd* __restrict__ corners) {
     __shared__ cd sk[2][kMaxM], cdiff[2][kMaxM];
@@ -489,7 +489,7 @@ __global__ void __launch_bounds__(32) rs_lead_kernel(double gamma, const double*
     const int e = blockIdx.x;
     if (e >= num_e) return;
     const int side = lane >> 4, k = lane & 15;
-    const double u = (flags[e] & kRsZeroU) ? 0.0 : (side == 0 ? Uc0 : Uc1);
+    const double u = side == 0 ? Uc0 : Uc1;
     const cd EmU = {Ere[e] - u, Eim[e]};
     if (k < m) {
         const double beta = 2.0 * gamma * cospi((double)k / m);
@@ -794,8 +794,7 @@ __device__ __forceinline__ bool rs_chain(int K, R gamma, cplx<R> E, cplxd cc, co
     return ok;
 }
 
-// Chain kernel: warp e -> energy e in the precision and with the potentials
-// its flags give (Uatoms, or Uzero for the U = 0 pass).
+// Chain kernel: warp e -> energy e in the precision its flags give.
 // gX: [num_e][K][m*m] FP64-complex slots (an FP32 chain uses the first half
 // of its slot); rows: [num_e][N].
 template <int m>
@@ -804,8 +803,7 @@ __global__ void __launch_bounds__(32, 16) rs_chain_kernel(int K, double gamma, c
                                                           const double* __restrict__ cre,
                                                           const double* __restrict__ cim, int num_e,
                                                           const int* __restrict__ flags,
-                                                          const double* __restrict__ Uatoms,
-                                                          const double* __restrict__ Uzero,
+                                                          const double* __restrict__ Ua,
                                                           const cplxd* __restrict__ corners, cplxd* __restrict__ gX,
                                                           double* __restrict__ rows, int* __restrict__ status) {
     extern __shared__ cplxd sh[];
@@ -814,7 +812,6 @@ __global__ void __launch_bounds__(32, 16) rs_chain_kernel(int K, double gamma, c
     if (e >= num_e) return;
     constexpr int mm2 = m * m;
     const int fl = flags[e];
-    const double* __restrict__ Ua = (fl & kRsZeroU) ? Uzero : Uatoms;
     const cplxd* sL = corners + (size_t)e * 2 * mm2;
     const cplxd* sR = sL + mm2;
     cplxd* myX = gX + (size_t)e * K * mm2;
@@ -964,9 +961,8 @@ namespace {
 template <int m>
 cudaError_t launch_rs(int K, double gamma, const double* d_Ere, const double* d_Eim, const double* d_cre,
                       const double* d_cim, int num_e, int num_neq, const int* d_flags, const double* d_Uatoms,
-                      const double* d_Uzero, double Uc0, double Uc1, const RsLeads& leads, void* d_corners,
-                      void* d_gL,
-                      void* d_gLn, double* d_rows, double* d_Q, const double* d_sub, int* d_status,
+                      double Uc0, double Uc1, const RsLeads& leads, void* d_corners, void* d_gL, void* d_gLn,
+                      double* d_rows, double* d_Q, const double* d_sub, int* d_status,
                       cudaStream_t stream) {
     cudaError_t e = cudaFuncSetAttribute(rs_chain_kernel<m>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)rs_chain_smem_bytes(m));
@@ -976,7 +972,7 @@ cudaError_t launch_rs(int K, double gamma, const double* d_Ere, const double* d_
     if (e != cudaSuccess) return e;
     const int num_eq = num_e - num_neq;
     if (num_e > 0) {
-        rs_lead_kernel<m><<<num_e, 32, 0, stream>>>(gamma, d_Ere, d_Eim, num_e, d_flags, Uc0, Uc1,
+        rs_lead_kernel<m><<<num_e, 32, 0, stream>>>(gamma, d_Ere, d_Eim, num_e, Uc0, Uc1,
                                                     leads.use_decimation, leads.dec_layers, leads.dec_iters,
                                                     static_cast<cplxd*>(d_corners));
         e = cudaGetLastError();
@@ -992,7 +988,7 @@ cudaError_t launch_rs(int K, double gamma, const double* d_Ere, const double* d_
     }
     if (num_eq > 0) {
         rs_chain_kernel<m><<<num_eq, 32, rs_chain_smem_bytes(m), stream>>>(
-            K, gamma, d_Ere, d_Eim, d_cre, d_cim, num_eq, d_flags, d_Uatoms, d_Uzero,
+            K, gamma, d_Ere, d_Eim, d_cre, d_cim, num_eq, d_flags, d_Uatoms,
             static_cast<const cplxd*>(d_corners), static_cast<cplxd*>(d_gL), d_rows, d_status);
         e = cudaGetLastError();
         if (e != cudaSuccess) return e;
@@ -1005,14 +1001,13 @@ cudaError_t launch_rs(int K, double gamma, const double* d_Ere, const double* d_
 
 cudaError_t launch_realspace(int m, int K, double gamma, const double* d_Ere, const double* d_Eim,
                              const double* d_cre, const double* d_cim, int num_e, int num_neq, const int* d_flags,
-                             const double* d_Uatoms, const double* d_Uzero, double Uc0, double Uc1,
-                             const RsLeads& leads,
+                             const double* d_Uatoms, double Uc0, double Uc1, const RsLeads& leads,
                              void* d_corners, void* d_gL, void* d_gLn, double* d_rows, double* d_Q,
                              const double* d_sub, int* d_status, cudaStream_t stream) {
     if (num_e < 0 || num_neq < 0 || num_neq > num_e || K < 1) return cudaErrorInvalidValue;
 #define RS_CASE(M)                                                                                                 \
     case M:                                                                                                        \
-        return launch_rs<M>(K, gamma, d_Ere, d_Eim, d_cre, d_cim, num_e, num_neq, d_flags, d_Uatoms, d_Uzero, Uc0,  \
+        return launch_rs<M>(K, gamma, d_Ere, d_Eim, d_cre, d_cim, num_e, num_neq, d_flags, d_Uatoms, Uc0,           \
                             Uc1, leads, d_corners, d_gL, d_gLn, d_rows, d_Q, d_sub, d_status, stream);
     switch (m) {
         RS_CASE(1) RS_CASE(2) RS_CASE(3) RS_CASE(4) RS_CASE(5) RS_CASE(6) RS_CASE(7) RS_CASE(8)

@@ -279,7 +279,9 @@ int negf_set_timing(int enable);
  * the contact ring's atoms) weighted by the mode-space coefficients, in
  * FP64.  d_Uatoms (device, [N][m]) gives per-atom potentials; null uses the
  * tube's ring potential on every atom, in which case the result equals the
- * mode-space charge with all m//2 + 1 distinct modes.  Tubes in mixed
+ * mode-space charge with all m//2 + 1 distinct modes; FP64 tubes then run
+ * those modes (the ring's Fourier vectors decouple the blocks exactly), as
+ * the U = 0 pass does for every tube.  Tubes in mixed
  * precision run the contour and pole chains at least mixed_fp64_band above
  * the real axis in FP32 (m x m products on the tensor cores in TF32 with a
  * high/remainder split, the complex product in three real products); the

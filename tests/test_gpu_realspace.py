@@ -196,3 +196,27 @@ def test_realspace_decimation_leads_equal_mode_space(bias):
     Qr = g.realspace_charge()
     Qm = g.Solve_NEGF()
     assert _rel(Qr, Qm) <= TOL, _rel(Qr, Qm)
+
+
+@pytest.mark.parametrize("bias", [False, True])
+@pytest.mark.parametrize("m,cells", [(1, 3), (2, 2), (3, 5), (6, 4), (8, 3), (12, 2), (13, 6), (16, 9)])
+def test_ring_modes_equal_ring_blocks(m, cells, bias):
+    """A ring-uniform potential in FP64 runs as the ring's Fourier modes; given
+    per atom, the same potential runs as ring blocks.  Both are the same charge
+    (odd and even rings, m divisible by 3 and 6, where several modes share a
+    band gap, and the mode of even rings whose hopping vanishes)."""
+    import torch
+    from electrostatic_b200.negf import CNT
+    kw = dict(_bias_kw(m, cells) if bias else _eq_kw(m, cells, num_modes=1))
+    g = CNT(**kw)
+    y = g.site_positions()
+    U = 0.15 * np.cos(2.0 * y) + 0.1 * (y - y[0]) / (y[-1] - y[0])
+    g.set_potential(U, (U[0], U[-1]))
+    Qm = g.realspace_charge()
+    Qb = g.realspace_charge(U_atoms=torch.tensor(np.repeat(U, m).reshape(-1, m), device="cuda"))
+    assert _rel(Qm, Qb) <= TOL, _rel(Qm, Qb)
+    # changed contacts: the modes of the new paths
+    g.set_contact_mu((-0.2, -0.6) if bias else (-0.7, -0.7))
+    Qm = g.realspace_charge()
+    Qb = g.realspace_charge(U_atoms=torch.tensor(np.repeat(U, m).reshape(-1, m), device="cuda"))
+    assert _rel(Qm, Qb) <= TOL, _rel(Qm, Qb)
