@@ -275,7 +275,7 @@ struct Workspace {
     cudaStream_t side = nullptr;                 // the FP32 warps of the fused schedule
     cudaEvent_t fork = nullptr, join = nullptr;  // around them
     // real-space pass (negf_rs_compute_charge)
-    DevBuf rsE, rsFlags, rsUa, rsCorners, rsGL, rsGLn, rsRows, rsStatus;
+    DevBuf rsE, rsUa, rsCorners, rsGL, rsGLn, rsRows, rsStatus;
     // cached chain table
     std::vector<long long> key_serials;
     std::vector<int> key_versions;
@@ -296,7 +296,7 @@ struct Workspace {
         if (join) cudaEventDestroy(join);
         if (side) cudaStreamDestroy(side);
         DevBuf* bufs[] = {&tubes, &chains, &warps, &rts,  &units, &partial,   &scratch, &qbuf,   &pieces,
-                          &ck,    &cc,   &tm,    &groups, &trTable, &trOut, &trLdos, &order, &rsE,    &rsFlags, &rsUa, &rsCorners, &rsGL,    &rsGLn,  &rsRows,
+                          &ck,    &cc,   &tm,    &groups, &trTable, &trOut, &trLdos, &order, &rsE,    &rsUa, &rsCorners, &rsGL,    &rsGLn,  &rsRows,
                           &rsStatus};
         for (DevBuf* b : bufs) {
             if (b->p) cudaFree(b->p);
@@ -2628,7 +2628,6 @@ int negf_rs_compute_charge(negf_tube* t, const double* d_Uatoms, double* d_Q, vo
     // first in the launch, the real-axis points last.
     struct RsE {
         double Er, Ei, cr, ci;
-        int flags;
     };
     std::vector<RsE> e64, e32, eneq;
     const bool mixed = t->d.precision == NEGF_PREC_MIXED;
@@ -2636,11 +2635,11 @@ int negf_rs_compute_charge(negf_tube* t, const double* d_Uatoms, double* d_Q, vo
     for (int idx = 0; idx < neq; ++idx) {
         const Item it = pass_item(*t, false, idx);
         if (it.kind == negf::kRealAxis) {
-            eneq.push_back({it.E.real(), it.E.imag(), it.b0, it.b1, 0});
+            eneq.push_back({it.E.real(), it.E.imag(), it.b0, it.b1});
             continue;
         }
         const bool fp32 = mixed && std::fabs(it.E.imag()) >= t->d.mixed_fp64_band;
-        (fp32 ? e32 : e64).push_back({it.E.real(), it.E.imag(), it.c.real(), it.c.imag(), fp32 ? 1 : 0});
+        (fp32 ? e32 : e64).push_back({it.E.real(), it.E.imag(), it.c.real(), it.c.imag()});
     }
     std::vector<RsE> all(e64);
     all.insert(all.end(), e32.begin(), e32.end());
@@ -2649,14 +2648,13 @@ int negf_rs_compute_charge(negf_tube* t, const double* d_Uatoms, double* d_Q, vo
     const size_t mm = (size_t)m * m;
     const size_t pe = (size_t)std::max(P, 1);
     // grow-only buffers of this (device, stream) kept across calls
-    DevBuf &bE = Wp->rsE, &bFlags = Wp->rsFlags, &bUa = Wp->rsUa, &bCorners = Wp->rsCorners,
-           &bGL = Wp->rsGL, &bGLn = Wp->rsGLn, &bRows = Wp->rsRows, &bStatus = Wp->rsStatus;
+    DevBuf &bE = Wp->rsE, &bUa = Wp->rsUa, &bCorners = Wp->rsCorners, &bGL = Wp->rsGL,
+           &bGLn = Wp->rsGLn, &bRows = Wp->rsRows, &bStatus = Wp->rsStatus;
     NEGF_CUDA(bE.reserve(sizeof(double) * 4 * pe));
-    NEGF_CUDA(bFlags.reserve(sizeof(int) * pe));
     NEGF_CUDA(bUa.reserve(sizeof(double) * (size_t)N * m));
     NEGF_CUDA(bCorners.reserve(16 * 2 * mm * pe));
     NEGF_CUDA(bGL.reserve(16 * mm * K * (size_t)std::max(P - Pn, 1)));
-    if (Pn > 0) NEGF_CUDA(bGLn.reserve(16 * mm * (2 * (size_t)K + 1) * Pn));
+    if (Pn > 0) NEGF_CUDA(bGLn.reserve(16 * mm * 2 * (size_t)K * Pn));
     NEGF_CUDA(bRows.reserve(sizeof(double) * (size_t)N * pe));
     NEGF_CUDA(bStatus.reserve(sizeof(int)));
     NEGF_CUDA(cudaMemsetAsync(bStatus.p, 0, sizeof(int), s));
@@ -2665,32 +2663,23 @@ int negf_rs_compute_charge(negf_tube* t, const double* d_Uatoms, double* d_Q, vo
     leads.dec_layers = t->d.decimation_layers;
     leads.dec_iters = t->d.decimation_max_iter + 2;
     double* dE = bE.as<double>();
-    auto upload = [&](const std::vector<RsE>& v, std::vector<double>& host, std::vector<int>& hflags) -> int {
-        const int n = (int)v.size();
-        host.assign(4 * (size_t)std::max(n, 1), 0.0);
-        hflags.assign((size_t)std::max(n, 1), 0);
-        for (int i = 0; i < n; ++i) {
-            host[i] = v[i].Er;
-            host[n + i] = v[i].Ei;
-            host[2 * n + i] = v[i].cr;
-            host[3 * n + i] = v[i].ci;
-            hflags[i] = v[i].flags;
-        }
-        NEGF_CUDA(cudaMemcpyAsync(dE, host.data(), sizeof(double) * 4 * n, cudaMemcpyHostToDevice, s));
-        NEGF_CUDA(cudaMemcpyAsync(bFlags.p, hflags.data(), sizeof(int) * n, cudaMemcpyHostToDevice, s));
-        return NEGF_OK;
-    };
-    std::vector<double> host1;
-    std::vector<int> hflags1;
     const double* Ua = d_Uatoms;
     if (!Ua) {
         NEGF_CUDA(negf::rs_expand(t->d_U, N, m, bUa.as<double>(), s));
         Ua = bUa.as<double>();
     }
-    if (int rc = upload(all, host1, hflags1)) return rc;
-    NEGF_CUDA(negf::launch_realspace(m, K, t->d.gamma, dE, dE + P, dE + 2 * P, dE + 3 * P, P, Pn, bFlags.as<int>(),
-                                     Ua, t->Uc[0], t->Uc[1], leads, bCorners.p, bGL.p, bGLn.p,
-                                     bRows.as<double>(), d_Q, t->d_rs_rho0, bStatus.as<int>(), s));
+    std::vector<double> host(4 * pe);
+    for (int i = 0; i < P; ++i) {
+        host[i] = all[i].Er;
+        host[P + i] = all[i].Ei;
+        host[2 * P + i] = all[i].cr;
+        host[3 * P + i] = all[i].ci;
+    }
+    NEGF_CUDA(cudaMemcpyAsync(dE, host.data(), sizeof(double) * 4 * P, cudaMemcpyHostToDevice, s));
+    const negf::RsParallel par{Wp->side, Wp->fork, Wp->join};
+    NEGF_CUDA(negf::launch_realspace(m, K, t->d.gamma, dE, dE + P, dE + 2 * P, dE + 3 * P, P, (int)e64.size(), Pn, par,
+                                     Ua, t->Uc[0], t->Uc[1], leads, bCorners.p, bGL.p, bGLn.p, bRows.as<double>(),
+                                     d_Q, t->d_rs_rho0, bStatus.as<int>(), s));
     int status = 0;
     NEGF_CUDA(cudaMemcpyAsync(&status, bStatus.p, sizeof(int), cudaMemcpyDeviceToHost, s));
     NEGF_CUDA(cudaEventRecord(Wp->done, s));

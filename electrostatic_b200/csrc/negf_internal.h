@@ -128,16 +128,16 @@ cudaError_t launch_sweep(const GroupSet& gs, const SweepShape& sh, double* ck, d
 cudaError_t launch_transport(const GroupSet& gs, const SweepShape& sh, int M, double* ck, double* cc, double* tm,
                              double* part, double* red, double* ldos, cudaStream_t s);
 
-// Real-space ring-block RGF (negf_realspace.cu): leads, chain and reduction
+// Real-space ring-block RGF (negf_realspace.cu): leads, chains and reduction
 // for num_e >= 0 energies with coefficients c, Q[r] = sum_e Im(c sum_atoms
-// G_jj) - d_sub[r] (d_sub may be null).  The last num_neq energies are
-// real-axis points whose coefficients (b0, b1) = (c_re, c_im) weight the
-// source and drain spectral functions: they add b0 A^L + b1 A^R per ring
-// (FP64).
-// d_flags[e]: 1 = chain in FP32 (tensor-core products).  Atom potentials
-// d_Uatoms ([2K][m]), contact potentials Uc0, Uc1.
+// G_jj) - d_sub[r] (d_sub may be null).  The first num_64 energies run in
+// FP64, the last num_neq are real-axis points whose coefficients (b0, b1) =
+// (c_re, c_im) weight the source and drain spectral functions: they add b0 A^L
+// + b1 A^R per ring (FP64); those between run in FP32 (tensor-core products),
+// on par.side between the events when there are others.  Atom potentials
+// d_Uatoms ([2K][m]), contact potentials Uc0, Uc1; K >= 2.
 // d_corners: num_e * 2 * m^2 complex, d_gL: (num_e - num_neq) * K * m^2
-// complex, d_gLn: num_neq * (2K + 1) * m^2 complex, d_rows: num_e * 2K
+// complex, d_gLn: num_neq * 2K * m^2 complex, d_rows: num_e * 2K
 // doubles; *d_status set to 1 on a zero pivot.
 // Leads of the real-space pass: the mode chains' surface values by the
 // analytic formula, or by the reference's decimation (dec_layers layers,
@@ -145,10 +145,14 @@ cudaError_t launch_transport(const GroupSet& gs, const SweepShape& sh, int M, do
 struct RsLeads {
     int use_decimation = 0, dec_layers = 10, dec_iters = 32;
 };
+struct RsParallel {
+    cudaStream_t side;
+    cudaEvent_t fork, join;
+};
 cudaError_t launch_realspace(int m, int K, double gamma, const double* d_Ere, const double* d_Eim,
-                             const double* d_cre, const double* d_cim, int num_e, int num_neq, const int* d_flags,
-                             const double* d_Uatoms, double Uc0, double Uc1, const RsLeads& leads, void* d_corners,
-                             void* d_gL, void* d_gLn, double* d_rows,
+                             const double* d_cre, const double* d_cim, int num_e, int num_64, int num_neq,
+                             const RsParallel& par, const double* d_Uatoms, double Uc0, double Uc1,
+                             const RsLeads& leads, void* d_corners, void* d_gL, void* d_gLn, double* d_rows,
                              double* d_Q, const double* d_sub, int* d_status, cudaStream_t stream);
 cudaError_t rs_expand(const double* d_U, int N, int m, double* d_Ua, cudaStream_t stream);
 // Self-test of the real-space tile primitives for m in {4, 13, 16}: which 2 / 3

@@ -19,10 +19,10 @@
 //   backward G_kk = g_L + gamma^2 g_L[:, b] G_{k+1}[a][a] g_L[b, :] gives
 //            G[a][a] = X + gamma^4 X (Y G' Y^T) X  and
 //            tr G[b][b] = tr g_L[b][b] + gamma^2 tr(g_L[b][b] G' g_L[b][b])
-//            with G' = G_{k+1}[a][a]: three m x m products per block.  The
-//            right lead enters through G_K[a][a] = (I - gamma^2 s_R
-//            g_L[b][b])^-1 s_R of its first ring.
-// One block update costs one m x m inversion and three m x m products
+//            with G' = G_{k+1}[a][a]: three m x m products per block (two in
+//            FP64, see rs_side).  The right lead enters through G_K[a][a] =
+//            (I - gamma^2 s_R g_L[b][b])^-1 s_R of its first ring.
+// One block update costs one m x m inversion and two or three m x m products
 // instead of three 2m x 2m inversions (about 10x fewer operations).
 //
 // Leads: a lead is uniform (the contact potential on every atom), so the
@@ -30,23 +30,25 @@
 // the ring corner of its surface Green's function is the circulant of the
 // per-mode surface values (rs_lead_kernel).
 
-// Kernels (one warp per energy; m x m complex tiles in shared memory,
-// row-major; m x m products on the FP64 tensor cores, mma.sync m8n8k4, with
-// the results staged in registers so that outputs may alias inputs):
+// Kernels (m x m complex tiles in shared memory, row-major; m x m products on
+// the FP64 tensor cores, mma.sync m8n8k4, with the results staged in registers
+// so that outputs may alias inputs):
 //   rs_lead_kernel   both lead corners s_L = g[b][b], s_R = g[a][a] (ring
 //                    Fourier modes, per-mode surface values);
-//   rs_chain_kernel  forward sweep (X_k to global scratch), backward sweep
-//                    with the ring sums of c G_jj written per energy;
-//   rs_chain_neq_kernel  the same sweeps at a real-axis energy of a biased
-//                    tube, carrying the source and drain columns of G in
-//                    ring corners: ring sums of the contact spectral
-//                    functions (the non-equilibrium term, FP64);
+//   rs_pair_kernel   an energy's FP64 chain by two warps from its two ends:
+//                    forward sweeps (X_k to global scratch), backward sweeps with
+//                    the ring sums of c G_jj written per energy; at a real-axis
+//                    energy of a biased tube the sweeps carry the source and
+//                    drain columns of G in ring corners: ring sums of the contact
+//                    spectral functions (the non-equilibrium term);
+//   rs_chain_kernel  an energy's FP32 chain of mixed mode, one warp;
 //   rs_reduce_kernel sum over energies per ring in a fixed order (Kahan).
 // The U = 0 pass (Rho0) and, in FP64, ring-uniform potentials do not come
 // here: the ring's Fourier modes decouple them (ring_modes_charge in
 // negf_api.cpp).
-// Inversions: Gauss-Jordan on [S | I] (lane = column), on the diagonal
-// pivots with a fall-back to partial pivoting when a pivot is small.
+// Inversions: FP64 blocks by symmetric sweeps on 2 x 2 pivots, the others by
+// Gauss-Jordan on [S | I] (lane = column); on the diagonal pivots with a
+// fall-back to partial pivoting when a pivot is small.
 //
 // Mixed precision: the chain of an energy runs in FP32 when its tube is in
 // mixed mode and the point lies at least mixed_fp64_band above the real axis
@@ -56,8 +58,8 @@
 // split into a TF32 high part and a TF32 remainder (three products per
 // pair, about FP32 accuracy) and the complex product in the three-multiply
 // form Re = ArBr - AiBi, Im = (Ar + Ai)(Br + Bi) - ArBr - AiBi; the
-// inversion runs on the FP32 cores.  One launch holds both precisions (the
-// FP64 energies first).
+// inversion runs on the FP32 cores.  The FP32 chains run beside the FP64 ones,
+// on a side stream.
 
 #include "negf_internal.h"
 
@@ -162,16 +164,21 @@ __device__ __forceinline__ void dmma(double (&d)[2], double a, double b) {
         : "d"(a), "d"(b));
 }
 
-// C = s op(A) op(B) (+ D when ADD) in FP64 on the tensor cores: the m x m
-// tiles are read as zero-padded 16 x 16 operands (2 x 2 output tiles of
-// 8 x 8, k in steps of 4), complex products in the three-multiply form
-// Re = ArBr - AiBi, Im = (Ar + Ai)(Br + Bi) - ArBr - AiBi.  C may alias any
-// operand: the products are staged in registers.
-template <int m, bool TA, bool TB, bool ADD>
-__device__ __forceinline__ void mm(Mat<m, double> C, Mat<m, double> A, Mat<m, double> B, Mat<m, double> D, double s,
-                                   int lane) {
+// op(A) op(B) of m x m tiles in FP64 on the tensor cores, the entries handed to
+// f(r, c, v, valid, off) by the lanes that hold them: 2 x 2 output tiles of 8 x
+// 8 (rows and columns past m are clamped duplicates, valid = false), k in steps
+// of 4, complex products in the three-multiply form Re = ArBr - AiBi, Im = (Ar +
+// Ai)(Br + Bi) - ArBr - AiBi.  One or two indices left over by the steps of 4
+// are rank-one updates on the FP64 cores: 60 issue cycles each at 2 x 2 tiles
+// where a padded step takes 192 (an m8n8k4 runs 16 cycles: the tensor cores
+// have the FP64 cores' rate here).  SYM: the product is symmetric, and the tile
+// above the diagonal is left out: the entries of tile (1, 0) come with off =
+// true and stand for (c, r) too.  f may overwrite A and B.
+template <int m, bool TA, bool TB, bool SYM, class F>
+__device__ __forceinline__ void mm_each(Mat<m, double> A, Mat<m, double> B, int lane, F&& f) {
     const int g = lane >> 2, t = lane & 3;
     constexpr int NT = (m + 7) / 8;  // 8 x 8 output tiles per dimension
+    constexpr int KD = m % 4 == 3 ? m + 1 : m - (m % 4 <= 2 ? m % 4 : 0);
     double p1[NT][NT][2], p2[NT][NT][2], p3[NT][NT][2];  // Ar Br, Ai Bi, (Ar + Ai)(Br + Bi)
 #pragma unroll
     for (int i = 0; i < NT; ++i)
@@ -180,44 +187,76 @@ __device__ __forceinline__ void mm(Mat<m, double> C, Mat<m, double> A, Mat<m, do
 #pragma unroll
             for (int q = 0; q < 2; ++q) p1[i][j][q] = p2[i][j][q] = p3[i][j][q] = 0.0;
 #pragma unroll
-    for (int k0 = 0; k0 < m; k0 += 4) {
-        const int k = k0 + t;
+    for (int k0 = 0; k0 < KD; k0 += 4) {
+        const int k = min(k0 + t, m - 1);
         cplxd a[NT], b[NT];
 #pragma unroll
         for (int i = 0; i < NT; ++i) {
-            const int r = 8 * i + g;
-            a[i] = cmk(0.0, 0.0);
-            if (r < m && k < m) a[i] = TA ? A.at(k, r) : A.at(r, k);
-            b[i] = cmk(0.0, 0.0);
-            if (k < m && r < m) b[i] = TB ? B.at(r, k) : B.at(k, r);  // column 8 i + g of B
+            const int r = min(8 * i + g, m - 1);
+            a[i] = TA ? A.at(k, r) : A.at(r, k);
+            b[i] = TB ? B.at(r, k) : B.at(k, r);  // column 8 i + g of B
+            if (k0 + 4 > m && k0 + t >= m) a[i] = b[i] = cmk(0.0, 0.0);
         }
 #pragma unroll
         for (int i = 0; i < NT; ++i) {
             const double as = a[i].x + a[i].y;
 #pragma unroll
-            for (int j = 0; j < NT; ++j) {
+            for (int j = 0; j < (SYM ? i + 1 : NT); ++j) {
                 dmma(p1[i][j], a[i].x, b[j].x);
                 dmma(p2[i][j], a[i].y, b[j].y);
                 dmma(p3[i][j], as, b[j].x + b[j].y);
             }
         }
     }
+#pragma unroll
+    for (int k = KD; k < m; ++k) {
+        cplxd a[NT], b[NT][2];
+#pragma unroll
+        for (int i = 0; i < NT; ++i) {
+            const int r = min(8 * i + g, m - 1);
+            a[i] = TA ? A.at(k, r) : A.at(r, k);
+#pragma unroll
+            for (int q = 0; q < 2; ++q) {
+                const int c = min(8 * i + 2 * t + q, m - 1);
+                b[i][q] = TB ? B.at(c, k) : B.at(k, c);
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < NT; ++i) {
+            const double as = a[i].x + a[i].y;
+#pragma unroll
+            for (int j = 0; j < (SYM ? i + 1 : NT); ++j)
+#pragma unroll
+                for (int q = 0; q < 2; ++q) {
+                    p1[i][j][q] = fma(a[i].x, b[j][q].x, p1[i][j][q]);
+                    p2[i][j][q] = fma(a[i].y, b[j][q].y, p2[i][j][q]);
+                    p3[i][j][q] = fma(as, b[j][q].x + b[j][q].y, p3[i][j][q]);
+                }
+        }
+    }
     __syncwarp();
 #pragma unroll
     for (int i = 0; i < NT; ++i)
 #pragma unroll
-        for (int j = 0; j < NT; ++j)
+        for (int j = 0; j < (SYM ? i + 1 : NT); ++j)
 #pragma unroll
             for (int q = 0; q < 2; ++q) {
                 const int r = 8 * i + g, c = 8 * j + 2 * t + q;
-                if (r < m && c < m) {
-                    const double re = p1[i][j][q] - p2[i][j][q], im = p3[i][j][q] - p1[i][j][q] - p2[i][j][q];
-                    cplxd v = cmk(re * s, im * s);
-                    if (ADD) v = cadd(v, D.at(r, c));
-                    C.at(r, c) = v;
-                }
+                const double re = p1[i][j][q] - p2[i][j][q], im = p3[i][j][q] - p1[i][j][q] - p2[i][j][q];
+                f(min(r, m - 1), min(c, m - 1), cmk(re, im), r < m && c < m, SYM && i != j);
             }
     __syncwarp();
+}
+
+// C = s op(A) op(B) (+ D when ADD); C may alias any operand.
+template <int m, bool TA, bool TB, bool ADD>
+__device__ __forceinline__ void mm(Mat<m, double> C, Mat<m, double> A, Mat<m, double> B, Mat<m, double> D, double s,
+                                   int lane) {
+    mm_each<m, TA, TB, false>(A, B, lane, [&](int r, int c, cplxd v, bool valid, bool) {
+        v = cscale(v, s);
+        if (ADD) v = cadd(v, D.at(r, c));
+        if (valid) C.at(r, c) = v;
+    });
 }
 
 // TF32 tensor-core product D += A B of a 16 x 8 x 8 tile (mma.sync
@@ -434,6 +473,94 @@ __device__ __forceinline__ bool invert(Mat<m, R> out, Mat<m, R> S, cplx<R>* buf,
     return true;
 }
 
+// Row layout of the FP64 chains: two lanes per row r = lane / 2, the pairs of
+// columns (2q, 2q + 1) on the lanes in turn: lane parity h holds column col(h, j)
+// as its j-th (columns past m - 1 are padding, whose values go nowhere).
+template <int m>
+struct RowLay {
+    static constexpr int H = 2 * (m / 4) + (m % 4 < 2 ? m % 4 : 2);
+    static constexpr int kBuf = 6 * kMaxM;  // column pairs of the sweeps: three buffers
+    __device__ static __forceinline__ int col(int h, int j) { return 4 * (j >> 1) + 2 * h + (j & 1); }
+};
+
+// a = -S of a complex symmetric m x m matrix S in the row layout; S^-1 in place,
+// by symmetric sweeps on 2 x 2 diagonal blocks B (a 1 x 1 one at the end of an
+// odd m).  A sweep keeps the matrix symmetric, so the block's rows are its
+// columns: with u_r the two entries of row r under B and t_r = u_r B^-1,
+//   a_rc -= t_r . u_c,  a_r,block = t_r   (rows outside the block)
+// and the same with u_r = -e_r on a zeroed row for the block's own rows.  Only the
+// two columns travel through shared memory (one __syncwarp per block; buf: three
+// buffers, as the rest of a sweep overlaps the next one's start), and the next
+// block's columns are updated first.  Bound by the chain store - load -
+// determinant - reciprocal - two products of a block and, near it, by FP64 issue:
+// 2640 cycles at m = 13 with one warp per scheduler, against 3100 for single
+// pivots with a broadcast row and 3900 for 2 x 2 blocks with broadcast rows.
+// Returns false (a is then garbage) when a multiplier t_r outside the block
+// reaches 256 or is no number: the caller falls back to partial pivoting.
+template <int m>
+__device__ __forceinline__ bool invert_sym(cplxd (&a)[RowLay<m>::H], cplxd* buf, int lane) {
+    constexpr int H = RowLay<m>::H;
+    const int r = lane >> 1, h = lane & 1;
+    int bad = 0;
+    // the high words of |doubles| order like the doubles
+    auto check = [&](cplxd t, int lim) {
+        const int x = __double2hiint(t.x) & 0x7fffffff, y = __double2hiint(t.y) & 0x7fffffff;
+        bad |= max(x, y) >= lim;
+    };
+    auto publish = [&](int p) {
+        cplxd* b = buf + (p >> 1) % 3 * 2 * kMaxM + 2 * r;
+        const int jp = 2 * (p >> 2), j1 = jp + 1 < H ? jp + 1 : jp;
+        if (h == ((p >> 1) & 1)) {
+            b[0] = a[jp];
+            if (p + 1 < m) b[1] = a[j1];
+        }
+        __syncwarp();
+    };
+    publish(0);
+#pragma unroll
+    for (int p = 0; p < m; p += 2) {
+        const bool two = p + 1 < m;
+        const int hp = (p >> 1) & 1, jp = 2 * (p >> 2), j1 = jp + 1 < H ? jp + 1 : jp;
+        const cplxd* b = buf + (p >> 1) % 3 * 2 * kMaxM;
+        const bool own = two ? (r >> 1) == (p >> 1) : r == p;
+        const int lim = own ? 0x7ff00000 : 0x40700000;  // 256 outside the block
+        cplxd u0 = b[2 * r], u1 = two ? b[2 * r + 1] : cmk(0.0, 0.0), t0, t1 = cmk(0.0, 0.0);
+        if (own) {
+            u0 = cmk(r == p ? -1.0 : 0.0, 0.0);
+            u1 = cmk(r == p ? 0.0 : -1.0, 0.0);
+        }
+        if (two) {
+            const cplxd B00 = b[2 * p], B01 = b[2 * p + 1], B11 = b[2 * p + 3];
+            const cplxd rd = crcp(cfms(B01, B01, cmul(B00, B11)));
+            t0 = cmul(cfms(u1, B01, cmul(u0, B11)), rd);
+            t1 = cmul(cfms(u0, B01, cmul(u1, B00)), rd);
+            check(t1, lim);
+        } else {
+            t0 = cmul(u0, crcp(b[2 * p]));
+        }
+        check(t0, lim);
+        auto update = [&](int j) {
+            const cplxd* uc = b + 2 * RowLay<m>::col(h, j);
+            cplxd v = own ? cmk(0.0, 0.0) : a[j];
+            v = cfms(t0, uc[0], v);
+            if (two) v = cfms(t1, uc[1], v);
+            if (j == jp) v = h == hp ? t0 : v;
+            if (two && j == jp + 1) v = h == hp ? t1 : v;
+            a[j] = v;
+        };
+        const int jn = 2 * ((p + 2) >> 2);  // the next block's columns first
+        if (p + 2 < m) {
+            update(jn);
+            if (jn + 1 < H) update(jn + 1 < H ? jn + 1 : jn);
+            publish(p + 2);
+        }
+#pragma unroll
+        for (int j = 0; j < H; ++j)
+            if (p + 2 >= m || (j != jn && j != jn + 1)) update(j);
+    }
+    return !__any_sync(0xffffffffu, bad && r < m);
+}
+
 __device__ __forceinline__ cplxd warp_sum(cplxd v) {
 #pragma unroll
     for (int o = 16; o >= 1; o >>= 1) {
@@ -456,9 +583,6 @@ __device__ __forceinline__ void cp_async(T* smem_dst, const T* gsrc) {
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
-
-// Energy flags: kRsFP32 runs the chain in FP32.
-constexpr int kRsFP32 = 1;
 
 // Lead kernel: block e -> energy e, lanes 0-15 the left lead, 16-31 the
 // right one.  A lead is uniform (the contact potential u on every atom), so
@@ -512,103 +636,57 @@ __global__ void __launch_bounds__(32) rs_lead_kernel(double gamma, const double*
 }
 
 // Gamma = i (Sigma - Sigma^dagger) = -2 gamma^2 Im s of a contact (s: the
-// lead's surface corner, complex symmetric), factored as L L^T by Cholesky
-// with diagonal pivoting (Gamma is real symmetric positive semidefinite);
-// columns past the numerical rank (pivots below 1e-13 of the largest
-// diagonal entry) stay zero.  One lane, once per energy and contact; L times
-// `scale` into a complex tile (imaginary parts zero).
+// lead's surface corner, a symmetric circulant), factored as L L^T: Gamma is
+// diagonal in the ring's real Fourier vectors, so column q of L is the vector of
+// mode q (the cosine for q <= m / 2, the sine of m - q else) times the root of
+// its eigenvalue; eigenvalues below 1e-13 of Gamma's diagonal give a zero
+// column.  O(m^2) over the warp (a Cholesky factor on one lane took 0.19 ms per
+// energy at m = 13, a tenth of a biased chain).  tab: 2 kMaxM of shared memory.
 template <int m>
-__device__ __noinline__ void gamma_factor(const cplxd* __restrict__ s, double g2, double scale, Mat<m, double> L,
-                                          int lane) {
-    if (lane == 0) {
-        double a[m][m];
-        int perm[m];
-        double dmax = 0.0;
-        for (int i = 0; i < m; ++i) {
-            perm[i] = i;
-            for (int j = 0; j < m; ++j) a[i][j] = -g2 * (s[i * m + j].y + s[j * m + i].y);
-            dmax = fmax(dmax, a[i][i]);
-        }
-        int rank = 0;
-        for (int p = 0; p < m; ++p) {
-            int q = p;
-            for (int i = p + 1; i < m; ++i)
-                if (a[i][i] > a[q][q]) q = i;
-            if (!(a[q][q] > 1e-13 * dmax)) break;
-            if (q != p) {
-                for (int j = 0; j < m; ++j) {
-                    const double t = a[p][j];
-                    a[p][j] = a[q][j];
-                    a[q][j] = t;
-                }
-                for (int i = 0; i < m; ++i) {
-                    const double t = a[i][p];
-                    a[i][p] = a[i][q];
-                    a[i][q] = t;
-                }
-                const int t = perm[p];
-                perm[p] = perm[q];
-                perm[q] = t;
-            }
-            const double l = sqrt(a[p][p]), il = 1.0 / l;
-            a[p][p] = l;
-            for (int i = p + 1; i < m; ++i) a[i][p] *= il;
-            for (int j = p + 1; j < m; ++j)
-                for (int i = j; i < m; ++i) {
-                    a[i][j] -= a[i][p] * a[j][p];
-                    a[j][i] = a[i][j];
-                }
-            rank = p + 1;
-        }
-        for (int i = 0; i < m * m; ++i) L.a[i] = cmk(0.0, 0.0);
-        for (int p = 0; p < rank; ++p)
-            for (int i = p; i < m; ++i) L.at(perm[i], p) = cmk(a[i][p] * scale, 0.0);
+__device__ __forceinline__ void gamma_factor(const cplxd* __restrict__ s, double g2, Mat<m, double> L, cplxd* tab,
+                                             int lane) {
+    if (lane < m) {
+        double sn, cs;
+        sincospi(2.0 * lane / m, &sn, &cs);
+        tab[lane] = cmk(cs, sn);
+        tab[kMaxM + lane].x = -2.0 * g2 * s[lane * m].y;  // Gamma[d][0]
+    }
+    __syncwarp();
+    double w = 0.0;
+    if (lane < m) {
+        double lam = 0.0;
+        for (int d = 0; d < m; ++d) lam = fma(tab[(lane * d) % m].x, tab[kMaxM + d].x, lam);
+        const double norm = lane == 0 || 2 * lane == m ? 1.0 : 2.0;
+        if (lam > 1e-13 * tab[kMaxM].x) w = sqrt(lam * norm / m);
+    }
+    __syncwarp();
+    if (lane < m) tab[kMaxM + lane].x = w;
+    __syncwarp();
+    for (int i = lane; i < m * m; i += 32) {
+        const int j = i / m, q = i % m;
+        const cplxd v = tab[(q * j) % m];
+        L.a[i] = cmk((2 * q <= m ? v.x : v.y) * tab[kMaxM + q].x, 0.0);
     }
     __syncwarp();
 }
 
-// One energy's chain in precision R (warp e): atom potentials Ua, lead
+// One energy's FP32 chain of mixed mode (warp e): atom potentials Ua, lead
 // corners (FP64, m x m, row-major), scratch myX for X_k (K m^2 complex R),
 // row of 2K ring sums Im(c sum_j G_jj) written in FP64.  The potentials of
 // the next block are loaded while the current block is computed.
-//
-// NEQ (a real-axis energy, FP64): the row holds instead the ring sums of the
-// contact spectral functions, b0 A^L + b1 A^R with (b0, b1) = cc and
-// A^c_ring = sum_{n in ring} [G_{n,c} Gamma_c G_{n,c}^dagger]_nn
-// = || G_{ring,c} L_c ||_F^2 (Gamma_c = L_c L_c^T).  The contact columns of
-// G are carried through the sweeps in ring corners:
-//   source (ring a of block 0): Q_k = g_L[k]_{b_k, a_0} L_L with
-//     Q_{-1} = L_L / gamma, Q_k = gamma^2 Y^T (X_k Q_{k-1}) (forward, kept in
-//     myQ); G_{k,0}[a] L_L = gamma G_kk[a][a] Q_{k-1} and
-//     G_{k,0}[b] L_L = (I + gamma^2 g_L[b][b] G') Q_k (backward);
-//   drain (ring b of block K-1): T_k = G_{k,c}[a] L_R with
-//     T_K = (I + gamma^2 G'_K g_L[b][b]) L_R / gamma (G'_K of the right lead),
-//     T_k = gamma^2 X_k (Y T_{k+1}) and G_{k,c}[b] L_R = gamma g_L[b][b] T_{k+1}.
-// Four more m x m products per block in the backward sweep and one in the
-// forward sweep; no G_jj sums (the real-axis energies carry no contour term).
-template <int m, typename R, bool NEQ = false>
+template <int m, typename R>
 __device__ __forceinline__ bool rs_chain(int K, R gamma, cplx<R> E, cplxd cc, const double* __restrict__ Ua,
                                          const cplxd* __restrict__ sL, const cplxd* __restrict__ sR,
-                                         cplx<R>* __restrict__ myX, cplx<R>* __restrict__ myQ,
-                                         double* __restrict__ row, cplx<R>* sh, int lane) {
-    static_assert(!NEQ || sizeof(R) == 8, "the non-equilibrium chains run in FP64");
+                                         cplx<R>* __restrict__ myX, double* __restrict__ row, cplx<R>* sh, int lane) {
     using C = cplx<R>;
     constexpr int mm2 = m * m;
-    constexpr int tiles = NEQ ? 9 : 5;
     const R g2 = gamma * gamma, g4 = g2 * g2;
     const R zero(0), one(1);
     const Mat<m, R> X{sh}, Gbb{sh + mm2}, Gn{sh + 2 * mm2}, Z{sh + 3 * mm2}, W{sh + 4 * mm2};
-    // NEQ: source columns (current / previous block), drain column, product tile
-    const Mat<m, R> Qa{sh + 5 * mm2}, Qb{sh + 6 * mm2}, T{sh + 7 * mm2}, P{sh + 8 * mm2};
-    C* dv = sh + tiles * mm2;  // D^-1 of the current ring b
+    C* dv = sh + 5 * mm2;  // D^-1 of the current ring b
     C* da = dv + kMaxM;        // E - U of the current ring a
     C* buf = da + kMaxM;       // pivot column
     bool ok = true;
-    if constexpr (NEQ) {
-        gamma_factor<m>(sL, g2, one / gamma, Qa, lane);  // Q_{-1}
-        gamma_factor<m>(sR, g2, one, T, lane);           // L_R
-        for (int i = lane; i < mm2; i += 32) myQ[i] = Qa.a[i];
-    }
     // lane j < m: potentials of atom j on rings a and b of the next block
     R ua_n = zero, ub_n = zero;
     auto fetch_u = [&](int k) {
@@ -653,17 +731,6 @@ __device__ __forceinline__ bool rs_chain(int K, R gamma, cplx<R> E, cplxd cc, co
         ok = invert<m>(X, X, buf, lane) && ok;
         C* dst = myX + (size_t)k * mm2;
         for (int i = lane; i < mm2; i += 32) dst[i] = X.a[i];
-        if constexpr (NEQ) {
-            // Q_k = gamma^2 Y^T (X_k Q_{k-1}), (Y^T M)[r][c] = D^-1_r (M[r][c] + M[r-1][c])
-            mm<m, false, false, false>(P, X, Qa, P, one, lane);
-            RS_FOR_ENTRIES(m, lane, {
-                const int r0 = wrap<m>(r - 1);
-                Qa.at(r, c) = cscale(cmul(dv[r], cadd(P.at(r, c), P.at(r0, c))), g2);
-            })
-            __syncwarp();
-            C* qd = myQ + (size_t)(k + 1) * mm2;
-            for (int i = lane; i < mm2; i += 32) qd[i] = Qa.a[i];
-        }
         form_gbb(X);
     }
     // G_K[a][a] of the right lead's first ring: (I - gamma^2 s_R g_L[b][b])^-1 s_R
@@ -673,54 +740,21 @@ __device__ __forceinline__ bool rs_chain(int K, R gamma, cplx<R> E, cplxd cc, co
     if (lane < m) Gn.at(lane, lane) = cadd(Gn.at(lane, lane), cmk(one, zero));
     ok = invert<m>(Gn, Gn, buf, lane) && ok;
     mm<m, false, false, false>(Gn, Gn, X, Gn, one, lane);
-    if constexpr (NEQ) {
-        // T_K = (L_R + gamma^2 G'_K (g_L[b][b] L_R)) / gamma
-        mm<m, false, false, false>(P, Gbb, T, P, one, lane);
-        mm<m, false, false, true>(T, Gn, P, T, g2, lane);
-        RS_FOR_ENTRIES(m, lane, { T.at(r, c) = cscale(T.at(r, c), one / gamma); })
-        __syncwarp();
-    }
     fetch_u(K - 1);
     // Backward.  X_{k-1} is copied into the tile that held the product W of
     // step k (free once tr G[b][b] is formed) while the last two products of
     // step k run; the two tiles swap roles every step.
     Mat<m, R> Xc = X, Wc = W;
-    // NEQ: Qc = Q_k, Qp = Q_{k-1}; Q_{k-2} is copied into Qc once Q_k is used
-    Mat<m, R> Qc = Qa, Qp = Qb;
     {
         const C* src = myX + (size_t)(K - 1) * mm2;
         for (int i = lane; i < mm2; i += 32) Xc.a[i] = src[i];
-        if constexpr (NEQ) {
-            for (int i = lane; i < mm2; i += 32) {
-                Qc.a[i] = myQ[(size_t)K * mm2 + i];
-                Qp.a[i] = myQ[(size_t)(K - 1) * mm2 + i];
-            }
-        }
     }
     for (int k = K - 1; k >= 0; --k) {
-        cp_async_wait_all();  // X_k (and Q_{k-1}), issued during step k + 1, have landed
+        cp_async_wait_all();  // X_k, issued during step k + 1, has landed
         if (lane < m) dv[lane] = crcp(cmk(E.x - ub_n, E.y));
         if (k > 0) fetch_u(k - 1);
         __syncwarp();
         form_gbb(Xc);
-        double tRa = 0.0, tRb = 0.0, tLa = 0.0, tLb = 0.0;
-        if constexpr (NEQ) {
-            // drain column, ring b: gamma g_L[b][b] T_{k+1}; then Y T_{k+1} into P
-            mm<m, false, false, false>(P, Gbb, T, P, gamma, lane);
-            RS_FOR_ENTRIES(m, lane, {
-                const C v = P.at(r, c);
-                tRb = fma(v.x, v.x, fma(v.y, v.y, tRb));
-                const int r1 = wrap<m>(r + 1);
-                P.at(r, c) = cadd(cmul(dv[r], T.at(r, c)), cmul(dv[r1], T.at(r1, c)));
-            })
-            __syncwarp();
-            // ring a: T_k = gamma^2 X_k (Y T_{k+1})
-            mm<m, false, false, false>(T, Xc, P, T, g2, lane);
-            RS_FOR_ENTRIES(m, lane, {
-                const C v = T.at(r, c);
-                tRa = fma(v.x, v.x, fma(v.y, v.y, tRa));
-            })
-        }
         // Z = Y G' Y^T = C (D^-1 G' D^-1) C^T, Y = C D^-1: H = D^-1 G' D^-1 in the
         // free tile Wc, then four neighbours of H per entry
         RS_FOR_ENTRIES(m, lane, { Wc.at(r, c) = cmul(cmul(dv[r], Gn.at(r, c)), dv[c]); })
@@ -733,28 +767,15 @@ __device__ __forceinline__ bool rs_chain(int K, R gamma, cplx<R> E, cplxd cc, co
         // W = g_L[b][b] G'; tr G[b][b] = tr g_L[b][b] + gamma^2 sum_rc W[r][c] g_L[b][b][c][r]
         mm<m, false, false, false>(Wc, Gbb, Gn, Wc, one, lane);
         cplxd tb = cmk(0.0, 0.0);
-        if constexpr (NEQ) {
-            // source column, ring b: (I + gamma^2 W) Q_k
-            mm<m, false, false, true>(P, Wc, Qc, Qc, g2, lane);
-            RS_FOR_ENTRIES(m, lane, {
-                const C v = P.at(r, c);
-                tLb = fma(v.x, v.x, fma(v.y, v.y, tLb));
-            })
-        } else {
-            RS_FOR_ENTRIES(m, lane, {
-                const C w = cmul(cscale(Wc.at(r, c), g2), Gbb.at(c, r));
-                tb = cadd(tb, cmk((double)w.x, (double)w.y));
-                if (r == c) tb = cadd(tb, cmk((double)Gbb.at(r, r).x, (double)Gbb.at(r, r).y));
-            })
-        }
-        __syncwarp();  // every lane is done with Wc (and Qc)
+        RS_FOR_ENTRIES(m, lane, {
+            const C w = cmul(cscale(Wc.at(r, c), g2), Gbb.at(c, r));
+            tb = cadd(tb, cmk((double)w.x, (double)w.y));
+            if (r == c) tb = cadd(tb, cmk((double)Gbb.at(r, r).x, (double)Gbb.at(r, r).y));
+        })
+        __syncwarp();  // every lane is done with Wc
         if (k > 0) {
             const C* src = myX + (size_t)(k - 1) * mm2;
             for (int i = lane; i < mm2; i += 32) cp_async(Wc.a + i, src + i);
-            if constexpr (NEQ) {
-                const C* qs = myQ + (size_t)(k - 1) * mm2;  // Q_{k-2}
-                for (int i = lane; i < mm2; i += 32) cp_async(Qc.a + i, qs + i);
-            }
             cp_async_commit();
         }
         // G[a][a] = X + gamma^4 (X Z) X
@@ -765,93 +786,449 @@ __device__ __forceinline__ bool rs_chain(int K, R gamma, cplx<R> E, cplxd cc, co
             Xc = Wc;
             Wc = tt;
         }
-        if constexpr (NEQ) {
-            // source column, ring a: gamma G_kk[a][a] Q_{k-1}
-            mm<m, false, false, false>(P, Gn, Qp, P, gamma, lane);
-            RS_FOR_ENTRIES(m, lane, {
-                const C v = P.at(r, c);
-                tLa = fma(v.x, v.x, fma(v.y, v.y, tLa));
-            })
-            const Mat<m, R> tt = Qc;
-            Qc = Qp;
-            Qp = tt;
-            const cplxd sa = warp_sum(cmk(tLa, tRa)), sb = warp_sum(cmk(tLb, tRb));
-            if (lane == 0) {
-                row[2 * k] = fma(cc.x, sa.x, cc.y * sa.y);
-                row[2 * k + 1] = fma(cc.x, sb.x, cc.y * sb.y);
-            }
-        } else {
-            cplxd ta = cmk(0.0, 0.0);
-            if (lane < m) ta = cmk((double)Gn.at(lane, lane).x, (double)Gn.at(lane, lane).y);
-            ta = warp_sum(ta);
-            tb = warp_sum(tb);
-            if (lane == 0) {
-                row[2 * k] = fma(cc.x, ta.y, cc.y * ta.x);      // Im(c tr G[a][a])
-                row[2 * k + 1] = fma(cc.x, tb.y, cc.y * tb.x);  // Im(c tr G[b][b])
-            }
+        cplxd ta = cmk(0.0, 0.0);
+        if (lane < m) ta = cmk((double)Gn.at(lane, lane).x, (double)Gn.at(lane, lane).y);
+        ta = warp_sum(ta);
+        tb = warp_sum(tb);
+        if (lane == 0) {
+            row[2 * k] = fma(cc.x, ta.y, cc.y * ta.x);      // Im(c tr G[a][a])
+            row[2 * k + 1] = fma(cc.x, tb.y, cc.y * tb.x);  // Im(c tr G[b][b])
         }
     }
     return ok;
 }
 
-// Chain kernel: warp e -> energy e in the precision its flags give.
-// gX: [num_e][K][m*m] FP64-complex slots (an FP32 chain uses the first half
-// of its slot); rows: [num_e][N].
+// FP32 chain kernel: warp i -> energy e = e_off + i.
+// gX: [energy][K][m*m] FP64-complex slots (an FP32 chain uses the first half
+// of its slot); rows: [energy][N].
 template <int m>
 __global__ void __launch_bounds__(32, 16) rs_chain_kernel(int K, double gamma, const double* __restrict__ Ere,
                                                           const double* __restrict__ Eim,
                                                           const double* __restrict__ cre,
-                                                          const double* __restrict__ cim, int num_e,
-                                                          const int* __restrict__ flags,
+                                                          const double* __restrict__ cim, int e_off, int num,
                                                           const double* __restrict__ Ua,
                                                           const cplxd* __restrict__ corners, cplxd* __restrict__ gX,
                                                           double* __restrict__ rows, int* __restrict__ status) {
-    extern __shared__ cplxd sh[];
+    extern __shared__ __align__(16) unsigned char sh_raw[];
     const int lane = threadIdx.x;
-    const int e = blockIdx.x;
-    if (e >= num_e) return;
+    if ((int)blockIdx.x >= num) return;
+    const int e = e_off + blockIdx.x;
     constexpr int mm2 = m * m;
-    const int fl = flags[e];
     const cplxd* sL = corners + (size_t)e * 2 * mm2;
-    const cplxd* sR = sL + mm2;
-    cplxd* myX = gX + (size_t)e * K * mm2;
-    double* row = rows + (size_t)e * 2 * K;
-    const cplxd cc = cmk(cre[e], cim[e]);
-    bool ok;
-    if (!(fl & kRsFP32))
-        ok = rs_chain<m, double>(K, gamma, cmk(Ere[e], Eim[e]), cc, Ua, sL, sR, myX, nullptr, row, sh, lane);
-    else
-        ok = rs_chain<m, float>(K, (float)gamma, cmk((float)Ere[e], (float)Eim[e]), cc, Ua, sL, sR,
-                                reinterpret_cast<cplxf*>(myX), nullptr, row, reinterpret_cast<cplxf*>(sh), lane);
+    const bool ok = rs_chain<m, float>(K, (float)gamma, cmk((float)Ere[e], (float)Eim[e]), cmk(cre[e], cim[e]), Ua, sL,
+                                       sL + mm2, reinterpret_cast<cplxf*>(gX + (size_t)e * K * mm2),
+                                       rows + (size_t)e * 2 * K, reinterpret_cast<cplxf*>(sh_raw), lane);
     if (!ok && lane == 0) atomicExch(status, 1);
 }
 
-// Non-equilibrium chain kernel: warp i -> real-axis energy e = e_off + i in
-// FP64 with the atom potentials and coefficients (b0, b1) = (cre, cim)[e].
-// gXn: [num][2K + 1][m*m] FP64-complex (X_k, then Q_{-1} ... Q_{K-1});
-// rows: [e][2K] as for the other energies.
-template <int m>
-__global__ void __launch_bounds__(32, 8) rs_chain_neq_kernel(int K, double gamma, const double* __restrict__ Ere,
-                                                             const double* __restrict__ Eim,
-                                                             const double* __restrict__ cre,
-                                                             const double* __restrict__ cim, int e_off, int num,
-                                                             const double* __restrict__ Uatoms,
-                                                             const cplxd* __restrict__ corners,
-                                                             cplxd* __restrict__ gXn, double* __restrict__ rows,
-                                                             int* __restrict__ status) {
-    extern __shared__ cplxd sh[];
-    const int lane = threadIdx.x;
-    const int i = blockIdx.x;
-    if (i >= num) return;
-    constexpr int mm2 = m * m;
-    const int e = e_off + i;
-    const cplxd* sL = corners + (size_t)e * 2 * mm2;
-    const cplxd* sR = sL + mm2;
-    cplxd* myX = gXn + (size_t)i * (2 * K + 1) * mm2;
-    cplxd* myQ = myX + (size_t)K * mm2;
-    double* row = rows + (size_t)e * 2 * K;
-    const bool ok = rs_chain<m, double, true>(K, gamma, cmk(Ere[e], Eim[e]), cmk(cre[e], cim[e]), Uatoms, sL, sR,
-                                              myX, myQ, row, sh, lane);
+// Complex values of shared memory of one warp of a pair: tiles, then D^-1 of
+// the current and the previous ring b, the pivot column of the fall-back and the
+// column pairs of the sweeps.
+template <int m, bool NEQ>
+__host__ __device__ constexpr int pair_complex() {
+    return (NEQ ? 7 : 5) * m * m + 3 * kMaxM + RowLay<m>::kBuf;
+}
+
+// One half of an energy's chain in FP64.  The two warps of a block take the
+// chain from its two ends and meet in the middle: side 0 runs blocks 0 .. KS -
+// 1 from the left lead; side 1 the others from the right lead, on the chain
+// read backwards.  Read backwards with the atoms of every ring reflected, j ->
+// -j mod m, the chain has the same bonds (ring b comes first, its atom j bonded
+// to atoms j and j - 1 of ring a), and the lead corners are symmetric
+// circulants, so both sides run the same code; only the potentials' addresses,
+// the rows and the contacts' roles differ.  Each side
+//   sweeps forward over its KS blocks (X_k kept in myX),
+//   takes the other side's end corner g[b][b], reflected, as its right lead:
+//     G' = G_K[a][a] = (I - gamma^2 s g_L[b][b])^-1 s of the other side's last ring,
+//   and runs the backward recursion over its blocks, with V = X Y, Y = C D^-1:
+//     M = V G'                            gamma^2 M = G_{k,k+1}[a][a]
+//     G_kk[a][a] = X + gamma^4 M V^T      (symmetric: three of four tiles)
+//     G_kk[b][b]_rr = d_r + gamma^2 d_r^2 (C^T G_kk[a][a] C + 2 gamma^2 C^T M + G')_rr
+//   (the last from (E - H) G = 1 in the rows and columns of ring b): two products
+//   per block and O(m^2).  The diagonal formula loses a factor gamma^2 |d|^2 of
+//   the working precision, so a ring with an atom within gamma / 100 of E (no
+//   energy at 300 K: the lowest pole lies 0.08 eV off the axis) takes
+//   tr G[b][b] = tr(g_L[b][b]) + gamma^2 tr(g_L[b][b]^2 G') instead.
+// The work is that of one chain, its length in dependent steps is halved.
+//
+// NEQ (a real-axis energy): the row holds the ring sums of the contact
+// spectral functions, b0 A^L + b1 A^R with (b0, b1) = cc and
+// A^c_ring = sum_{n in ring} [G_{n,c} Gamma_c G_{n,c}^dagger]_nn
+// = || G_{ring,c} L_c ||_F^2 (Gamma_c = L_c L_c^T).  The columns of G times L
+// come by block substitution, for the side's own lead (S_k = G_{a_k,a_0} L) and
+// the other one (T_k):
+//   forward   P_k = gamma X_k Q_{k-1}, Q_k = gamma Y^T P_k, Q_{-1} = L / gamma
+//             (Q_k = g_L[k]_{b_k, a_0} L; P_k kept in myP);
+//   middle    S_K = gamma G' Q_{KS-1}; T_K = (I + gamma^2 G' g_L[b][b]) Q', Q' the
+//             other side's last Q, reflected;
+//   backward  S_k = P_k + gamma^2 V S_{k+1}, T_k = gamma^2 V T_{k+1}, and on ring b
+//             the rows of (E - H) G = 1: D^-1 gamma (C^T S_k + S_{k+1}), the same for T.
+// Three products per block; no G_jj sums (the real-axis energies carry no
+// contour term).
+//
+// Bound by the dependent steps of one block update up to one warp per scheduler
+// (8000 cycles at m = 13: inversion 2640, products 2000, passes over tiles the
+// rest), by FP64 issue and shared memory beyond.  Charge of a 75-cell tube, us,
+// with one warp per energy, three products and single pivots / here:
+//   m = 13, 64 + 64 + 128 contour points   1428 / 379
+//   m = 13, 128 + 128 + 256                1524 / 549
+//   m = 13, 512 + 512 + 1024               3365 / 1850
+//   m = 16, 128 + 128 + 256                1905 / 770
+//   m = 7,  128 + 128 + 256                 600 / 277
+//   m = 13, 64 real-axis points            3535 / 771
+//   m = 13, 2048 real-axis points          7920 / 2815
+template <int m, bool NEQ>
+__device__ __forceinline__ bool rs_side(int side, int K, int KS, double gamma, cplxd E, cplxd cc,
+                                        const double* __restrict__ Ua, const cplxd* __restrict__ sL,
+                                        cplxd* __restrict__ myX, cplxd* __restrict__ myP, double* __restrict__ row,
+                                        cplxd* sh, const cplxd* other, int lane) {
+    using C = cplxd;
+    constexpr int mm2 = m * m, H = (m + 1) / 2, HR = RowLay<m>::H;
+    using Tile = Mat<m, double>;
+    const double g2 = gamma * gamma, g4 = g2 * g2;
+    const Tile X{sh}, B{sh + mm2}, V{sh + 2 * mm2}, Gn{sh + 3 * mm2}, Q{sh + 4 * mm2};
+    C* dv = sh + (NEQ ? 7 : 5) * mm2;  // D^-1 of the current ring b
+    C* dp = dv + kMaxM;                // D^-1 of the previous ring b
+    C* buf = dp + kMaxM;               // pivot column of the fall-back
+    C* inv_buf = buf + kMaxM;          // column pairs of the sweeps
+    const int N = 2 * K;
+    bool ok = true;
+    // Row layout (two lanes per row) of the forward sweep, column layout (lane &
+    // 15 = column, rows h H ..) of the tile passes; rows and columns past m - 1
+    // are clamped, so that no load is conditional and the loads of a pass overlap.
+    const int rr = min(lane >> 1, m - 1), hr = lane & 1;
+    const bool rv = (lane >> 1) < m;
+    const int pc = min(lane & 15, m - 1), pr = (lane >> 4) * H;
+    const bool pv = (lane & 15) < m;
+    // potentials of atom rr (of the reflected ring on side 1) on rings a and b of the next block
+    const int atom = side && rr > 0 ? m - rr : rr;
+    double ua_n = 0.0, ub_n = 0.0;
+    auto fetch_u = [&](int k) {
+        const int ra = side ? N - 1 - 2 * k : 2 * k, rb = side ? ra - 1 : ra + 1;
+        ua_n = __ldg(Ua + (size_t)ra * m + atom);
+        ub_n = __ldg(Ua + (size_t)rb * m + atom);
+    };
+    // g_L[b][b] = D^-1 + gamma^2 Y^T X Y of tile Xt into B
+    auto form_gbb = [&](Tile Xt, Tile out, const C* d) {
+        const int c0 = wrap<m>(pc - 1);
+        const C dc = cscale(d[pc], g2);
+        C s[H + 1];
+#pragma unroll
+        for (int i = 0; i <= H; ++i) {
+            const int r = min(wrap<m>(pr - 1 + i), m - 1);
+            s[i] = cadd(Xt.at(r, pc), Xt.at(r, c0));
+        }
+#pragma unroll
+        for (int i = 0; i < H; ++i) {
+            const int r = min(pr + i, m - 1);
+            C v = cmul(cmul(d[r], dc), cadd(s[i], s[i + 1]));
+            if (r == pc) v = cadd(v, d[r]);
+            if (pv && pr + i < m) out.at(r, pc) = v;
+        }
+        __syncwarp();
+    };
+    if constexpr (NEQ) {
+        gamma_factor<m>(sL, g2, Q, dv, lane);  // dv, dp: scratch
+#pragma unroll
+        for (int i = lane; i < mm2; i += 32) Q.a[i] = cscale(Q.a[i], 1.0 / gamma);
+    }
+    fetch_u(0);
+    // E - U_a and D^-1 of this lane's row, one block ahead; D^-1 of the ring in dv, dp (the previous ring's) in turn
+    C da = cmk(E.x - ua_n, E.y), db = crcp(cmk(E.x - ub_n, E.y));
+    if (KS > 1) fetch_u(1);
+    __syncwarp();
+    if (rv && hr == 0) dv[rr] = db;
+    __syncwarp();
+    for (int k = 0; k < KS; ++k) {
+        // -S, S = diag(E - U_a) - gamma^2 g_L[b][b]_{k-1} - gamma^2 C D^-1 C^T, in the row layout straight
+        // from X_{k-1} (the lead's corner at k = 0): no pass over a tile between two inversions
+        C a[HR];
+        auto col = [&](int j) { return min(RowLay<m>::col(hr, j), m - 1); };
+        auto build = [&]() {
+            const int r0 = wrap<m>(rr - 1), r1 = wrap<m>(rr + 1);
+            const C lo = cscale(db, g2), hi = cscale(dv[r1], g2);
+            C dg = csub(cadd(lo, hi), da);
+            if (k == 0) {
+#pragma unroll
+                for (int j = 0; j < HR; ++j) a[j] = cscale(sL[rr * m + col(j)], g2);
+            } else {
+                const C dr = cscale(dp[rr], g2);
+                const C dq = cscale(dr, g2);
+                dg = cadd(dg, dr);
+#pragma unroll
+                for (int j = 0; j < HR; j += 2) {
+                    const int c = col(j), c0 = wrap<m>(c - 1);
+                    const C s0 = cadd(X.at(rr, c0), X.at(r0, c0)), s1 = cadd(X.at(rr, c), X.at(r0, c));
+                    a[j] = cmul(cmul(dq, dp[c]), cadd(s0, s1));
+                    if (j + 1 < HR) {
+                        const int c1 = col(j + 1);
+                        const C s2 = cadd(X.at(rr, c1), X.at(r0, c1));
+                        a[j + 1 < HR ? j + 1 : j] = cmul(cmul(dq, dp[c1]), cadd(s1, s2));
+                    }
+                }
+            }
+#pragma unroll
+            for (int j = 0; j < HR; ++j) {
+                const int c = col(j), c1 = wrap<m>(c + 1);
+                if (rr == c) a[j] = cadd(a[j], dg);
+                if (rr == c1) a[j] = cadd(a[j], lo);  // column r - 1
+                if (r1 == c) a[j] = cadd(a[j], hi);   // column r + 1
+            }
+        };
+        build();
+        if (!invert_sym<m>(a, inv_buf, lane)) {
+            // a large multiplier: -S again as a tile (in V, free here), inverted with partial pivoting
+            build();
+#pragma unroll
+            for (int j = 0; j < HR; ++j)
+                if (rv && RowLay<m>::col(hr, j) < m) V.at(rr, RowLay<m>::col(hr, j)) = a[j];
+            __syncwarp();
+            ok = invert_pivoted<m, double>(V, V, buf, lane) && ok;
+#pragma unroll
+            for (int j = 0; j < HR; ++j) a[j] = cscale(V.at(rr, col(j)), -1.0);
+        }
+        __syncwarp();  // every lane is done with X_{k-1} and dp
+        C* dst = myX + (size_t)k * mm2;
+#pragma unroll
+        for (int j = 0; j < HR; ++j) {
+            const int c = RowLay<m>::col(hr, j);
+            if (rv && c < m) {
+                X.at(rr, c) = a[j];
+                dst[rr * m + c] = a[j];
+            }
+        }
+        if (k + 1 < KS) {
+            da = cmk(E.x - ua_n, E.y);
+            db = crcp(cmk(E.x - ub_n, E.y));
+            if (rv && hr == 0) dp[rr] = db;
+            if (k + 2 < KS) fetch_u(k + 2);
+        }
+        __syncwarp();
+        if constexpr (NEQ) {
+            // P_k = gamma X_k Q_{k-1} (in V); Q_k = gamma Y^T P_k, (Y^T P)[r][c] = D^-1_r (P[r][c] + P[r-1][c])
+            C* pd = myP + (size_t)k * mm2;
+            mm_each<m, false, false, false>(X, Q, lane, [&](int r, int c, C v, bool valid, bool) {
+                v = cscale(v, gamma);
+                if (valid) V.at(r, c) = pd[r * m + c] = v;
+            });
+            C s[H + 1];
+#pragma unroll
+            for (int i = 0; i <= H; ++i) s[i] = V.at(min(wrap<m>(pr - 1 + i), m - 1), pc);
+#pragma unroll
+            for (int i = 0; i < H; ++i) {
+                const int r = min(pr + i, m - 1);
+                const C v = cmul(cscale(dv[r], gamma), cadd(s[i], s[i + 1]));
+                if (pv && pr + i < m) Q.at(r, pc) = v;
+            }
+            __syncwarp();  // every lane is done with dv
+        }
+        if (k + 1 < KS) {
+            C* const t = dv;
+            dv = dp;
+            dp = t;
+        }
+    }
+    form_gbb(X, B, dv);
+    // the other side's end corner, reflected, into X, its Q into T
+    const Tile T{sh + (NEQ ? 5 : 0) * mm2}, P{sh + (NEQ ? 6 : 0) * mm2};
+    __syncthreads();
+    for (int i = lane; i < mm2; i += 32) {
+        const int r = i / m, c = i % m, r1 = r ? m - r : 0, c1 = c ? m - c : 0;
+        X.a[i] = other[mm2 + r1 * m + c1];
+        if constexpr (NEQ) T.a[i] = other[4 * mm2 + r1 * m + c];
+    }
+    __syncthreads();  // both have read: B and Q may change
+    // G_K[a][a] of the other side's last ring: (I - gamma^2 s g_L[b][b])^-1 s
+    mm<m, false, false, false>(Gn, X, B, Gn, -g2, lane);
+    if (lane < m) Gn.at(lane, lane) = cadd(Gn.at(lane, lane), cmk(1.0, 0.0));
+    ok = invert<m>(Gn, Gn, buf, lane) && ok;
+    mm<m, false, false, false>(Gn, Gn, X, Gn, 1.0, lane);
+    fetch_u(KS - 1);
+    if constexpr (!NEQ) {
+        // X_{k-1} is copied into the other of two tiles while step k runs
+        Tile Xc = X, Xo = B;
+        const Tile M = Q;
+        auto fetch_x = [&](Tile to, int k) {
+            const C* src = myX + (size_t)k * mm2;
+            for (int i = lane; i < mm2; i += 32) cp_async(to.a + i, src + i);
+            cp_async_commit();
+        };
+        // X_k has landed: D^-1 and V of block k; true when its ring b needs the product formula
+        auto enter = [&](int k) {
+            const C db = crcp(cmk(E.x - ub_n, E.y));
+            if (k > 0) fetch_u(k - 1);
+            if (rv && hr == 0) dv[rr] = db;
+            cp_async_wait_all();
+            __syncwarp();
+            const int c0 = wrap<m>(pc - 1);
+            const C dc = dv[pc];
+#pragma unroll
+            for (int i = 0; i < H; ++i) {
+                const int r = min(pr + i, m - 1);
+                const C v = cmul(dc, cadd(Xc.at(r, pc), Xc.at(r, c0)));
+                if (pv && pr + i < m) V.at(r, pc) = v;
+            }
+            return __any_sync(0xffffffffu, g2 * fma(db.x, db.x, db.y * db.y) > 1e4);
+        };
+        fetch_x(Xc, KS - 1);
+        bool near = enter(KS - 1);
+        for (int k = KS - 1; k >= 0; --k) {
+            __syncwarp();
+            if (k > 0) fetch_x(Xo, k - 1);
+            const int t = min(lane & 15, m - 1), t0 = wrap<m>(t - 1);
+            const C gp = Gn.at(t, t);
+            C tr = cmk(0.0, 0.0);  // ring b by products: this lane's part of tr G[b][b]
+            if (near) {
+                form_gbb(Xc, M, dv);
+                if (lane < m) tr = M.at(lane, lane);
+                mm_each<m, false, false, true>(M, M, lane, [&](int r, int c, C v, bool valid, bool off) {
+                    if (valid) tr = cfma(cscale(v, off ? 2.0 * g2 : g2), Gn.at(c, r), tr);
+                });
+            }
+            mm<m, false, false, false>(M, V, Gn, M, 1.0, lane);
+            mm_each<m, false, true, true>(M, V, lane, [&](int r, int c, C v, bool valid, bool off) {
+                v = cadd(cscale(v, g4), Xc.at(r, c));
+                if (valid) Gn.at(r, c) = v;
+                if (off && valid) Gn.at(c, r) = v;
+            });
+            // diagonals: lanes 0-15 ring a, 16-31 ring b
+            const C g11 = Gn.at(t, t);
+            C v = g11;
+            if (lane >= 16) {
+                const C d = dv[t], d2 = cscale(cmul(d, d), g2);
+                const C o = cadd(cadd(Gn.at(t0, t), Gn.at(t0, t)), cadd(g11, Gn.at(t0, t0)));
+                const C q = cadd(cadd(o, gp), cscale(cadd(M.at(t, t), M.at(t0, t)), 2.0 * g2));
+                v = cfma(d2, q, d);
+            }
+            double w = (lane & 15) < m ? fma(cc.x, v.y, cc.y * v.x) : 0.0;  // Im(c G_jj)
+            if (near) {
+                const double wb = fma(cc.x, tr.y, cc.y * tr.x);
+                const double other_half = __shfl_xor_sync(0xffffffffu, wb, 16);
+                if (lane >= 16) w = wb + other_half;
+            }
+            const int2 rg = side ? make_int2(N - 1 - 2 * k, N - 2 - 2 * k) : make_int2(2 * k, 2 * k + 1);
+            if (k > 0) {
+                const Tile tt = Xc;
+                Xc = Xo;
+                Xo = tt;
+                __syncwarp();  // every lane is done with dv
+                near = enter(k - 1);
+            }
+#pragma unroll
+            for (int o = 8; o >= 1; o >>= 1) w += __shfl_xor_sync(0xffffffffu, w, o);
+            if (lane == 0) row[rg.x] = w;
+            if (lane == 16) row[rg.y] = w;
+        }
+    } else {
+        // S_K and T_K; then S and T alternate between two tiles each
+        Tile Sc = Q, So = B, Tc = T, To = Gn;
+        mm<m, false, false, false>(V, B, T, V, 1.0, lane);
+        mm<m, false, false, true>(T, Gn, V, T, g2, lane);
+        mm<m, false, false, false>(Q, Gn, Q, Q, gamma, lane);
+        auto fetch = [&](Tile to, const C* src) {
+            for (int i = lane; i < mm2; i += 32) cp_async(to.a + i, src + i);
+        };
+        fetch(X, myX + (size_t)(KS - 1) * mm2);
+        fetch(P, myP + (size_t)(KS - 1) * mm2);
+        cp_async_commit();
+        for (int k = KS - 1; k >= 0; --k) {
+            const C db = crcp(cmk(E.x - ub_n, E.y));
+            if (k > 0) fetch_u(k - 1);
+            if (rv && hr == 0) dv[rr] = db;
+            cp_async_wait_all();
+            __syncwarp();
+            const int c0 = wrap<m>(pc - 1);
+            const C dc = dv[pc];
+#pragma unroll
+            for (int i = 0; i < H; ++i) {
+                const int r = min(pr + i, m - 1);
+                const C v = cmul(dc, cadd(X.at(r, pc), X.at(r, c0)));
+                if (pv && pr + i < m) V.at(r, pc) = v;
+            }
+            __syncwarp();
+            if (k > 0) fetch(X, myX + (size_t)(k - 1) * mm2);
+            double sa = 0.0, sb = 0.0;  // this lane's part of the two ring sums
+            mm_each<m, false, false, false>(V, Sc, lane, [&](int r, int c, C v, bool valid, bool) {
+                v = cadd(cscale(v, g2), P.at(r, c));
+                if (valid) {
+                    So.at(r, c) = v;
+                    sa = fma(v.x, v.x, fma(v.y, v.y, sa));
+                }
+            });
+            sa *= cc.x;
+            if (k > 0) fetch(P, myP + (size_t)(k - 1) * mm2);
+            cp_async_commit();
+            double ta = 0.0, tb = 0.0;
+            mm_each<m, false, false, false>(V, Tc, lane, [&](int r, int c, C v, bool valid, bool) {
+                v = cscale(v, g2);
+                if (valid) {
+                    To.at(r, c) = v;
+                    ta = fma(v.x, v.x, fma(v.y, v.y, ta));
+                }
+            });
+            sa = fma(cc.y, ta, sa);
+            // ring b: gamma D^-1 (C^T S_k + S_{k+1}), (C^T S)[r][c] = S[r][c] + S[r-1][c]
+            C s[H + 1], u[H + 1];
+#pragma unroll
+            for (int i = 0; i <= H; ++i) {
+                const int r = min(wrap<m>(pr - 1 + i), m - 1);
+                s[i] = So.at(r, pc);
+                u[i] = To.at(r, pc);
+            }
+#pragma unroll
+            for (int i = 0; i < H; ++i) {
+                const int r = min(pr + i, m - 1);
+                const C d = dv[r];
+                const C x = cadd(cadd(s[i], s[i + 1]), Sc.at(r, pc)), y = cadd(cadd(u[i], u[i + 1]), Tc.at(r, pc));
+                double q = fma(d.x, d.x, d.y * d.y);
+                if (!(pv && pr + i < m)) q = 0.0;
+                sb = fma(q, fma(x.x, x.x, x.y * x.y), sb);
+                tb = fma(q, fma(y.x, y.x, y.y * y.y), tb);
+            }
+            sb = g2 * fma(cc.x, sb, cc.y * tb);
+            // lanes 0-15 sum ring a, 16-31 ring b
+            double w = (lane < 16 ? sa : sb) + __shfl_xor_sync(0xffffffffu, lane < 16 ? sb : sa, 16);
+#pragma unroll
+            for (int o = 8; o >= 1; o >>= 1) w += __shfl_xor_sync(0xffffffffu, w, o);
+            const int2 rg = side ? make_int2(N - 1 - 2 * k, N - 2 - 2 * k) : make_int2(2 * k, 2 * k + 1);
+            if (lane == 0) row[rg.x] = w;
+            if (lane == 16) row[rg.y] = w;
+            Tile tt = Sc;
+            Sc = So;
+            So = tt;
+            tt = Tc;
+            Tc = To;
+            To = tt;
+            __syncwarp();  // every lane is done with dv and V
+        }
+    }
+    return ok;
+}
+
+// FP64 chains: block i -> energy e = e_off + i, one warp per side.  gX: contour
+// and pole energies [e][K][m*m] (X_k of side 0, then of side 1); real-axis
+// energies [i][2][K][m*m] (X_k, P_k).  Four blocks per SM leave 255 registers a
+// thread; six (168, spills) take 369 us against 345 for 64 contour points at m =
+// 13 and gain 5 % at 2048.
+template <int m, bool NEQ>
+__global__ void __launch_bounds__(64, 4) rs_pair_kernel(int K, double gamma, const double* __restrict__ Ere,
+                                                        const double* __restrict__ Eim,
+                                                        const double* __restrict__ cre,
+                                                        const double* __restrict__ cim, int e_off, int num,
+                                                        const double* __restrict__ Ua,
+                                                        const cplxd* __restrict__ corners, cplxd* __restrict__ gX,
+                                                        double* __restrict__ rows, int* __restrict__ status) {
+    extern __shared__ __align__(16) unsigned char sh_raw[];
+    if ((int)blockIdx.x >= num) return;
+    constexpr int mm2 = m * m, per = pair_complex<m, NEQ>();
+    cplxd* sh = reinterpret_cast<cplxd*>(sh_raw);
+    const int lane = threadIdx.x & 31, side = threadIdx.x >> 5;
+    const int e = e_off + blockIdx.x, K0 = K / 2, KS = side ? K - K0 : K0;
+    cplxd* X = gX + ((size_t)(NEQ ? 2 * blockIdx.x : e) * K + (side ? K0 : 0)) * mm2;
+    const cplxd cc = NEQ && side ? cmk(cim[e], cre[e]) : cmk(cre[e], cim[e]);
+    const bool ok = rs_side<m, NEQ>(side, K, KS, gamma, cmk(Ere[e], Eim[e]), cc, Ua,
+                                    corners + ((size_t)e * 2 + side) * mm2, X, X + (size_t)K * mm2,
+                                    rows + (size_t)e * 2 * K, sh + side * per, sh + (1 - side) * per, lane);
     if (!ok && lane == 0) atomicExch(status, 1);
 }
 
@@ -924,8 +1301,7 @@ __global__ void rs_expand_kernel(const double* __restrict__ U, int N, int m, dou
     if (i < N * m) Ua[i] = U[i / m];
 }
 
-size_t rs_chain_smem_bytes(int m) { return sizeof(cplxd) * (5 * m * m + 3 * kMaxM); }
-size_t rs_chain_neq_smem_bytes(int m) { return sizeof(cplxd) * (9 * m * m + 3 * kMaxM); }
+size_t rs_chain_smem_bytes(int m) { return sizeof(cplxf) * (5 * m * m + 3 * kMaxM); }
 
 }  // namespace
 
@@ -960,39 +1336,51 @@ cudaError_t rs_selftest(int which, int m, int count, const double* d_in, double*
 namespace {
 template <int m>
 cudaError_t launch_rs(int K, double gamma, const double* d_Ere, const double* d_Eim, const double* d_cre,
-                      const double* d_cim, int num_e, int num_neq, const int* d_flags, const double* d_Uatoms,
-                      double Uc0, double Uc1, const RsLeads& leads, void* d_corners, void* d_gL, void* d_gLn,
-                      double* d_rows, double* d_Q, const double* d_sub, int* d_status,
+                      const double* d_cim, int num_e, int num_64, int num_neq, const RsParallel& par,
+                      const double* d_Uatoms, double Uc0, double Uc1, const RsLeads& leads, void* d_corners,
+                      void* d_gL, void* d_gLn, double* d_rows, double* d_Q, const double* d_sub, int* d_status,
                       cudaStream_t stream) {
-    cudaError_t e = cudaFuncSetAttribute(rs_chain_kernel<m>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)rs_chain_smem_bytes(m));
+    const int smem = (int)(2 * sizeof(cplxd) * pair_complex<m, false>());
+    const int smem_neq = (int)(2 * sizeof(cplxd) * pair_complex<m, true>());
+    cudaError_t e = cudaFuncSetAttribute(rs_pair_kernel<m, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return e;
-    e = cudaFuncSetAttribute(rs_chain_neq_kernel<m>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)rs_chain_neq_smem_bytes(m));
+    e = cudaFuncSetAttribute(rs_pair_kernel<m, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_neq);
     if (e != cudaSuccess) return e;
-    const int num_eq = num_e - num_neq;
+    const int num_eq = num_e - num_neq, num_32 = num_eq - num_64;
+    const cplxd* corners = static_cast<const cplxd*>(d_corners);
+    cplxd* gX = static_cast<cplxd*>(d_gL);
     if (num_e > 0) {
-        rs_lead_kernel<m><<<num_e, 32, 0, stream>>>(gamma, d_Ere, d_Eim, num_e, Uc0, Uc1,
-                                                    leads.use_decimation, leads.dec_layers, leads.dec_iters,
-                                                    static_cast<cplxd*>(d_corners));
+        rs_lead_kernel<m><<<num_e, 32, 0, stream>>>(gamma, d_Ere, d_Eim, num_e, Uc0, Uc1, leads.use_decimation,
+                                                    leads.dec_layers, leads.dec_iters, static_cast<cplxd*>(d_corners));
         e = cudaGetLastError();
         if (e != cudaSuccess) return e;
     }
-    if (num_neq > 0) {
-        // the longer chains first
-        rs_chain_neq_kernel<m><<<num_neq, 32, rs_chain_neq_smem_bytes(m), stream>>>(
-            K, gamma, d_Ere, d_Eim, d_cre, d_cim, num_eq, num_neq, d_Uatoms, static_cast<const cplxd*>(d_corners),
-            static_cast<cplxd*>(d_gLn), d_rows, d_status);
-        e = cudaGetLastError();
+    // the FP32 chains beside the FP64 ones
+    const bool fork = num_32 > 0 && num_e > num_32;
+    if (fork) {
+        e = cudaEventRecord(par.fork, stream);
+        if (e == cudaSuccess) e = cudaStreamWaitEvent(par.side, par.fork, 0);
         if (e != cudaSuccess) return e;
     }
-    if (num_eq > 0) {
-        rs_chain_kernel<m><<<num_eq, 32, rs_chain_smem_bytes(m), stream>>>(
-            K, gamma, d_Ere, d_Eim, d_cre, d_cim, num_eq, d_flags, d_Uatoms,
-            static_cast<const cplxd*>(d_corners), static_cast<cplxd*>(d_gL), d_rows, d_status);
-        e = cudaGetLastError();
-        if (e != cudaSuccess) return e;
+    if (num_32 > 0)
+        rs_chain_kernel<m><<<num_32, 32, rs_chain_smem_bytes(m), fork ? par.side : stream>>>(
+            K, gamma, d_Ere, d_Eim, d_cre, d_cim, num_64, num_32, d_Uatoms, corners, gX, d_rows, d_status);
+    // the longer chains first
+    if (num_neq > 0)
+        rs_pair_kernel<m, true><<<num_neq, 64, smem_neq, stream>>>(K, gamma, d_Ere, d_Eim, d_cre, d_cim, num_eq, num_neq,
+                                                                   d_Uatoms, corners, static_cast<cplxd*>(d_gLn),
+                                                                   d_rows, d_status);
+    if (num_64 > 0)
+        rs_pair_kernel<m, false><<<num_64, 64, smem, stream>>>(K, gamma, d_Ere, d_Eim, d_cre, d_cim, 0, num_64, d_Uatoms,
+                                                               corners, gX, d_rows, d_status);
+    e = cudaGetLastError();
+    if (fork) {
+        // joined also after a failed launch, so that a capture ends whole
+        cudaError_t j = cudaEventRecord(par.join, par.side);
+        if (j == cudaSuccess) j = cudaStreamWaitEvent(stream, par.join, 0);
+        if (e == cudaSuccess) e = j;
     }
+    if (e != cudaSuccess) return e;
     const int N = 2 * K;
     rs_reduce_kernel<<<(N + 31) / 32, dim3(32, kRsGroups), 0, stream>>>(d_rows, num_e, N, d_sub, d_Q);
     return cudaGetLastError();
@@ -1000,14 +1388,14 @@ cudaError_t launch_rs(int K, double gamma, const double* d_Ere, const double* d_
 }  // namespace
 
 cudaError_t launch_realspace(int m, int K, double gamma, const double* d_Ere, const double* d_Eim,
-                             const double* d_cre, const double* d_cim, int num_e, int num_neq, const int* d_flags,
+                             const double* d_cre, const double* d_cim, int num_e, int num_64, int num_neq, const RsParallel& par,
                              const double* d_Uatoms, double Uc0, double Uc1, const RsLeads& leads,
                              void* d_corners, void* d_gL, void* d_gLn, double* d_rows, double* d_Q,
                              const double* d_sub, int* d_status, cudaStream_t stream) {
-    if (num_e < 0 || num_neq < 0 || num_neq > num_e || K < 1) return cudaErrorInvalidValue;
+    if (num_64 < 0 || num_neq < 0 || num_64 + num_neq > num_e || K < 2) return cudaErrorInvalidValue;
 #define RS_CASE(M)                                                                                                 \
     case M:                                                                                                        \
-        return launch_rs<M>(K, gamma, d_Ere, d_Eim, d_cre, d_cim, num_e, num_neq, d_flags, d_Uatoms, Uc0,           \
+        return launch_rs<M>(K, gamma, d_Ere, d_Eim, d_cre, d_cim, num_e, num_64, num_neq, par, d_Uatoms, Uc0,      \
                             Uc1, leads, d_corners, d_gL, d_gLn, d_rows, d_Q, d_sub, d_status, stream);
     switch (m) {
         RS_CASE(1) RS_CASE(2) RS_CASE(3) RS_CASE(4) RS_CASE(5) RS_CASE(6) RS_CASE(7) RS_CASE(8)

@@ -220,3 +220,52 @@ def test_ring_modes_equal_ring_blocks(m, cells, bias):
     Qm = g.realspace_charge()
     Qb = g.realspace_charge(U_atoms=torch.tensor(np.repeat(U, m).reshape(-1, m), device="cuda"))
     assert _rel(Qm, Qb) <= TOL, _rel(Qm, Qb)
+
+
+@pytest.mark.parametrize("m,cells", [(13, 3), (6, 2), (1, 3)])
+def test_ring_blocks_near_an_atom_potential(oracle, m, cells):
+    """Poles at 40 K lie 0.011 eV apart and pass every atom's potential within
+    gamma / 100: rings on both sides of the line between the two forms of
+    tr G[b][b] (the diagonal form loses at most 1e4 of 1e-16)."""
+    import torch
+    kw = _eq_kw(m, cells, num_modes=1, contact_T=(40.0, 40.0))
+    n = CNT_sites(kw)
+    g, o = _pair(oracle, U=np.full(n, -0.8), **kw)
+    assert np.sum(np.abs(g.energy_points(2)[0].imag) < 0.025) >= 1
+    Ua = (-0.8 + 0.01 * np.random.default_rng(8).standard_normal((n, m)))
+    Ua[1::4] += 0.5
+    Qg = g.realspace_charge(U_atoms=torch.tensor(Ua, device="cuda"))
+    Qo = o.rs_charge(Uatoms=Ua, nthreads=8)
+    assert _rel(Qg, Qo) <= TOL, _rel(Qg, Qo)
+
+
+def CNT_sites(kw):
+    from electrostatic_b200.negf import CNT
+    return CNT(**kw).num_field_sites
+
+
+def test_ring_blocks_singular_leading_block(oracle):
+    """Atom 0 of the first ring has the potential at which the leading 2 x 2
+    block of the first inversion is singular (to the imaginary part) at one
+    real-axis energy: the sweep hands over to partial pivoting."""
+    import torch
+    m, gamma = 4, 2.5
+    kw = _bias_kw(m, 3, E_zPlus_imag=1e-6)
+    n = CNT_sites(kw)
+    g, o = _pair(oracle, U=np.zeros(n), **kw)
+    E = g.energy_points(3)[0]
+    E = E[np.argmin(np.abs(E.real + 0.15))]
+    beta = 2.0 * gamma * np.cos(np.pi * np.arange(m) / m)
+    # lead: s = (E - gamma^2 s) / (E (E - gamma^2 s) - beta^2), Im s < 0
+    sq = np.array([min(np.roots([-E * gamma**2, E * E - b * b + gamma**2, -E]), key=lambda z: z.imag) for b in beta])
+    s = np.array([(np.cos(2.0 * np.pi * np.arange(m) * d / m) * sq).sum() / m for d in range(m)])
+    d = 1.0 / E  # ring b of the first block is at zero potential
+    a01 = -gamma**2 * (s[1] + d)
+    a11 = E - gamma**2 * (s[0] + 2.0 * d)
+    Ua = np.zeros((n, m))
+    Ua[0, 0] = (E - gamma**2 * (s[0] + 2.0 * d) - a01 * a01 / a11).real
+    b00 = E - Ua[0, 0] - gamma**2 * (s[0] + 2.0 * d)
+    assert abs(b00 * a11 - a01 * a01) < 1e-4 * abs(a01)**2
+    Qg = g.realspace_charge(U_atoms=torch.tensor(Ua, device="cuda"))
+    Qo = o.rs_charge(Uatoms=Ua, nthreads=8)
+    assert _rel(Qg, Qo) <= TOL, _rel(Qg, Qo)
