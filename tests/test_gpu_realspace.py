@@ -269,3 +269,19 @@ def test_ring_blocks_singular_leading_block(oracle):
     Qg = g.realspace_charge(U_atoms=torch.tensor(Ua, device="cuda"))
     Qo = o.rs_charge(Uatoms=Ua, nthreads=8)
     assert _rel(Qg, Qo) <= TOL, _rel(Qg, Qo)
+
+
+@pytest.mark.parametrize("m,cells", [(1, 2), (5, 2), (13, 2), (16, 2)])
+def test_realspace_mixed_many_energies_against_fp64(m, cells):
+    """More FP32 energies than two waves of blocks: the warps' roles swap."""
+    import torch
+    from electrostatic_b200.negf import CNT
+    kw = _eq_kw(m, cells, num_modes=1, eq_integration_pts=(150, 150, 300))
+    g64, g32 = CNT(**kw), CNT(**kw, precision="mixed")
+    n = g64.num_field_sites
+    Ua = 0.1 * np.random.default_rng(m).standard_normal((n, m))
+    for g in (g64, g32):
+        g.set_potential(Ua[:, 0], (Ua[0, 0], Ua[-1, 0]))
+    Ut = torch.tensor(Ua, device="cuda")
+    Q64, Q32 = g64.realspace_charge(U_atoms=Ut), g32.realspace_charge(U_atoms=Ut)
+    assert _rel(Q32, Q64) <= MIXED_TOL, _rel(Q32, Q64)
