@@ -2204,8 +2204,7 @@ int negf_broyden_step(negf_broyden* b, const double* d_n_out, double* d_n_in_out
         if (status) *status = 1;
         return fail(NEGF_ERR_STATE, "Broyden_Step has exceeded the Broyden_Threshold_MaxStep");
     }
-    NEGF_CUDA(negf::broyden_norm(b->dev, d_n_out, s));
-    NEGF_CUDA(negf::broyden_update(b->dev, b->step - 1, s));
+    NEGF_CUDA(negf::broyden_step(b->dev, d_n_out, b->step - 1, s));
     b->step += 1;
     NEGF_CUDA(negf::set_int(b->dev.step_dev, b->step, s));
     if (d_n_in_out)
@@ -2346,20 +2345,14 @@ int negf_broyden_step_number(negf_broyden* b, int* step) {
 
 int negf_broyden_step_device(negf_broyden* b, const double* d_n_out, double max_norm, int* d_flags, void* stream) {
     if (!b || !d_n_out || !d_flags) return fail(NEGF_ERR_ARG, "null argument");
-    cudaStream_t s = (cudaStream_t)stream;
-    NEGF_CUDA(negf::broyden_norm(b->dev, d_n_out, s, d_flags));
-    NEGF_CUDA(negf::broyden_update(b->dev, 0, s, d_flags));
-    NEGF_CUDA(negf::broyden_finish_step(b->dev, max_norm, 0.0, d_flags, s));
+    NEGF_CUDA(negf::broyden_step_device(b->dev, d_n_out, max_norm, 0.0, d_flags, (cudaStream_t)stream));
     return NEGF_OK;
 }
 
 int negf_broyden_step_device_switch(negf_broyden* b, const double* d_n_out, double max_norm, double switch_norm,
                                     int* d_flags, void* stream) {
     if (!b || !d_n_out || !d_flags || !(switch_norm > 0)) return fail(NEGF_ERR_ARG, "bad argument");
-    cudaStream_t s = (cudaStream_t)stream;
-    NEGF_CUDA(negf::broyden_norm(b->dev, d_n_out, s, d_flags));
-    NEGF_CUDA(negf::broyden_update(b->dev, 0, s, d_flags));
-    NEGF_CUDA(negf::broyden_finish_step(b->dev, max_norm, switch_norm, d_flags, s));
+    NEGF_CUDA(negf::broyden_step_device(b->dev, d_n_out, max_norm, switch_norm, d_flags, (cudaStream_t)stream));
     return NEGF_OK;
 }
 

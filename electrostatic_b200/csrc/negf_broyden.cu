@@ -11,6 +11,8 @@
 // Storage: V^T and W as [max_step][S] row-major (row `it` = iteration it),
 // so every dot product and row update is a coalesced sweep over sites.
 
+#include <cooperative_groups.h>
+
 #include "negf_internal.h"
 
 namespace negf {
@@ -198,9 +200,8 @@ __global__ void final_kernel(BroydenDev b, int m_host, const int* flags) {
 // switch_norm sets flags[4] and later steps use the FP64 plan, and only an
 // FP64 charge can end the solve.  flags[5] / flags[6] are the skip words of
 // the low-precision and FP64 plans; flags[7] counts low-precision steps.
-__global__ void step_kernel(BroydenDev b, double max_norm, double switch_norm, int* flags) {
-    if (flags[3]) return;
-    const double nrm = b.scal[0];
+__device__ __forceinline__ void end_step(const BroydenDev& b, double nrm, double max_norm, double switch_norm,
+                                         int* flags) {
     flags[1] += 1;
     const int step = *b.step_dev + 1;
     *b.step_dev = step;
@@ -219,6 +220,143 @@ __global__ void step_kernel(BroydenDev b, double max_norm, double switch_norm, i
         flags[5] = (flags[3] || flags[4]) ? 1 : 0;
         flags[6] = (flags[3] || !flags[4]) ? 1 : 0;
     }
+}
+
+__global__ void step_kernel(BroydenDev b, double max_norm, double switch_norm, int* flags) {
+    if (flags[3]) return;
+    end_step(b, b.scal[0], max_norm, switch_norm, flags);
+}
+
+// A whole step of one segment in one launch (flags null: iteration m_host of a
+// step that the host ends): a cluster of 8 blocks, block r holding sites [r chunk,
+// (r + 1) chunk).  The dot products of the rows with dF and with F are formed in
+// one pass over V (those of the new row dF / |dF|^2 with F from dF . F), the
+// partial sums are added over the cluster in rank order, and one pass over W gives
+// the new row and the new input.  The seven kernels of the general path (norm,
+// finish, dots, row, dots, input, step) are bound by their launches and by chains
+// of one block each; a cluster moves V and W at 8 SMs' rate.  us a step, general /
+// here, at 30 rows: 2800 sites 35 / 13, 16384 sites 63 / 25, 65536 sites 163 / 74;
+// at 60 rows 38 / 15, 69 / 36, 172 / 171: the line kMixSites keeps the general
+// path where a long history (200 rows) makes it the faster one.
+constexpr int kMixBlocks = 8, kMixThreads = 512, kMixSites = 16384;
+namespace cg = cooperative_groups;
+__global__ void __cluster_dims__(kMixBlocks, 1, 1) __launch_bounds__(kMixThreads)
+    mix_kernel(BroydenDev b, const double* __restrict__ n_out, double max_norm, double switch_norm, int* flags,
+               int m_host, int chunk) {
+    if (skipped(flags)) return;  // written by rank 0 after the last read of every block (cluster.sync)
+    extern __shared__ double sh[];
+    const int t = threadIdx.x, lane = t & 31, wid = t >> 5;
+    cg::cluster_group cluster = cg::this_cluster();
+    const int rank = (int)cluster.block_rank();
+    const int m = flags ? *b.step_dev - 1 : m_host, row = (flags ? b.step_dev[1] : b.base) + m;
+    const int R = m > 0 ? row - 1 : row;  // rows in hand
+    double* const mine = sh;              // max, sum of squares, dF.dF, dF.F, then V.dF, V.F per row
+    double* const tot = mine + 4 + 2 * b.max_step;
+    double* const Fs = tot + 4 + 2 * b.max_step;
+    double* const dFs = Fs + chunk;
+    const int lo = min(rank * chunk, b.S), n = min(chunk, b.S - lo);
+    double v[4] = {0.0, 0.0, 0.0, 0.0};
+    for (int i = t; i < n; i += kMixThreads) {
+        const int s = lo + i;
+        const double nin = b.n_in[s], nout = n_out[s];
+        const double Fc = nin - nout;
+        double nr, sq;
+        if (b.norm_type == 0) {
+            nr = fabs(Fc);
+            sq = Fc * Fc;
+        } else {
+            nr = fabs(Fc / (nin + nout));
+            sq = nr * nr;
+        }
+        const double d = Fc - b.F[s];
+        b.norm[s] = nr;
+        b.dF[s] = d;
+        b.F[s] = Fc;
+        Fs[i] = Fc;
+        dFs[i] = d;
+        v[0] = nanmax(v[0], nr);
+        v[1] += sq;
+        v[2] += d * d;
+        v[3] += d * Fc;
+    }
+    __shared__ double red[4][kMixThreads / 32];
+#pragma unroll
+    for (int o = 16; o >= 1; o >>= 1) {
+        v[0] = nanmax(v[0], __shfl_xor_sync(0xffffffffu, v[0], o));
+#pragma unroll
+        for (int k = 1; k < 4; ++k) v[k] += __shfl_xor_sync(0xffffffffu, v[k], o);
+    }
+    if (lane == 0)
+        for (int k = 0; k < 4; ++k) red[k][wid] = v[k];
+    __syncthreads();  // F, dF and the warps' sums
+    if (t < 4) {
+        double a = red[t][0];
+        for (int w = 1; w < kMixThreads / 32; ++w) a = t ? a + red[t][w] : nanmax(a, red[t][w]);
+        mine[t] = a;
+    }
+    for (int it = 1 + wid; it <= R; it += kMixThreads / 32) {
+        const double* __restrict__ V = b.V + (size_t)it * b.S + lo;
+        double a1 = 0.0, a2 = 0.0;
+#pragma unroll 4
+        for (int i = lane; i < n; i += 32) {
+            const double x = V[i];
+            a1 += x * dFs[i];
+            a2 += x * Fs[i];
+        }
+#pragma unroll
+        for (int o = 16; o >= 1; o >>= 1) {
+            a1 += __shfl_xor_sync(0xffffffffu, a1, o);
+            a2 += __shfl_xor_sync(0xffffffffu, a2, o);
+        }
+        if (lane == 0) {
+            mine[2 + 2 * it] = a1;
+            mine[3 + 2 * it] = a2;
+        }
+    }
+    cluster.sync();
+    for (int i = t; i < 4 + 2 * R; i += kMixThreads) {
+        double a = *cluster.map_shared_rank(mine + i, 0);
+        for (int r = 1; r < kMixBlocks; ++r) {
+            const double x = *cluster.map_shared_rank(mine + i, r);
+            a = i ? a + x : nanmax(a, x);
+        }
+        tot[i] = a;
+    }
+    __syncthreads();
+    const double denom = tot[2], cn = denom > 0.0 ? tot[3] / denom : 0.0;
+    for (int i = t; i < n; i += kMixThreads) {
+        const int s = lo + i;
+        const double* __restrict__ W = b.W + s;
+        double a1 = 0.0, a2 = 0.0;
+#pragma unroll 8
+        for (int it = 1; it <= R; ++it) {
+            const double x = W[(size_t)it * b.S];
+            a1 += x * tot[2 + 2 * it];
+            a2 += x * tot[3 + 2 * it];
+        }
+        const double nin = b.n_in[s];
+        if (m > 0) {
+            const double dF = dFs[i];
+            // a zero step adds no direction (newrow_kernel)
+            const double w = -b.fraction * dF + (nin - b.n_prev[s]) - a1;
+            b.V[(size_t)row * b.S + s] = denom > 0.0 ? dF / denom : 0.0;
+            b.W[(size_t)row * b.S + s] = w;
+            a2 += w * cn;
+        }
+        b.sum[s] = a2;
+        b.n_prev[s] = nin;
+        b.n_in[s] = nin - b.scalar * b.fraction * Fs[i] - b.scalar * a2;
+    }
+    if (rank == 0) {
+        for (int it = 1 + t; it <= row; it += kMixThreads) b.c[it] = it <= R ? tot[3 + 2 * it] : cn;
+        if (t == 0) {
+            b.scal[0] = tot[0];
+            b.scal[1] = sqrt(tot[1]);
+            b.scal[2] = tot[2];
+            if (flags) end_step(b, tot[0], max_norm, switch_norm, flags);
+        }
+    }
+    cluster.sync();  // no block leaves while its sums are read
 }
 
 __global__ void set_int_kernel(int* p, int v) { *p = v; }
@@ -332,23 +470,31 @@ cudaError_t affine_toeplitz(const double* tab, int ntab, const int* idx, const d
     return cudaGetLastError();
 }
 
-cudaError_t broyden_norm(const BroydenDev& b, const double* n_out, cudaStream_t s, const int* flags) {
-    norm_kernel<<<b.nblocks, kThreads, 0, s>>>(b, n_out, flags);
-    norm_finalize<<<1, 32, 0, s>>>(b, flags);
+namespace {
+// One cluster while it is the faster form (see mix_kernel) and the rows' sums fit its shared memory.
+bool mix_fits(const BroydenDev& b, int& chunk, size_t& smem) {
+    chunk = (b.S + kMixBlocks - 1) / kMixBlocks;
+    smem = sizeof(double) * (2 * (4 + 2 * (size_t)b.max_step) + 2 * (size_t)chunk);
+    return b.nseg == 1 && b.S <= kMixSites && smem <= 200 * 1024;
+}
+cudaError_t mix(const BroydenDev& b, const double* n_out, double max_norm, double switch_norm, int* flags, int m_host,
+                int chunk, size_t smem, cudaStream_t s) {
+    const cudaError_t e = cudaFuncSetAttribute(mix_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    mix_kernel<<<kMixBlocks, kMixThreads, smem, s>>>(b, n_out, max_norm, switch_norm, flags, m_host, chunk);
     return cudaGetLastError();
 }
+void norm(const BroydenDev& b, const double* n_out, const int* flags, cudaStream_t s) {
+    norm_kernel<<<b.nblocks, kThreads, 0, s>>>(b, n_out, flags);
+    norm_finalize<<<1, 32, 0, s>>>(b, flags);
+}
+}  // namespace
 
-cudaError_t broyden_update(const BroydenDev& b, int m, cudaStream_t s, const int* flags) {
-    if (b.step_dev && flags) {
-        // device-resident: shapes cover every m up to max_step, rows above m return
-        const dim3 g(b.max_step > 1 ? b.max_step : 1, b.nseg);
-        dots_kernel<<<g, kThreads, 0, s>>>(b, b.dF, 0, 0, flags);
-        if (b.nseg > 1) segsq_kernel<<<b.nseg, kThreads, 0, s>>>(b, 0, flags);
-        newrow_kernel<<<b.nblocks, kThreads, 0, s>>>(b, 0, flags);
-        dots_kernel<<<g, kThreads, 0, s>>>(b, b.F, 0, 1, flags);
-        final_kernel<<<b.nblocks, kThreads, 0, s>>>(b, 0, flags);
-        return cudaGetLastError();
-    }
+cudaError_t broyden_step(const BroydenDev& b, const double* n_out, int m, cudaStream_t s) {
+    int chunk;
+    size_t smem;
+    if (mix_fits(b, chunk, smem)) return mix(b, n_out, 0.0, 0.0, nullptr, m, chunk, smem, s);
+    norm(b, n_out, nullptr, s);
     if (m > 0) {
         if (b.base + m - 1 >= 1) dots_kernel<<<dim3(b.base + m - 1, b.nseg), kThreads, 0, s>>>(b, b.dF, m, 0, nullptr);
         if (b.nseg > 1) segsq_kernel<<<b.nseg, kThreads, 0, s>>>(b, m, nullptr);
@@ -359,7 +505,19 @@ cudaError_t broyden_update(const BroydenDev& b, int m, cudaStream_t s, const int
     return cudaGetLastError();
 }
 
-cudaError_t broyden_finish_step(const BroydenDev& b, double max_norm, double switch_norm, int* flags, cudaStream_t s) {
+cudaError_t broyden_step_device(const BroydenDev& b, const double* n_out, double max_norm, double switch_norm, int* flags,
+                                cudaStream_t s) {
+    int chunk;
+    size_t smem;
+    if (mix_fits(b, chunk, smem)) return mix(b, n_out, max_norm, switch_norm, flags, 0, chunk, smem, s);
+    norm(b, n_out, flags, s);
+    // shapes cover every m up to max_step, rows above m return
+    const dim3 g(b.max_step > 1 ? b.max_step : 1, b.nseg);
+    dots_kernel<<<g, kThreads, 0, s>>>(b, b.dF, 0, 0, flags);
+    if (b.nseg > 1) segsq_kernel<<<b.nseg, kThreads, 0, s>>>(b, 0, flags);
+    newrow_kernel<<<b.nblocks, kThreads, 0, s>>>(b, 0, flags);
+    dots_kernel<<<g, kThreads, 0, s>>>(b, b.F, 0, 1, flags);
+    final_kernel<<<b.nblocks, kThreads, 0, s>>>(b, 0, flags);
     step_kernel<<<1, 1, 0, s>>>(b, max_norm, switch_norm, flags);
     return cudaGetLastError();
 }

@@ -275,11 +275,11 @@ struct BroydenDev {
     int* seg_of;      // device int[S]: segment of each site (nseg > 1)
     double* dd;       // [nseg]: per-segment dF^T dF
 };
-cudaError_t broyden_norm(const BroydenDev& b, const double* n_out, cudaStream_t s, const int* flags = nullptr);
-cudaError_t broyden_update(const BroydenDev& b, int m, cudaStream_t s, const int* flags = nullptr);
-// Device-resident step end: flags int[4] = converged, iterations, error
-// (1 MaxStep exceeded, 2 non-finite norm), skip; advances *step_dev.
-cudaError_t broyden_finish_step(const BroydenDev& b, double max_norm, double switch_norm, int* flags, cudaStream_t s);
+// One mixing step (iteration m), and a device-resident one with its end: flags int[4] = converged, iterations,
+// error (1 MaxStep exceeded, 2 non-finite norm), skip; advances *step_dev.
+cudaError_t broyden_step(const BroydenDev& b, const double* n_out, int m, cudaStream_t s);
+cudaError_t broyden_step_device(const BroydenDev& b, const double* n_out, double max_norm, double switch_norm, int* flags,
+                                cudaStream_t s);
 cudaError_t set_int(int* p, int v, cudaStream_t s);
 cudaError_t broyden_set(double* p, double v, int n, cudaStream_t s);
 cudaError_t affine_potential(const double* K, const double* U0, const double* Q, double* U, int n, cudaStream_t s,
