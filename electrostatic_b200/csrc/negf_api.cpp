@@ -745,16 +745,6 @@ int auto_pieces(int nw, int max_N) {
     return nw >= target / 2 ? 1 : std::min(maxp, (target + nw - 1) / std::max(nw, 1));
 }
 
-// Boundary states of the FP64 chains by the scan over segments (parallel in
-// length) rather than by sweeps.  A sweep of few chains takes its N dependent
-// steps, 17 ns a site; the scan takes 3 us more to start and then works at 8.4
-// ps per site and chain (measured: 4000 sites and 512 chains 27 us against 73
-// us by sweeps, 4096 chains 138 us against 78 us, 400 sites and 228 chains 14
-// us against 17 us).
-bool scan_better(long long site_chains, int max_N) {
-    return 3.0 + 8.4e-6 * double(site_chains) < 0.017 * max_N;
-}
-
 int choose_schedule(int setting, int nw, int pieces) {
     if (pieces > 1) return negf::kScheduleTwoPass;
     if (setting == NEGF_SCHEDULE_FUSED) return negf::kScheduleFused;
@@ -916,13 +906,73 @@ long long group_state_doubles(const negf::GroupDev& g) {
     return (long long)((g.nch + 31) / 32) * g.nblk * (g.kind == negf::kRealAxis ? 6 : 4) * 256;
 }
 
+// How the boundary states of a launch are formed: whole sweeps, sweeps in pieces
+// of `sites` (a multiple of 128, 0: whole), or the scan over segments.
+struct StatesPlan {
+    bool scan = false;
+    int sites = 0;
+};
+// By the estimated time in us (measured on (17,0) tubes; site_chains = sum of
+// chains x sites):
+//   whole sweeps  N dependent steps, 17 ns a site, or 1.1 ps per site and chain;
+//   in pieces     two launches and the carry over the pieces, 30 ns a site of a
+//                 piece (matrices, then both sweeps) and 0.2 us a piece, or 2.2 ps
+//                 per site and chain; pieces fill at most 8 warps per SM;
+//   scan          10 ps per site and chain behind a shorter start.
+// Measured, whole / pieces / scan: 64000 sites and 230 chains 1120 / 60 / 153 us,
+// 16000 sites and 1300 chains 279 / 73 / 138, 4000 sites and 35 chains 69 / 17 / 8,
+// 604 sites and 1200 chains 14 / 14 / 11, 1600 sites and 9000 chains 33 / 50 / 93.
+StatesPlan plan_states(const negf::GroupDev* g, int n, int setting) {
+    StatesPlan p;
+    double site_chains = 0.0;
+    int max_N = 0;
+    for (int i = 0; i < n; ++i) {
+        site_chains += double(g[i].nch) * g[i].N;
+        max_N = std::max(max_N, g[i].N);
+    }
+    p.scan = setting > 1;
+    if (setting != 0) return p;
+    double best = 3.5 + std::max(0.017 * max_N, 1.1e-6 * site_chains);
+    const long long slots = 8LL * device_sm_count();
+    for (int L = 128; L < max_N; L += 128) {
+        // pieces have to gain a tenth on whole sweeps
+        const double t = 1.1 * (10.0 + std::max(0.030 * L + 0.2 * max_N / L, 2.2e-6 * site_chains));
+        if (t >= best) {
+            if (0.030 * L > best) break;
+            continue;
+        }
+        long long warps = 0;
+        for (int i = 0; i < n; ++i) warps += 2LL * ((g[i].nch + 31) / 32) * ((g[i].N + L - 1) / L);
+        if (warps > slots) continue;
+        best = t;
+        p.sites = L;
+    }
+    p.scan = 4.0 + 10e-6 * site_chains < best;
+    if (p.scan) p.sites = 0;
+    return p;
+}
+// A group's pieces of L sites (0: one), its blocks in range_kernel and its matrices.
+void place_pieces(negf::GroupDev& g, int L, negf::SweepShape& sh, long long& tm_doubles) {
+    g.piece_segs = L ? L / negf::kSweepSeg : g.nseg;
+    g.pieces = (g.nseg + g.piece_segs - 1) / g.piece_segs;
+    if (g.pieces > 1 && g.nseg - (g.pieces - 1) * g.piece_segs < 2) --g.pieces;  // the last segment overlaps its neighbour
+    const int cw = (g.nch + 31) / 32;
+    g.range_base = sh.range_blocks;
+    g.tm_off = tm_doubles;
+    if (g.pieces > 1) {
+        sh.range_blocks += cw * (g.pieces + 2);
+        tm_doubles += (long long)cw * (g.pieces * 9 + 4) * 32;
+    }
+    g.sweep_base = sh.sweep_blocks;
+    sh.sweep_blocks += 2 * cw * g.pieces;
+}
+
 // Groups of the FP64 chains of a launch, longest tubes first.  pieces: the
 // setting (0 automatic, 1 sweeps, more: parallel in length).
 void plan_groups(SweepPart& sp, const TubePass* passes, const negf::TubeDev* tdev, int num_passes, int pieces) {
     std::vector<int> order(num_passes);
     longest_first(passes, num_passes, order.data());
-    long long work = 0, site_chains = 0;  // chain x segment-block iterations of seg_kernel
-    int max_N = 0;
+    long long work = 0;  // chain x segment-block iterations of seg_kernel
     for (int o : order) {
         const ChainSet& cs = *sp.sets[o];
         const int k = tdev[o].N < negf::kSweepSeg ? 1 : 0;
@@ -937,12 +987,12 @@ void plan_groups(SweepPart& sp, const TubePass* passes, const negf::TubeDev* tde
             const int cpw = 32 / g.lanes;
             work += (long long)g.nsb * ((g.nch + cpw - 1) / cpw);
             sp.chains += g.nch;
-            site_chains += (long long)g.nch * g.N;
             sp.warps += (g.nch + 31) / 32;
-            max_N = std::max(max_N, g.N);
         }
     }
-    sp.scan = pieces > 1 || (pieces == 0 && scan_better(site_chains, max_N));
+    // tubes of fewer than kSweepSeg sites alone: sweeps of a few steps
+    const StatesPlan states = plan_states(sp.groups[0].data(), (int)sp.groups[0].size(), pieces);
+    sp.scan = states.scan;
     // Units of seg_kernel: whole waves of the 11 warps an SM holds, of at most
     // 32 chain iterations each (a unit costs about 3 us to start and 0.6 us
     // per iteration; fewer and longer units also mean fewer partial rows).
@@ -956,10 +1006,9 @@ void plan_groups(SweepPart& sp, const TubePass* passes, const negf::TubeDev* tde
         int max_nseg = 1;
         for (negf::GroupDev& g : sp.groups[k]) {
             g.chains_per_unit = iters * (32 / g.lanes);
-            g.sweep_base = sh.sweep_blocks;
+            place_pieces(g, k ? 0 : states.sites, sh, sp.tm_doubles);
             g.chain_base = sh.chains;
             g.seg_base = sh.seg_blocks;
-            sh.sweep_blocks += 2 * ((g.nch + 31) / 32);
             sh.chains += g.nch;
             sh.seg_blocks += g.nsb * ((g.nch + g.chains_per_unit - 1) / g.chains_per_unit);
             g.ck_off = sp.ck_doubles;
@@ -992,12 +1041,11 @@ int place_rows(SweepPart& sp, int pass, int N, long long& row, TableCounts& cnt)
     return rows;
 }
 
-// Pieces a chain runs in: its segments when parallel in length, else one sweep.
+// Pieces a chain runs in: its segments by the scan, else the pieces of its sweep.
 int reported_pieces(const SweepPart& sp) {
     int n = 1;
-    if (sp.scan)
-        for (const std::vector<negf::GroupDev>& v : sp.groups)
-            for (const negf::GroupDev& g : v) n = std::max(n, g.nseg);
+    for (const std::vector<negf::GroupDev>& v : sp.groups)
+        for (const negf::GroupDev& g : v) n = std::max(n, sp.scan ? g.nseg : g.pieces);
     return n;
 }
 
@@ -1010,6 +1058,7 @@ negf::GroupSet group_set(const std::vector<negf::GroupDev>& v, const negf::Group
         gs.sweep_base[i] = v[i].sweep_base;
         gs.chain_base[i] = v[i].chain_base;
         gs.seg_base[i] = v[i].seg_base;
+        gs.range_base[i] = v[i].range_base;
     }
     if (gs.ng > 2)
         gs.ext = dev;
@@ -1349,14 +1398,17 @@ int transport_run(negf_tube& t, const std::vector<Pt>& pts, std::vector<double>&
     g.nsb = (g.nseg + 31) / 32;
     negf::SweepShape sh{};
     sh.K = K;
-    sh.scan = scan_better((long long)g.nch * N, N);
+    const StatesPlan states = plan_states(&g, K == negf::kSweepSeg ? 1 : 0, 0);
+    sh.scan = states.scan;
     sh.chains = g.nch;
-    sh.sweep_blocks = 2 * ((g.nch + 31) / 32);
+    long long tm_doubles = 0;
+    place_pieces(g, states.sites, sh, tm_doubles);
     sh.scan_threads = std::min(512, (g.nseg + 31) / 32 * 32);
     if (g.nseg > sh.scan_threads) g.tm_segs = g.nseg;
     NEGF_CUDA(W.ck.reserve(sizeof(double) * group_state_doubles(g)));
     NEGF_CUDA(W.cc.reserve(sizeof(double) * (size_t)g.nch * negf::kConst));
-    if (sh.scan) NEGF_CUDA(W.tm.reserve(std::max<size_t>(1, sizeof(double) * 9 * (size_t)g.nch * g.tm_segs)));
+    if (sh.scan) tm_doubles = 9LL * g.nch * g.tm_segs;
+    NEGF_CUDA(W.tm.reserve(sizeof(double) * std::max<long long>(1, tm_doubles)));
     const size_t nred = (size_t)P * 8, npart = (size_t)P * g.nsb;
     NEGF_CUDA(W.trOut.reserve(sizeof(double) * (nred + npart)));
     if (ldos) NEGF_CUDA(W.trLdos.reserve(sizeof(double) * (size_t)P * N));

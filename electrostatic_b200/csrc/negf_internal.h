@@ -98,9 +98,11 @@ struct __align__(16) GroupDev {
     long long ck_off;    // boundary states (layout in negf_sweep.cu)
     long long cc_off;    // constants [chain][kConst]
     long long row_base;  // first partial row (one per unit of chains)
-    int sweep_base, chain_base, seg_base;    // first block of the group in each kernel
+    int sweep_base, chain_base, seg_base, range_base;  // first block of the group in each kernel
     int chains_per_unit, nsb, lanes;         // seg_kernel: chains of a unit, segment blocks, segments side by side in a warp
     int tm_segs;                             // scan_kernel: matrices per chain in its scratch
+    int pieces, piece_segs;                  // sweeps in pieces of piece_segs segments (a multiple of 8)
+    long long tm_off;                        // pieces > 1: their transfer matrices
     int pad;
     double beta[kMaxModes], degen[kMaxModes];
 };
@@ -112,13 +114,14 @@ constexpr int kMaxBases = 64;
 struct GroupSet {
     const GroupDev* ext;
     int ng;
-    int sweep_base[kMaxBases], chain_base[kMaxBases], seg_base[kMaxBases];
+    int sweep_base[kMaxBases], chain_base[kMaxBases], seg_base[kMaxBases], range_base[kMaxBases];
     GroupDev g[2];
 };
 struct SweepShape {
     int K;                  // kSweepSeg or 2
     int scan;               // boundary states by scan_kernel (parallel in length) instead of sweep_kernel
     int chains, scan_threads, sweep_blocks, seg_blocks;
+    int range_blocks;       // > 0: sweeps in pieces (range_kernel first)
 };
 cudaError_t launch_sweep(const GroupSet& gs, const SweepShape& sh, double* ck, double* cc, double* tm, double* partial,
                          const int* skip, cudaStream_t s, cudaEvent_t mid);

@@ -27,7 +27,9 @@
 // Two phases.  First the boundary states (y, lambda) at the first site and
 // (x, rho) at the last site of every K-site segment, by one of
 //   sweep_kernel  lane = chain, one warp per 32 chains and direction: 6 FP64
-//                 instructions a site, N dependent steps (many chains);
+//                 instructions a site, N dependent steps (many chains); or one
+//                 per piece of the tube as well, behind range_kernel, which
+//                 forms the pieces' transfer matrices (long tubes);
 //   scan_kernel   thread = segment, one block per chain: the 2 x 2 transfer
 //                 matrix of every segment, a scan over them in registers
 //                 (parallel in length: few chains).
@@ -166,194 +168,7 @@ __device__ __forceinline__ void lin_step(Lin& s, double ar, double ai, double r,
     s.qi = nqi;
 }
 
-// ------------------------------------------------------------------ boundary states: sweeps
-// A warp sweeps 32 chains of one group in one direction (even block: forward,
-// odd: backward), stores the normalised state of every segment boundary in a
-// shared tile of 8 segments and writes full 64-byte pieces of the chains' rows
-// [component][segment], the layout that seg_kernel reads with lane = segment.
-// Bound: 7 FP64 instructions a site and chain (6 of the step, 1 of the
-// boundary); one direction per warp doubles the warps of the pass (the
-// dependent chain of a step is two FMAs, 16 cycles against 12 issue cycles,
-// so it takes two or more warps per scheduler to fill the FP64 pipe).
-// The potentials travel through a shared ring of four tiles of 64 steps
-// (cp.async, one 16-byte pair of sites per lane and tile), since ptxas moves
-// loads into registers to their use: a lone warp then took 63 cycles a site.
-constexpr int kRing = 256, kTile = 64;
-struct __align__(128) SweepShared {
-    double tile[3 * kBlk];
-    double ring[kRing];
-};
-// Bulk copy of shared memory to global memory (16-byte aligned, a multiple of
-// 16 bytes) by one lane, after the other lanes' writes were made visible to
-// the async proxy; bulk_read_done: the shared source may be rewritten.
-__device__ __forceinline__ void fence_async_proxy() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
-__device__ __forceinline__ void bulk_store(double* dst, const double* src, unsigned bytes) {
-    asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(dst),
-                 "r"((unsigned)__cvta_generic_to_shared(src)), "r"(bytes)
-                 : "memory");
-    asm volatile("cp.async.bulk.commit_group;" ::: "memory");
-}
-__device__ __forceinline__ void bulk_read_done() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
-__device__ __forceinline__ void bulk_done() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
-
-template <int K, bool BACK, bool RA>
-__device__ __forceinline__ void sweep_chain(const GroupDev& g, int w, SweepShared& sm, double* __restrict__ ck,
-                                            double* __restrict__ cc) {
-    constexpr int NC = RA ? 6 : 4, ROWS = NC / 2;
-    const int lane = threadIdx.x;
-    const int N = g.N, nseg = g.nseg, nblk = g.nblk;
-    const int c = min(w * kWarp + lane, g.nch - 1);
-    const double* __restrict__ U = g.U;
-    const int tail = N - (nseg - 1) * K;  // sites of the natural last segment, in [2, K]
-    const bool cut = tail < K;
-    // Step m of a sweep: forward at site m, backward at site N - 1 - m (the parities agree since N is
-    // even).  Position m + off of the ring holds it, pairs of steps in site order; off makes every full
-    // segment start at a multiple of K, so that its loads have constant offsets.
-    const int off = BACK && cut ? K - tail : 0;
-    auto fetch = [&](int t) {
-        const int p = t * kTile + 2 * lane, m = p - off;
-        if (m >= 0 && m < N) cp_async16(&sm.ring[p & (kRing - 1)], U + (BACK ? N - 2 - m : m));
-        cp_async_commit();
-    };
-    fetch(0);
-    fetch(1);
-    fetch(2);
-    const ChainIn ch = load_chain(g, c);
-    const cd sig = sigma_over_gamma(g, ch, BACK);
-    if (w * kWarp + lane < g.nch) write_constants(g, ch, sig, BACK, cc + g.cc_off + (long long)c * kConst);
-    const double ig = 1.0 / g.gamma, Eg = ch.e.Er * ig, ei = ch.e.Ei * ig, r = ch.beta * ch.beta * ig * ig;
-    double* __restrict__ out = ck + g.ck_off + ((long long)w * nblk * NC + (BACK ? ROWS : 0)) * kBlk;
-    Lin s{sig.x, sig.y, 1.0, 0.0};
-    // The record (p / q, lambda) of a boundary is formed beside the first half of the next segment's
-    // steps and the running state is scaled by rq = 1 / |q_b|^2 after them: issue is in order, so a
-    // record formed at the boundary itself would hold up the recurrence for its whole chain.  With that
-    // scaling the moduli telescope to lambda_{b+1} = lambda_b prod(rho) rq_b rq_{b+1}.
-    double lam = 1.0, rq = 1.0, yr, yi;
-    auto record = [&](const Lin& t, double rprod) {
-        const double q1 = rcp(fma(t.qr, t.qr, t.qi * t.qi));
-        yr = fma(t.pr, t.qr, t.pi * t.qi) * q1;
-        yi = fma(t.pi, t.qr, -t.pr * t.qi) * q1;
-        if (RA) lam *= rprod * rq * q1;
-        rq = q1;
-    };
-    auto scale = [&]() {
-        s.pr *= rq;
-        s.pi *= rq;
-        s.qr *= rq;
-        s.qi *= rq;
-    };
-    bool first = true;  // the tile's first segment: the bulk copy of the previous tile must have read it
-    auto store = [&](int seg) {
-        if (first) {
-            if (lane == 0) bulk_read_done();
-            __syncwarp();
-            first = false;
-        }
-        double* t = sm.tile + lane * 8 + ((seg ^ lane) & 7);
-        t[0] = yr;
-        t[kBlk] = yi;
-        if (RA) t[2 * kBlk] = lam;
-        if (BACK ? (seg & 7) == 0 : ((seg & 7) == 7 || seg == nseg - 1)) {
-            fence_async_proxy();
-            __syncwarp();
-            if (lane == 0) bulk_store(out + (long long)(seg >> 3) * (NC * kBlk), sm.tile, ROWS * kBlk * sizeof(double));
-            first = true;
-        }
-    };
-    // tiles T and T + 1 are complete while the sweep is in tile T
-    int tile = 0, pos = off;
-    auto enter = [&]() {
-        if (pos / kTile > tile) {
-            tile = pos / kTile;
-            __syncwarp();  // every lane has left the tile whose slot is filled next
-            fetch(tile + 2);
-            cp_async_wait<1>();
-            __syncwarp();
-        }
-    };
-    cp_async_wait<1>();
-    __syncwarp();
-    double rseg = 1.0;  // product of rho over a full segment
-#pragma unroll
-    for (int j = 0; j < K / 2; ++j) rseg *= r;
-    // a of the two steps at position p
-    auto pair = [&](int p) {
-        const double2 v = *reinterpret_cast<const double2*>(&sm.ring[p & (kRing - 1)]);
-        return make_double2(fma(BACK ? -v.y : -v.x, ig, Eg), fma(BACK ? -v.x : -v.y, ig, Eg));
-    };
-    double rprod = 1.0;  // product of rho since the previous boundary
-    // the shortened step to (forward) or from (backward) the last segment
-    auto shorter = [&]() {
-        enter();
-        record(s, rprod);
-        scale();
-        rprod = 1.0;
-        for (int j = 0; j < tail; j += 2) {
-            const double2 a = pair(pos + j);
-            lin_step(s, a.x, ei, r, false);
-            lin_step(s, a.y, ei, r, true);
-            rprod *= r;
-        }
-        pos += tail;
-    };
-    int seg = BACK ? nseg - 1 : 0;
-    if (BACK && cut) {
-        shorter();
-        store(seg--);
-    }
-    double2 a = pair(pos);  // one pair ahead
-    for (int k = nseg - 1 - (cut ? 1 : 0); k > 0; --k) {
-        enter();
-        const Lin t = s;
-        const double* at = &sm.ring[pos & (kRing - 1)];
-        auto two = [&](int j) {
-            const double2 v = *reinterpret_cast<const double2*>(j + 2 < K ? at + j + 2 : &sm.ring[(pos + K) & (kRing - 1)]);
-            lin_step(s, a.x, ei, r, false);
-            lin_step(s, a.y, ei, r, true);
-            a = make_double2(fma(BACK ? -v.y : -v.x, ig, Eg), fma(BACK ? -v.x : -v.y, ig, Eg));
-        };
-#pragma unroll
-        for (int j = 0; j < K / 2; j += 2) two(j);
-        record(t, rprod);
-        scale();
-#pragma unroll
-        for (int j = (K / 2 + 1) / 2 * 2; j < K; j += 2) two(j);
-        store(seg);
-        rprod = rseg;
-        pos += K;
-        seg += BACK ? -1 : 1;
-    }
-    if (!BACK && cut) {  // from (nseg - 2) K to N - K
-        shorter();
-        store(seg++);
-    }
-    record(s, rprod);
-    store(seg);
-    cp_async_wait<0>();
-    if (lane == 0) bulk_done();  // the copies read this block's shared memory
-}
-
-template <int K>
-__global__ void __launch_bounds__(32, 16) sweep_kernel(const __grid_constant__ GroupSet gs, double* __restrict__ ck,
-                                                       double* __restrict__ cc, const int* __restrict__ skip) {
-    if (skip && *skip) return;
-    __shared__ __align__(16) SweepShared sm;
-    const GroupDev& g = group(gs, find_group<&GroupDev::sweep_base>(gs, gs.sweep_base, blockIdx.x));
-    const int rel = blockIdx.x - g.sweep_base, w = rel >> 1;
-    if (g.kind == kRealAxis) {
-        if (rel & 1)
-            sweep_chain<K, true, true>(g, w, sm, ck, cc);
-        else
-            sweep_chain<K, false, true>(g, w, sm, ck, cc);
-    } else {
-        if (rel & 1)
-            sweep_chain<K, true, false>(g, w, sm, ck, cc);
-        else
-            sweep_chain<K, false, false>(g, w, sm, ck, cc);
-    }
-}
-
-// ------------------------------------------------------------------ boundary states: scan over segments
+// ------------------------------------------------------------------ transfer matrices
 // Transfer matrix of a run of sites, scaled to determinant 1 (by the
 // square root of its product of rho, so that lambda needs no powers of r) and
 // then to entries of order 1 by 2^-e:
@@ -396,7 +211,7 @@ __device__ __forceinline__ void tm_apply(const Tm& m, bool back, cd& Z, double& 
     const cd k1 = back ? m.B : m.C, k2 = back ? m.C : m.B;
     const cd num = {fma(-m.D.x, Z.x, fma(m.D.y, Z.y, k1.x)), fma(-m.D.x, Z.y, fma(-m.D.y, Z.x, k1.y))};
     const cd den = {fma(-k2.x, Z.x, fma(k2.y, Z.y, m.A.x)), fma(-k2.x, Z.y, fma(-k2.y, Z.x, m.A.y))};
-    const double iq = 1.0 / fma(den.x, den.x, den.y * den.y);
+    const double iq = rcp(fma(den.x, den.x, den.y * den.y));
     Z = {fma(num.x, den.x, num.y * den.y) * iq, fma(num.y, den.x, -num.x * den.y) * iq};
     lam *= iq;
     const int e2 = -2 * m.e;  // lambda 2^(-2 e), in two factors inside the exponent range
@@ -404,6 +219,360 @@ __device__ __forceinline__ void tm_apply(const Tm& m, bool back, cd& Z, double& 
     lam *= pow2d(h);
     lam *= pow2d(h2);
 }
+
+// Pieces of a group's chains (pieces > 1): [chains / 32][piece][9][32] matrices,
+// then [2][2][32] contact self-energies.
+__device__ __forceinline__ long long tm_at(const GroupDev& g, int w, int piece) {
+    return g.tm_off + ((long long)w * (g.pieces * 9 + 4) + piece * 9) * 32;
+}
+// The state before a piece: the contact's through the n pieces between, their
+// matrices in a ring of kCarry shared stages (an L2 latency from load to use).  The
+// state stays a pair (P, Q), scaled by the exponent of the pair before, so that an
+// application is a chain of four FMAs and a product; one division at the end.
+constexpr int kCarry = 8, kCarryStage = 9 * 32;
+template <bool BACK, bool RA>
+__device__ __forceinline__ void carry(const GroupDev& g, int w, int n, const double* __restrict__ tm, cd& Z,
+                                      double& lam) {
+    extern __shared__ __align__(16) double carry_ring[];
+    const int lane = threadIdx.x;
+    auto copy = [&](int j) {
+        if (j < n) {
+            const double* src = tm + tm_at(g, w, BACK ? g.pieces - 1 - j : j) + 2 * lane;
+            double* dst = carry_ring + j % kCarry * kCarryStage + 2 * lane;
+#pragma unroll
+            for (int q = 0; q < 4; ++q) cp_async16(dst + 64 * q, src + 64 * q);
+            if (lane < 16) cp_async16(dst + 256, src + 256);
+        }
+        cp_async_commit();
+    };
+    for (int j = 0; j < kCarry; ++j) copy(j);
+    const double* sig = tm + tm_at(g, w, g.pieces) + (BACK ? 64 : 0) + lane;
+    cd P = {sig[0], sig[32]}, Q = {1.0, 0.0};
+    auto exponent = [&]() {  // of the larger of P and Q, 0 when there is none
+        auto hi = [](double x) { return __double2hiint(x) & 0x7fffffff; };
+        const int be = max(max(hi(P.x), hi(P.y)), max(hi(Q.x), hi(Q.y))) >> 20;
+        return be > 0 && be < 0x7fe ? be - 1023 : 0;
+    };
+    int e = 0;  // the pair times 2^e
+    for (int j = 0; j < n; ++j) {
+        cp_async_wait<kCarry - 1>();
+        __syncwarp();
+        const double* q = carry_ring + j % kCarry * kCarryStage + lane;
+        const cd A = {q[0], q[32]}, D = {q[192], q[224]};
+        const cd k1 = BACK ? cd{q[64], q[96]} : cd{q[128], q[160]}, k2 = BACK ? cd{q[128], q[160]} : cd{q[64], q[96]};
+        const int x = exponent();
+        const double f = pow2d(-x);
+        e += x + (int)q[256];
+        const cd p = cms(k1, Q, cmul(D, P)), d = cms(A, Q, cmul(k2, P));
+        P = cscale(f, p);
+        Q = cscale(f, d);
+        __syncwarp();
+        copy(j + kCarry);
+    }
+    cp_async_wait<0>();
+    const int x = exponent();
+    P = cscale(pow2d(-x), P);
+    Q = cscale(pow2d(-x), Q);
+    const double iq = rcp(fma(Q.x, Q.x, Q.y * Q.y));
+    Z = {fma(P.x, Q.x, P.y * Q.y) * iq, fma(P.y, Q.x, -P.x * Q.y) * iq};
+    // lambda = 2^(-2 e) / |Q|^2, the power in two factors inside the exponent range
+    const int e2 = -2 * (e + x), h = max(-1000, min(1000, e2 / 2)), h2 = max(-1000, min(1000, e2 - e2 / 2));
+    lam = RA ? iq * pow2d(h) * pow2d(h2) : 1.0;
+}
+
+// ------------------------------------------------------------------ boundary states: sweeps
+// A warp sweeps 32 chains of one group in one direction (even block: forward,
+// odd: backward), stores the normalised state of every segment boundary in a
+// shared tile of 8 segments and writes full 64-byte pieces of the chains' rows
+// [component][segment], the layout that seg_kernel reads with lane = segment.
+// Bound: 7 FP64 instructions a site and chain (6 of the step, 1 of the
+// boundary); one direction per warp doubles the warps of the pass (the
+// dependent chain of a step is two FMAs, 16 cycles against 12 issue cycles,
+// so it takes two or more warps per scheduler to fill the FP64 pipe).
+// The potentials travel through a shared ring of four tiles of 64 steps
+// (cp.async, one 16-byte pair of sites per lane and tile), since ptxas moves
+// loads into registers to their use: a lone warp then took 63 cycles a site.
+constexpr int kRing = 256, kTile = 64;
+struct __align__(128) SweepShared {
+    double tile[3 * kBlk];
+    double ring[kRing];
+};
+// Bulk copy of shared memory to global memory (16-byte aligned, a multiple of
+// 16 bytes) by one lane, after the other lanes' writes were made visible to
+// the async proxy; bulk_read_done: the shared source may be rewritten.
+__device__ __forceinline__ void fence_async_proxy() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
+__device__ __forceinline__ void bulk_store(double* dst, const double* src, unsigned bytes) {
+    asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(dst),
+                 "r"((unsigned)__cvta_generic_to_shared(src)), "r"(bytes)
+                 : "memory");
+    asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+}
+__device__ __forceinline__ void bulk_read_done() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
+__device__ __forceinline__ void bulk_done() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
+
+template <int K, bool BACK, bool RA>
+__device__ __forceinline__ void sweep_chain(const GroupDev& g, int w, int piece, SweepShared& sm,
+                                            double* __restrict__ ck, double* __restrict__ cc,
+                                            const double* __restrict__ tm) {
+    constexpr int NC = RA ? 6 : 4, ROWS = NC / 2;
+    const int lane = threadIdx.x;
+    const int N = g.N, nseg = g.nseg, nblk = g.nblk;
+    const int c = min(w * kWarp + lane, g.nch - 1);
+    const double* __restrict__ U = g.U;
+    const int tail = N - (nseg - 1) * K;  // sites of the natural last segment, in [2, K]
+    const bool cut = tail < K;
+    // Step m of a sweep: forward at site m, backward at site N - 1 - m (the parities agree since N is
+    // even).  Position m + off of the ring holds it, pairs of steps in site order; off makes every full
+    // segment start at a multiple of K, so that its loads have constant offsets.
+    const int off = BACK && cut ? K - tail : 0;
+    auto fetch = [&](int t) {
+        const int p = t * kTile + 2 * lane, m = p - off;
+        if (m >= 0 && m < N) cp_async16(&sm.ring[p & (kRing - 1)], U + (BACK ? N - 2 - m : m));
+        cp_async_commit();
+    };
+    // this piece: segments [s_lo, s_hi), from the contact or from the pieces before it
+    const int W = g.pieces, s_lo = piece * g.piece_segs;
+    const bool last = piece == W - 1;
+    const int s_hi = last ? nseg : s_lo + g.piece_segs;
+    int pos = BACK ? (last ? off : (nseg - s_hi) * K) : s_lo * K, tile = pos / kTile;
+    for (int t = 0; t < 3; ++t) fetch(tile + t);
+    const ChainIn ch = load_chain(g, c);
+    cd start;
+    double lam = 1.0;
+    if (W > 1) {
+        carry<BACK, RA>(g, w, BACK ? W - 1 - piece : piece, tm, start, lam);
+    } else {
+        start = sigma_over_gamma(g, ch, BACK);
+        if (w * kWarp + lane < g.nch) write_constants(g, ch, start, BACK, cc + g.cc_off + (long long)c * kConst);
+    }
+    const double ig = 1.0 / g.gamma, Eg = ch.e.Er * ig, ei = ch.e.Ei * ig, r = ch.beta * ch.beta * ig * ig;
+    double* __restrict__ out = ck + g.ck_off + ((long long)w * nblk * NC + (BACK ? ROWS : 0)) * kBlk;
+    Lin s{start.x, start.y, 1.0, 0.0};
+    // The record (p / q, lambda) of a boundary is formed beside the first half of the next segment's
+    // steps and the running state is scaled by rq = 1 / |q_b|^2 after them: issue is in order, so a
+    // record formed at the boundary itself would hold up the recurrence for its whole chain.  With that
+    // scaling the moduli telescope to lambda_{b+1} = lambda_b prod(rho) rq_b rq_{b+1}.
+    double rq = 1.0, yr, yi;
+    auto record = [&](const Lin& t, double rprod) {
+        const double q1 = rcp(fma(t.qr, t.qr, t.qi * t.qi));
+        yr = fma(t.pr, t.qr, t.pi * t.qi) * q1;
+        yi = fma(t.pi, t.qr, -t.pr * t.qi) * q1;
+        if (RA) lam *= rprod * rq * q1;
+        rq = q1;
+    };
+    auto scale = [&]() {
+        s.pr *= rq;
+        s.pi *= rq;
+        s.qr *= rq;
+        s.qi *= rq;
+    };
+    bool first = true;  // the tile's first segment: the bulk copy of the previous tile must have read it
+    auto store = [&](int seg) {
+        if (first) {
+            if (lane == 0) bulk_read_done();
+            __syncwarp();
+            first = false;
+        }
+        double* t = sm.tile + lane * 8 + ((seg ^ lane) & 7);
+        t[0] = yr;
+        t[kBlk] = yi;
+        if (RA) t[2 * kBlk] = lam;
+        if (BACK ? (seg & 7) == 0 : ((seg & 7) == 7 || seg == nseg - 1)) {
+            fence_async_proxy();
+            __syncwarp();
+            if (lane == 0) bulk_store(out + (long long)(seg >> 3) * (NC * kBlk), sm.tile, ROWS * kBlk * sizeof(double));
+            first = true;
+        }
+    };
+    // tiles T and T + 1 are complete while the sweep is in tile T
+    auto enter = [&]() {
+        if (pos / kTile > tile) {
+            tile = pos / kTile;
+            __syncwarp();  // every lane has left the tile whose slot is filled next
+            fetch(tile + 2);
+            cp_async_wait<1>();
+            __syncwarp();
+        }
+    };
+    cp_async_wait<1>();
+    __syncwarp();
+    double rseg = 1.0;  // product of rho over a full segment
+#pragma unroll
+    for (int j = 0; j < K / 2; ++j) rseg *= r;
+    // a of the two steps at position p
+    auto pair = [&](int p) {
+        const double2 v = *reinterpret_cast<const double2*>(&sm.ring[p & (kRing - 1)]);
+        return make_double2(fma(BACK ? -v.y : -v.x, ig, Eg), fma(BACK ? -v.x : -v.y, ig, Eg));
+    };
+    double rprod = 1.0;  // product of rho since the previous boundary
+    // the shortened step to (forward) or from (backward) the last segment
+    auto shorter = [&]() {
+        enter();
+        record(s, rprod);
+        scale();
+        rprod = 1.0;
+        for (int j = 0; j < tail; j += 2) {
+            const double2 a = pair(pos + j);
+            lin_step(s, a.x, ei, r, false);
+            lin_step(s, a.y, ei, r, true);
+            rprod *= r;
+        }
+        pos += tail;
+    };
+    int seg = BACK ? s_hi - 1 : s_lo;
+    const bool end = cut && last;
+    if (BACK && end) {
+        shorter();
+        store(seg--);
+    }
+    double2 a = pair(pos);  // one pair ahead
+    for (int k = s_hi - s_lo - 1 - (end ? 1 : 0); k > 0; --k) {
+        enter();
+        const Lin t = s;
+        const double* at = &sm.ring[pos & (kRing - 1)];
+        auto two = [&](int j) {
+            const double2 v = *reinterpret_cast<const double2*>(j + 2 < K ? at + j + 2 : &sm.ring[(pos + K) & (kRing - 1)]);
+            lin_step(s, a.x, ei, r, false);
+            lin_step(s, a.y, ei, r, true);
+            a = make_double2(fma(BACK ? -v.y : -v.x, ig, Eg), fma(BACK ? -v.x : -v.y, ig, Eg));
+        };
+#pragma unroll
+        for (int j = 0; j < K / 2; j += 2) two(j);
+        record(t, rprod);
+        scale();
+#pragma unroll
+        for (int j = (K / 2 + 1) / 2 * 2; j < K; j += 2) two(j);
+        store(seg);
+        rprod = rseg;
+        pos += K;
+        seg += BACK ? -1 : 1;
+    }
+    if (!BACK && end) {  // from (nseg - 2) K to N - K
+        shorter();
+        store(seg++);
+    }
+    record(s, rprod);
+    store(seg);
+    cp_async_wait<0>();
+    if (lane == 0) bulk_done();  // the copies read this block's shared memory
+}
+
+template <int K>
+__global__ void __launch_bounds__(32, 16) sweep_kernel(const __grid_constant__ GroupSet gs, double* __restrict__ ck,
+                                                       double* __restrict__ cc, const double* __restrict__ tm,
+                                                       const int* __restrict__ skip) {
+    if (skip && *skip) return;
+    __shared__ __align__(16) SweepShared sm;
+    const GroupDev& g = group(gs, find_group<&GroupDev::sweep_base>(gs, gs.sweep_base, blockIdx.x));
+    const int rel = blockIdx.x - g.sweep_base, w = (rel >> 1) / g.pieces, piece = (rel >> 1) % g.pieces;
+    if (g.kind == kRealAxis) {
+        if (rel & 1)
+            sweep_chain<K, true, true>(g, w, piece, sm, ck, cc, tm);
+        else
+            sweep_chain<K, false, true>(g, w, piece, sm, ck, cc, tm);
+    } else {
+        if (rel & 1)
+            sweep_chain<K, true, false>(g, w, piece, sm, ck, cc, tm);
+        else
+            sweep_chain<K, false, false>(g, w, piece, sm, ck, cc, tm);
+    }
+}
+
+// ------------------------------------------------------------------ boundary states: sweeps in pieces
+// Transfer matrix of one piece (lane = chain, a warp per 32 chains and piece): two
+// columns a site, 11 FP64 instructions, normalised at every segment with its part
+// of the determinant.  Two more warps form the contact self-energies and the
+// chain constants.  Bound by the steps of a piece, 12 ns a site, behind 4 us of
+// start.  64000 sites and 230 chains: 20 us and 40 us of sweeps in pieces, against
+// 153 us of scan_kernel and 1120 us of whole sweeps.
+template <int K>
+__global__ void __launch_bounds__(32, 16) range_kernel(const __grid_constant__ GroupSet gs, double* __restrict__ cc,
+                                                       double* __restrict__ tm, const int* __restrict__ skip) {
+    if (skip && *skip) return;
+    __shared__ __align__(16) double ring[kRing];
+    const GroupDev& g = group(gs, find_group<&GroupDev::range_base>(gs, gs.range_base, blockIdx.x));
+    const int rel = blockIdx.x - g.range_base, w = rel / (g.pieces + 2), piece = rel % (g.pieces + 2);
+    const int lane = threadIdx.x, N = g.N, c = min(w * kWarp + lane, g.nch - 1);
+    const int s_lo = piece * g.piece_segs, s_hi = piece == g.pieces - 1 ? g.nseg : s_lo + g.piece_segs;
+    const ChainIn ch = load_chain(g, c);
+    if (piece >= g.pieces) {  // contact self-energies and chain constants, beside the matrices
+        const int side = piece - g.pieces;
+        const cd sig = sigma_over_gamma(g, ch, side);
+        if (w * kWarp + lane < g.nch) write_constants(g, ch, sig, side, cc + g.cc_off + (long long)c * kConst);
+        double* o = tm + tm_at(g, w, g.pieces) + 64 * side + lane;
+        o[0] = sig.x;
+        o[32] = sig.y;
+        return;
+    }
+    auto fetch = [&](int t) {
+        const int p = t * kTile + 2 * lane;
+        if (p < N) cp_async16(&ring[p & (kRing - 1)], g.U + p);
+        cp_async_commit();
+    };
+    int tile = s_lo * K / kTile;
+    for (int t = 0; t < 3; ++t) fetch(tile + t);
+    const double ig = 1.0 / g.gamma, Eg = ch.e.Er * ig, ei = ch.e.Ei * ig, r = ch.beta * ch.beta * ig * ig;
+    // r^(-1/2), bounded: a vanishing beta decouples the sites and its lambda is 0 to working precision;
+    // its power over a segment as mantissa and exponent
+    const double hs = 1.0 / fmax(fabs(ch.beta) * ig, 1e-30);
+    auto part = [&](int len, double& mant, int& ex) {
+        double f = 1.0;
+        for (int j = 0; j < len / 2; ++j) f *= hs;
+        const long long b = __double_as_longlong(f);
+        ex = (int)((b >> 52) & 0x7ff) - 1023;
+        mant = __longlong_as_double((b & 0xfffffffffffffll) | (1023ll << 52));
+    };
+    double mant;
+    int ex, e = 0;
+    part(K, mant, ex);
+    Lin c1{1.0, 0.0, 0.0, 0.0}, c2{0.0, 0.0, 1.0, 0.0};
+    auto normalise = [&]() {
+        auto hi = [](double x) { return __double2hiint(x) & 0x7fffffff; };
+        const int be = max(max(max(hi(c1.pr), hi(c1.pi)), max(hi(c1.qr), hi(c1.qi))),
+                           max(max(hi(c2.pr), hi(c2.pi)), max(hi(c2.qr), hi(c2.qi)))) >> 20;
+        const bool scale = be > 0 && be < 0x7fe;  // else zero, subnormal, inf or NaN: leave as is
+        const double f = scale ? mant * pow2d(1023 - be) : mant;
+        e += ex + (scale ? be - 1023 : 0);
+        c1 = {c1.pr * f, c1.pi * f, c1.qr * f, c1.qi * f};
+        c2 = {c2.pr * f, c2.pi * f, c2.qr * f, c2.qi * f};
+    };
+    cp_async_wait<1>();
+    __syncwarp();
+    for (int s = s_lo; s < s_hi; ++s) {
+        const int n0 = s * K;
+        if (n0 / kTile > tile) {
+            tile = n0 / kTile;
+            __syncwarp();  // every lane has left the tile whose slot is filled next
+            fetch(tile + 2);
+            cp_async_wait<1>();
+            __syncwarp();
+        }
+        const double* at = &ring[n0 & (kRing - 1)];
+        auto two = [&](int j) {
+            const double2 v = *reinterpret_cast<const double2*>(at + j);
+            const double a0 = fma(-v.x, ig, Eg), a1 = fma(-v.y, ig, Eg);
+            lin_step(c1, a0, ei, r, false);
+            lin_step(c2, a0, ei, r, false);
+            lin_step(c1, a1, ei, r, true);
+            lin_step(c2, a1, ei, r, true);
+        };
+        if (n0 + K <= N) {
+#pragma unroll
+            for (int j = 0; j < K; j += 2) two(j);
+        } else {
+            for (int j = 0; j < N - n0; j += 2) two(j);
+            part(N - n0, mant, ex);
+        }
+        normalise();
+    }
+    cp_async_wait<0>();
+    const double v[9] = {c2.qr, c2.qi, -c1.qr, -c1.qi, c2.pr, c2.pi, -c1.pr, -c1.pi, (double)e};
+    double* o = tm + tm_at(g, w, piece) + lane;
+#pragma unroll
+    for (int k = 0; k < 9; ++k) o[32 * k] = v[k];
+}
+
+// ------------------------------------------------------------------ boundary states: scan over segments
 __device__ __forceinline__ Tm tm_shfl(const Tm& m, int src) {
     Tm o;
     o.A = {__shfl_sync(kFull, m.A.x, src), __shfl_sync(kFull, m.A.y, src)};
@@ -846,7 +1015,11 @@ cudaError_t launch_states(const GroupSet& gs, const SweepShape& sh, double* ck, 
     if (sh.scan)
         scan_kernel<K><<<sh.chains, sh.scan_threads, 0, s>>>(gs, ck, cc, tm, skip);
     else
-        sweep_kernel<K><<<sh.sweep_blocks, 32, 0, s>>>(gs, ck, cc, skip);
+    {
+        const size_t smem = sh.range_blocks > 0 ? sizeof(double) * kCarry * kCarryStage : 0;
+        if (sh.range_blocks > 0) range_kernel<K><<<sh.range_blocks, 32, 0, s>>>(gs, cc, tm, skip);
+        sweep_kernel<K><<<sh.sweep_blocks, 32, smem, s>>>(gs, ck, cc, tm, skip);
+    }
     return cudaGetLastError();
 }
 template <int K>

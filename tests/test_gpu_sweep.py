@@ -132,3 +132,32 @@ def test_transport_segments_match_oracle(oracle, tid, cells):
     I, probes, _ = g.Compute_Current(integrand=True)
     oI, oprobes = o.current(nthreads=8, probes=True)
     assert _rel(I, oI) <= FP64_TOL and _rel(probes, oprobes) <= FP64_TOL
+
+
+@pytest.mark.parametrize("cells", [4000, 4001, 4036, 5125])
+def test_sweeps_in_pieces(pieces, cells):
+    """Long tubes of a middling number of chains: sweeps in pieces (chosen by the
+    estimate) against whole ones, with a last piece of one segment more, whole and
+    overlapping last segments, the mode of a vanishing hopping and a short tube in
+    the same launch.  1e-11: one rounding per site of the matrices (2e4 eps = 5e-12)."""
+    import torch
+    from electrostatic_b200.negf import CNT, ChargePlan
+    from electrostatic_b200.workloads import site_potential
+
+    def tube(type_id, n, modes, seed):
+        t = CNT(type_id=type_id, num_unitcells=n, num_modes=modes, contact_mu=(0.0, -0.2), contact_T=(300.0, 300.0),
+                eq_integration_pts=(16, 16, 32), noneq_integration_pts=(70,), E_zPlus_imag=1e-3)
+        U = site_potential(t.site_positions(), seed, amp=0.2, ramp=0.2)
+        t.set_potential(U, (U[0], U[-1]))
+        return t
+    tubes = [tube((16, 0), cells, 8, 3), tube((17, 0), 40, 2, 4), tube((17, 0), 3, 2, 5)]
+    pieces(SWEEP)
+    ref = [t.Solve_NEGF() for t in tubes]
+    pieces(0)
+    assert _rel(tubes[0].Solve_NEGF(), ref[0]) <= 1e-11
+    Q = torch.zeros(sum(len(r) for r in ref), dtype=torch.float64, device="cuda")
+    plan = ChargePlan(tubes, Q)
+    assert 1 < plan.info()["pieces"] < 200
+    plan.launch()
+    torch.cuda.synchronize()
+    assert _rel(Q.cpu().numpy(), np.concatenate(ref)) <= 1e-11
