@@ -11,6 +11,8 @@ through the C-ABI of libnegf_b200.so; there is no Python or CPU compute path.
 from __future__ import annotations
 
 import ctypes as C
+import threading
+import weakref
 from typing import Sequence
 
 import numpy as np
@@ -32,6 +34,63 @@ def _ptr(x):
     if isinstance(x, int):
         return C.c_void_p(x)
     return C.c_void_p(x.data_ptr())
+
+
+class _ResultPool:
+    """Page-locked memory of large host results.  A result in fresh pageable
+    memory costs its page faults, the driver's staging copy and the unmapping
+    when it dies: with 4.8 MB of a local density of states 0.98 ms for density of
+    states and current, 0.38 ms here; 0.51 MB of charge 0.30 and 0.19 ms.  A block
+    goes back to the pool when its array and every view of it are gone.  Blocks
+    are powers of two, at most LIMIT bytes in all, free and in use; past that, and
+    below SMALL, results are ordinary arrays.  release_scratch() hands the free
+    blocks back."""
+
+    SMALL, LIMIT = 1 << 16, 1 << 26
+
+    def __init__(self):
+        self._lock = threading.RLock()  # finalizers may run inside any allocation
+        self._free: dict[int, list] = {}
+        self._bytes = 0
+
+    def array(self, n: int) -> np.ndarray:
+        """float64[n] for a call that writes all of it."""
+        if 8 * n < self.SMALL or 8 * n > self.LIMIT // 4:
+            return np.zeros(n)
+        import torch
+        size = 1 << (8 * n - 1).bit_length()
+        with self._lock:
+            blocks = self._free.get(size)
+            block = blocks.pop() if blocks else None
+            if block is None:
+                if self._bytes + size > self.LIMIT:
+                    self.clear()
+                if self._bytes + size > self.LIMIT:
+                    return np.zeros(n)
+                self._bytes += size
+        if block is None:
+            try:
+                block = torch.empty(size // 8, dtype=torch.float64, pin_memory=True)
+            except RuntimeError:
+                with self._lock:
+                    self._bytes -= size
+                return np.zeros(n)
+        memory = (C.c_double * n).from_address(block.data_ptr())  # base of the array and of all its views
+        weakref.finalize(memory, self._give, size, block).atexit = False
+        return np.frombuffer(memory)
+
+    def _give(self, size, block):
+        with self._lock:
+            self._free.setdefault(size, []).append(block)
+
+    def clear(self):
+        with self._lock:
+            for size, blocks in self._free.items():
+                self._bytes -= size * len(blocks)
+            self._free.clear()
+
+
+_results = _ResultPool()
 
 
 def _stream(stream):
@@ -311,7 +370,7 @@ class CNT:
         E = np.zeros(2 * P)
         dos, T, cond = np.zeros(P), np.zeros(P), np.zeros(P)
         tot = np.zeros(1)
-        ld = np.zeros(P * self.num_field_sites) if ldos else None
+        ld = _results.array(P * self.num_field_sites) if ldos else None
         check(L.negf_compute_dos(self._h, _dptr(E), _dptr(dos), _dptr(T), _dptr(cond), _dptr(tot),
                                  None if ld is None else ld.ctypes.data_as(C.c_void_p), _stream(stream)),
               "negf_compute_dos")
@@ -362,7 +421,7 @@ def compute_charge(tubes: Sequence[CNT], out=None, stream=None):
     arr = (C.c_void_p * len(tubes))(*[t.handle for t in tubes])
     total = sum(t.num_field_sites for t in tubes)
     if out is None:
-        Q = np.zeros(total)
+        Q = _results.array(total)
         check(L.negf_compute_charge(arr, len(tubes), Q.ctypes.data_as(C.c_void_p), 0, _stream(stream)),
               "negf_compute_charge")
         return Q
@@ -373,7 +432,8 @@ def compute_charge(tubes: Sequence[CNT], out=None, stream=None):
 def release_scratch(stream=None):
     """negf_release_scratch: hand back the device scratch that the charge
     calls keep for the current device and `stream` (reallocated by the next
-    call on that stream)."""
+    call on that stream), and the free page-locked blocks of host results."""
+    _results.clear()
     check(_lib.load().negf_release_scratch(_stream(stream)), "negf_release_scratch")
 
 
