@@ -182,6 +182,10 @@ __device__ __forceinline__ cd cms(cd a, cd b, cd c) {  // a b - c
     return {fma(a.x, b.x, fma(-a.y, b.y, -c.x)), fma(a.x, b.y, fma(a.y, b.x, -c.y))};
 }
 __device__ __forceinline__ double pow2d(int e) { return __longlong_as_double((long long)(e + 1023) << 52); }
+// A power of two f with f^2 x in [1/4, 2), from the exponent of x >= 0.
+__device__ __forceinline__ double inv_root2(double x) {
+    return __hiloint2double((int)((0xbfd00000u - (unsigned)__double2hiint(x)) >> 1 & 0x7ff00000u), 0);
+}
 __device__ __forceinline__ void tm_normalise(Tm& m) {
     const double s = fmax(fmax(fabs(m.A.x) + fabs(m.A.y), fabs(m.B.x) + fabs(m.B.y)),
                           fmax(fabs(m.C.x) + fabs(m.C.y), fabs(m.D.x) + fabs(m.D.y)));
@@ -349,22 +353,25 @@ __device__ __forceinline__ void sweep_chain(const GroupDev& g, int w, int piece,
     double* __restrict__ out = ck + g.ck_off + ((long long)w * nblk * NC + (BACK ? ROWS : 0)) * kBlk;
     Lin s{start.x, start.y, 1.0, 0.0};
     // The record (p / q, lambda) of a boundary is formed beside the first half of the next segment's
-    // steps and the running state is scaled by rq = 1 / |q_b|^2 after them: issue is in order, so a
-    // record formed at the boundary itself would hold up the recurrence for its whole chain.  With that
-    // scaling the moduli telescope to lambda_{b+1} = lambda_b prod(rho) rq_b rq_{b+1}.
-    double rq = 1.0, yr, yi;
+    // steps and the running state is scaled by f, a power of two next to 1 / |q_b|, after them: issue is
+    // in order, so a record formed at the boundary itself would hold up the recurrence for its whole
+    // chain.  The moduli telescope to lambda_{b+1} = lambda_b prod(rho) (f_b |q_b|)^2 / |q_{b+1}|^2.
+    // (Scaled by 1 / |q_b|^2, a step would take |q_b| to G_b / |q_b|: standing waves of the period of two
+    // segments, G_b large and small by turns, then grow it without bound, to inf after some 100 of them.)
+    double f = 1.0, w2 = 1.0, yr, yi;  // w2 = (f |q_b|)^2
     auto record = [&](const Lin& t, double rprod) {
-        const double q1 = rcp(fma(t.qr, t.qr, t.qi * t.qi));
+        const double q2 = fma(t.qr, t.qr, t.qi * t.qi), q1 = rcp(q2);
         yr = fma(t.pr, t.qr, t.pi * t.qi) * q1;
         yi = fma(t.pi, t.qr, -t.pr * t.qi) * q1;
-        if (RA) lam *= rprod * rq * q1;
-        rq = q1;
+        if (RA) lam *= rprod * w2 * q1;
+        f = inv_root2(q2);
+        if (RA) w2 = q2 * f * f;
     };
     auto scale = [&]() {
-        s.pr *= rq;
-        s.pi *= rq;
-        s.qr *= rq;
-        s.qi *= rq;
+        s.pr *= f;
+        s.pi *= f;
+        s.qr *= f;
+        s.qi *= f;
     };
     bool first = true;  // the tile's first segment: the bulk copy of the previous tile must have read it
     auto store = [&](int seg) {
