@@ -168,7 +168,7 @@ struct Proj {
     R pr, pi, qr, qi;  // P, Q (scaled projective state)
     R lam;             // lambda (or rho) at the last segment boundary
     R H;               // product of h^2 since the last segment boundary
-    R rq;              // 1 / |Q|^2 at the last segment boundary
+    R f, w2;           // scaling of the last segment boundary's state and |f Q|^2 there (FP64)
 };
 
 // Linear step with hopping square h2 at a site of potential u (interior
@@ -211,14 +211,18 @@ __device__ __forceinline__ void proj_step_edge(const Chain<R>& c, Proj<R>& p, R 
 }
 // Segment boundary, off the recurrence's critical path: the checkpoint
 // Y = P / Q and lambda from a snapshot of the state; the running state is
-// rescaled by rq = 1 / |Q_b|^2 half a segment later.  With that scaling the
-// telescoped moduli give lambda_{b+K} = lambda_b prod(h^2) rq_b rq_{b+K}.
+// rescaled by f, a power of two next to 1 / |Q_b|, half a segment later.  The
+// telescoped moduli give lambda_{b+K} = lambda_b prod(h^2) |f Q_b|^2 / |Q_{b+K}|^2.
+// (Scaled by 1 / |Q_b|^2, a segment would take |Q_b| to G_b / |Q_b|: standing
+// waves with the period of two segments, G_b large and small by turns, then
+// grow it without bound, to inf after some 100 of them.)
 // FP32 renormalises at the boundary itself (state := (Y, 1)): the deferred
-// scaling lets |Q| swing to |Q_b|^-2 between boundaries, which can leave the
-// FP32 range when |alpha - Y| is near its floor Im E.
+// scaling lets |Q| swing between boundaries, which can leave the FP32 range
+// when |alpha - Y| is near its floor Im E.
 template <typename R, bool RA>
 __device__ __forceinline__ void proj_boundary(Proj<R>& p, R& yr, R& yi) {
-    const R rq = rcp(p.qr * p.qr + p.qi * p.qi);
+    const R q2 = p.qr * p.qr + p.qi * p.qi;
+    const R rq = rcp(q2);
     yr = (p.pr * p.qr + p.pi * p.qi) * rq;
     yi = (p.pi * p.qr - p.pr * p.qi) * rq;
     if constexpr (sizeof(R) == 4) {
@@ -228,18 +232,20 @@ __device__ __forceinline__ void proj_boundary(Proj<R>& p, R& yr, R& yi) {
         p.qr = 1;
         p.qi = 0;
     } else {
-        if (RA) p.lam = p.lam * (p.H * p.rq * rq);
-        p.rq = rq;
+        if (RA) p.lam = p.lam * (p.H * p.w2 * rq);
+        // from the exponent of q2: w2 in [1/4, 2)
+        p.f = __hiloint2double((int)((0xbfd00000u - (unsigned)__double2hiint(q2)) >> 1 & 0x7ff00000u), 0);
+        p.w2 = q2 * p.f * p.f;
     }
     p.H = 1;
 }
 template <typename R>
 __device__ __forceinline__ void proj_scale(Proj<R>& p) {
     if constexpr (sizeof(R) == 8) {
-        p.pr *= p.rq;
-        p.pi *= p.rq;
-        p.qr *= p.rq;
-        p.qi *= p.rq;
+        p.pr *= p.f;
+        p.pi *= p.f;
+        p.qr *= p.f;
+        p.qi *= p.f;
     }
 }
 
@@ -391,8 +397,8 @@ __device__ __forceinline__ void pass1_chain(const TubeDev* __restrict__ tubes, c
     }
     const Chain<R> c = make_chain<R, RA>(T, cr, S0.x, S0.y, S1.x, S1.y);
     R* __restrict__ ck = reinterpret_cast<R*>(wscratch + 4 * kWarp) + lane;
-    Proj<R> f{(R)st.yr, (R)st.yi, 1, 0, (R)st.lam, 1, 1};
-    Proj<R> b{(R)st.xr, (R)st.xi, 1, 0, (R)st.rho, 1, 1};
+    Proj<R> f{(R)st.yr, (R)st.yi, 1, 0, (R)st.lam, 1, 1, 1};
+    Proj<R> b{(R)st.xr, (R)st.xi, 1, 0, (R)st.rho, 1, 1, 1};
     R hfull = 1;  // prod of h^2 over a full segment
 #pragma unroll
     for (int j = 0; j < K / 2; ++j) hfull *= c.hb2 * c.hg2;
@@ -978,8 +984,8 @@ __device__ __forceinline__ void fused_chain(const TubeDev* __restrict__ tubes, c
         return {p[0], p[kWarp], RA ? p[2 * kWarp] : (R)1};
     };
     const int A = nseg / 2;
-    Proj<R> f{0, 0, 1, 0, 1, 1, 1};  // Y_0 = 0, lambda_0 = 1
-    Proj<R> b{0, 0, 1, 0, 1, 1, 1};  // X_{N-1} = 0, rho_{N-1} = 1
+    Proj<R> f{0, 0, 1, 0, 1, 1, 1, 1};  // Y_0 = 0, lambda_0 = 1
+    Proj<R> b{0, 0, 1, 0, 1, 1, 1, 1};  // X_{N-1} = 0, rho_{N-1} = 1
     // ---- phase A
     if (A > 0) {
         R hfull = 1;  // prod of h^2 over a full segment

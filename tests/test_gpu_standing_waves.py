@@ -55,3 +55,33 @@ def test_flat_channel_sweeps(oracle, tuning, cells, u):
         tuning(TUNE_PASS1_PIECES, P)
         Qg = g.Solve_NEGF()
         assert np.all(np.isfinite(Qg)) and _rel(Qg, Qo) <= FP64_TOL, (P, _rel(Qg, Qo))
+
+
+MIXED_TOL = 1e-5
+
+
+@pytest.mark.parametrize("cells,u", CASES)
+def test_flat_channel_fused(oracle, tuning, cells, u):
+    from electrostatic_b200.negf import SCHEDULE_FUSED, TUNE_SCHEDULE
+    g, Qo = _tube_and_oracle(oracle, cells, u)
+    tuning(TUNE_SCHEDULE, SCHEDULE_FUSED)
+    Qg = g.Solve_NEGF()
+    assert np.all(np.isfinite(Qg)) and _rel(Qg, Qo) <= FP64_TOL, _rel(Qg, Qo)
+
+
+@pytest.mark.parametrize("cells,u", CASES)
+def test_flat_channel_fp64_chains_of_a_mixed_tube(oracle, tuning, cells, u):
+    """Mostly FP32 work: the FP64 chains near the axis ride along, in both schedules."""
+    from electrostatic_b200.negf import CNT, SCHEDULE_FUSED, SCHEDULE_TWO_PASS, TUNE_SCHEDULE
+    kw = dict(type_id=(17, 0), num_unitcells=cells, num_modes=2, contact_mu=(0.0, -0.3), contact_T=(300.0, 300.0),
+              eq_integration_pts=(900, 900, 1500), noneq_integration_pts=(3072,), E_zPlus_imag=1e-5)
+    o = oracle.OracleTube(**kw)
+    g = CNT(**kw, precision="mixed")
+    U = _flat(g.num_field_sites, u)
+    for t in (g, o):
+        t.set_potential(U, (0.0, 0.0))
+    Qo = o.charge(nthreads=8)
+    for schedule in (SCHEDULE_FUSED, SCHEDULE_TWO_PASS):
+        tuning(TUNE_SCHEDULE, schedule)
+        Qg = g.Solve_NEGF()
+        assert np.all(np.isfinite(Qg)) and _rel(Qg, Qo) <= MIXED_TOL, (schedule, _rel(Qg, Qo))
