@@ -472,14 +472,16 @@ cudaError_t affine_toeplitz(const double* tab, int ntab, const int* idx, const d
 
 namespace {
 // One cluster while it is the faster form (see mix_kernel) and the rows' sums fit its shared memory.
+constexpr int kMixShared = 200 * 1024;
 bool mix_fits(const BroydenDev& b, int& chunk, size_t& smem) {
     chunk = (b.S + kMixBlocks - 1) / kMixBlocks;
     smem = sizeof(double) * (2 * (4 + 2 * (size_t)b.max_step) + 2 * (size_t)chunk);
-    return b.nseg == 1 && b.S <= kMixSites && smem <= 200 * 1024;
+    return b.nseg == 1 && b.S <= kMixSites && smem <= kMixShared;
 }
 cudaError_t mix(const BroydenDev& b, const double* n_out, double max_norm, double switch_norm, int* flags, int m_host,
                 int chunk, size_t smem, cudaStream_t s) {
-    const cudaError_t e = cudaFuncSetAttribute(mix_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    // the limit belongs to the kernel, not to the launch: the same for every mixer, since other threads launch theirs
+    const cudaError_t e = cudaFuncSetAttribute(mix_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMixShared);
     if (e != cudaSuccess) return e;
     mix_kernel<<<kMixBlocks, kMixThreads, smem, s>>>(b, n_out, max_norm, switch_norm, flags, m_host, chunk);
     return cudaGetLastError();
