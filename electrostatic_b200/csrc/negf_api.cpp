@@ -1054,11 +1054,14 @@ int reported_pieces(const SweepPart& sp) {
 negf::GroupSet group_set(const std::vector<negf::GroupDev>& v, const negf::GroupDev* dev) {
     negf::GroupSet gs{};
     gs.ng = (int)v.size();
-    for (int i = 0; i < std::min(gs.ng, negf::kMaxBases); ++i) {
-        gs.sweep_base[i] = v[i].sweep_base;
-        gs.chain_base[i] = v[i].chain_base;
-        gs.seg_base[i] = v[i].seg_base;
-        gs.range_base[i] = v[i].range_base;
+    gs.stride = std::max(1, (gs.ng + negf::kMaxBases - 1) / negf::kMaxBases);
+    gs.nbases = (gs.ng + gs.stride - 1) / gs.stride;
+    for (int i = 0; i < gs.nbases; ++i) {
+        const negf::GroupDev& g = v[i * gs.stride];
+        gs.sweep_base[i] = g.sweep_base;
+        gs.chain_base[i] = g.chain_base;
+        gs.seg_base[i] = g.seg_base;
+        gs.range_base[i] = g.range_base;
     }
     if (gs.ng > 2)
         gs.ext = dev;
@@ -1228,15 +1231,20 @@ int upload_and_launch(Workspace& W, const std::vector<TubePass>& passes, const s
                                       cudaMemcpyHostToDevice, stream));
     }
     // the reduce table carries device pointers that can change (rho0 of a rebuilt tube)
-    for (size_t i = 0; i < passes.size(); ++i)
-        ct.rts[i].rho0 = (!passes[i].rho0_pass && passes[i].t->shard_rank == 0) ? passes[i].t->d_rho0 : nullptr;
+    bool new_rts = rebuild, new_groups = rebuild;  // since the last upload
+    for (size_t i = 0; i < passes.size(); ++i) {
+        const double* rho0 = (!passes[i].rho0_pass && passes[i].t->shard_rank == 0) ? passes[i].t->d_rho0 : nullptr;
+        new_rts |= ct.rts[i].rho0 != rho0;
+        ct.rts[i].rho0 = rho0;
+    }
     negf::ReduceSet rs{};
     if (passes.size() == 1) {
         rs.one = ct.rts[0];
     } else {
         rs.ext = W.rts.as<negf::ReduceTube>();
-        NEGF_CUDA(cudaMemcpyAsync(W.rts.p, ct.rts.data(), ct.rts.size() * sizeof(negf::ReduceTube),
-                                  cudaMemcpyHostToDevice, stream));
+        if (new_rts)
+            NEGF_CUDA(cudaMemcpyAsync(W.rts.p, ct.rts.data(), ct.rts.size() * sizeof(negf::ReduceTube),
+                                      cudaMemcpyHostToDevice, stream));
     }
     const int nw = (int)ct.warps.size(), nw_all = nw + ct.fp64.warps;
     if (nw > 0) {
@@ -1248,11 +1256,14 @@ int upload_and_launch(Workspace& W, const std::vector<TubePass>& passes, const s
     for (int k = 0; k < 2; ++k)
         for (size_t i = 0; i < ct.fp64.groups[k].size(); ++i) {
             const negf::TubeDev& d = tdev[ct.fp64.pass_of[k][i]];
-            ct.fp64.groups[k][i].U = d.U;
-            ct.fp64.groups[k][i].Uc0 = d.Uc0;
-            ct.fp64.groups[k][i].Uc1 = d.Uc1;
+            negf::GroupDev& g = ct.fp64.groups[k][i];
+            new_groups |= g.U != d.U || g.Uc0 != d.Uc0 || g.Uc1 != d.Uc1;
+            g.U = d.U;
+            g.Uc0 = d.Uc0;
+            g.Uc1 = d.Uc1;
         }
-    if (int rc = upload_groups(ct.fp64, W.groups, stream)) return rc;
+    if (new_groups)
+        if (int rc = upload_groups(ct.fp64, W.groups, stream)) return rc;
     if (G.timing) {
         for (auto& e : W.ev)
             if (!e) NEGF_CUDA(cudaEventCreate(&e));
@@ -1390,7 +1401,7 @@ int transport_run(negf_tube& t, const std::vector<Pt>& pts, std::vector<double>&
     NEGF_CUDA(cudaMemcpyAsync(W.trTable.p, host.data(), host.size(), cudaMemcpyHostToDevice, s));
     const int K = N < negf::kSweepSeg ? 2 : negf::kSweepSeg;
     negf::GroupSet gs{};
-    gs.ng = 1;
+    gs.ng = gs.stride = gs.nbases = 1;
     negf::GroupDev& g = gs.g[0];
     g = make_group(make_tubedev(t, false), W.trTable.as<negf::EnergyRec>(),
                    reinterpret_cast<const int*>(W.trTable.as<char>() + ib), negf::kRealAxis, P * M, K);
@@ -1818,21 +1829,21 @@ int negf_compute_charge(negf_tube* const* tubes, int num_tubes, double* Q, int q
     std::vector<negf::TubeDev> tdev;
     long long off = 0;
     Settings& G = settings();
-    std::vector<std::shared_ptr<const ChainSet>> sets;
     for (int i = 0; i < num_tubes; ++i) update_paths(*tubes[i]);
-    const bool split = use_groups(tubes, num_tubes, false);
     bool same = W.table_valid && W.key_serials.size() == (size_t)num_tubes && W.key_pieces == G.pass1_pieces &&
                 W.key_schedule == G.schedule;
     for (int i = 0; i < num_tubes; ++i) {
         negf_tube* t = tubes[i];
-        if (split) {
-            sets.emplace_back();
-            if (int rc = chain_set(*t, s, &sets.back())) return rc;
-        }
         passes.push_back({t, i, off, false});
         tdev.push_back(make_tubedev(*t, false));
         off += t->N;
         if (same && (W.key_serials[i] != t->serial || W.key_versions[i] != t->version)) same = false;
+    }
+    std::vector<std::shared_ptr<const ChainSet>> sets;  // of a new table; a kept one holds its own
+    if (!same && use_groups(tubes, num_tubes, false)) {
+        sets.resize(num_tubes);
+        for (int i = 0; i < num_tubes; ++i)
+            if (int rc = chain_set(*tubes[i], s, &sets[i])) return rc;
     }
     double* dQ = Q;
     if (!q_on_device) {

@@ -107,13 +107,14 @@ struct __align__(16) GroupDev {
     double beta[kMaxModes], degen[kMaxModes];
 };
 // Groups of a launch: up to two in the kernel's parameters (one tube: no
-// table upload), more in device memory.  The first blocks of up to
-// kMaxBases groups stand in the parameters in either case, so that a block
-// finds its group without a chain of global loads.
+// table upload), more in device memory.  The first blocks of every stride-th
+// group, at most kMaxBases of them, stand in the parameters in either case, so
+// that a block finds its group with few dependent global loads (none up to
+// kMaxBases groups).
 constexpr int kMaxBases = 64;
 struct GroupSet {
     const GroupDev* ext;
-    int ng;
+    int ng, stride, nbases;  // groups, and of how many the first blocks stand here
     int sweep_base[kMaxBases], chain_base[kMaxBases], seg_base[kMaxBases], range_base[kMaxBases];
     GroupDev g[2];
 };

@@ -66,20 +66,24 @@ __device__ __forceinline__ double rcp(double x) {
 
 __device__ __forceinline__ const GroupDev& group(const GroupSet& gs, int i) { return gs.ext ? gs.ext[i] : gs.g[i]; }
 
-// Group of block b by the groups' first blocks (ascending): bisection over
-// the parameters, or a walk of the table when there are more than fit.
+// Group of block b by the groups' first blocks (ascending): bisection over the
+// parameters, which hold every stride-th one, then over the table between two of
+// them (512 tubes of 120 sites, 1024 groups: 54 us a charge pass, 442 us with a walk
+// of the table, 56 us by the warp tables of negf_rgf.cu).
 template <int GroupDev::*Base>
 __device__ __forceinline__ int find_group(const GroupSet& gs, const int (&base)[kMaxBases], int b) {
     int i = 0;
-    if (gs.ng <= kMaxBases) {
-        for (int n = gs.ng; n > 1;) {
-            const int h = n / 2;
-            if (b >= base[i + h]) i += h;
-            n -= h;
-        }
-        return i;
+    for (int n = gs.nbases; n > 1;) {
+        const int h = n / 2;
+        if (b >= base[i + h]) i += h;
+        n -= h;
     }
-    while (i + 1 < gs.ng && b >= group(gs, i + 1).*Base) ++i;
+    i *= gs.stride;
+    for (int n = min(gs.stride, gs.ng - i); n > 1;) {
+        const int h = n / 2;
+        if (b >= gs.ext[i + h].*Base) i += h;
+        n -= h;
+    }
     return i;
 }
 
@@ -355,17 +359,22 @@ __device__ __forceinline__ void sweep_chain(const GroupDev& g, int w, int piece,
     // The record (p / q, lambda) of a boundary is formed beside the first half of the next segment's
     // steps and the running state is scaled by f, a power of two next to 1 / |q_b|, after them: issue is
     // in order, so a record formed at the boundary itself would hold up the recurrence for its whole
-    // chain.  The moduli telescope to lambda_{b+1} = lambda_b prod(rho) (f_b |q_b|)^2 / |q_{b+1}|^2.
+    // chain.  The moduli telescope to lambda_b = mu_b / |q_b|^2, mu_{b+1} = mu_b f_b^2 prod(rho).
     // (Scaled by 1 / |q_b|^2, a step would take |q_b| to G_b / |q_b|: standing waves of the period of two
-    // segments, G_b large and small by turns, then grow it without bound, to inf after some 100 of them.)
-    double f = 1.0, w2 = 1.0, yr, yi;  // w2 = (f |q_b|)^2
+    // segments, G_b large and small by turns, then grow it without bound, to inf after some 100 of them: 396 us for 33 488 chains of 4000
+    // sites, 400 us so.)
+    double f = 1.0, mu = lam, yr, yi;
     auto record = [&](const Lin& t, double rprod) {
         const double q2 = fma(t.qr, t.qr, t.qi * t.qi), q1 = rcp(q2);
         yr = fma(t.pr, t.qr, t.pi * t.qi) * q1;
         yi = fma(t.pi, t.qr, -t.pr * t.qi) * q1;
-        if (RA) lam *= rprod * w2 * q1;
         f = inv_root2(q2);
-        if (RA) w2 = q2 * f * f;
+        if (RA) {
+            mu *= rprod;
+            lam = mu * q1;
+            mu *= f;
+            mu *= f;
+        }
     };
     auto scale = [&]() {
         s.pr *= f;
