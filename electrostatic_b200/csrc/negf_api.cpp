@@ -1311,7 +1311,8 @@ int upload_and_launch(Workspace& W, const std::vector<TubePass>& passes, const s
     const int fused_kernels = (ct.n64 > 0 ? 1 : 0) + (ct.n32 > 0 ? 1 : 0);
     st.kernel_launches =
         (nw > 0 ? (fused ? fused_kernels : pieces > 1 ? 4 : 2) : 0) + (ct.max_N > 0 && !ct.rts.empty() ? 1 : 0);
-    for (int k = 0; k < 2; ++k) st.kernel_launches += ct.fp64.groups[k].empty() ? 0 : 2;
+    for (int k = 0; k < 2; ++k)
+        st.kernel_launches += ct.fp64.groups[k].empty() ? 0 : ct.fp64.shape[k].range_blocks > 0 ? 3 : 2;
     st.pieces = G.pass1_pieces > 0 || nw > 0 ? pieces : reported_pieces(ct.fp64);
     st.units = (fused ? 0 : (int)ct.units.size()) + ct.fp64.shape[0].seg_blocks + ct.fp64.shape[1].seg_blocks;
     st.checkpoint_bytes = (nw > 0 ? checkpoint_traffic(ct.warps, tdev, ct.scratch_doubles, schedule) : 0) +
