@@ -907,10 +907,14 @@ long long group_state_doubles(const negf::GroupDev& g) {
 }
 
 // How the boundary states of a launch are formed: whole sweeps, sweeps in pieces
-// of `sites` (a multiple of 128, 0: whole), or the scan over segments.
+// of `sites` (a multiple of 128, 0: whole) or in `pieces` pieces of each tube
+// (multiples of 128 sites too), or the scan over segments.
 struct StatesPlan {
     bool scan = false;
-    int sites = 0;
+    int sites = 0, pieces = 0;
+    int piece_sites(int N) const {
+        return pieces > 0 ? (N + 128 * pieces - 1) / (128 * pieces) * 128 : sites;
+    }
 };
 // By the estimated time in us (measured on (17,0) tubes; site_chains = sum of
 // chains x sites):
@@ -922,6 +926,9 @@ struct StatesPlan {
 // Measured, whole / pieces / scan: 64000 sites and 230 chains 1120 / 60 / 153 us,
 // 16000 sites and 1300 chains 279 / 73 / 138, 4000 sites and 35 chains 69 / 17 / 8,
 // 604 sites and 1200 chains 14 / 14 / 11, 1600 sites and 9000 chains 33 / 50 / 93.
+// setting: 0 by these estimates, 1 whole sweeps, P > 1 pieces; pieces of fewer than
+// 128 sites do not exist, so a P beyond that runs pieces of 128 sites or, where the
+// estimates prefer it, the scan.
 StatesPlan plan_states(const negf::GroupDev* g, int n, int setting) {
     StatesPlan p;
     double site_chains = 0.0;
@@ -930,13 +937,20 @@ StatesPlan plan_states(const negf::GroupDev* g, int n, int setting) {
         site_chains += double(g[i].nch) * g[i].N;
         max_N = std::max(max_N, g[i].N);
     }
-    p.scan = setting > 1;
-    if (setting != 0) return p;
+    const double t_scan = 4.0 + 10e-6 * site_chains;
+    // pieces of L sites
+    auto t_pieces = [&](int L) { return 10.0 + std::max(0.030 * L + 0.2 * max_N / L, 2.2e-6 * site_chains); };
+    if (setting == 1) return p;
+    if (setting > 1) {
+        p.pieces = setting;
+        p.scan = max_N <= 128 || ((long long)max_N < 128LL * setting && t_scan < t_pieces(128));
+        return p;
+    }
     double best = 3.5 + std::max(0.017 * max_N, 1.1e-6 * site_chains);
     const long long slots = 8LL * device_sm_count();
     for (int L = 128; L < max_N; L += 128) {
         // pieces have to gain a tenth on whole sweeps
-        const double t = 1.1 * (10.0 + std::max(0.030 * L + 0.2 * max_N / L, 2.2e-6 * site_chains));
+        const double t = 1.1 * t_pieces(L);
         if (t >= best) {
             if (0.030 * L > best) break;
             continue;
@@ -947,7 +961,7 @@ StatesPlan plan_states(const negf::GroupDev* g, int n, int setting) {
         best = t;
         p.sites = L;
     }
-    p.scan = 4.0 + 10e-6 * site_chains < best;
+    p.scan = t_scan < best;
     if (p.scan) p.sites = 0;
     return p;
 }
@@ -968,7 +982,7 @@ void place_pieces(negf::GroupDev& g, int L, negf::SweepShape& sh, long long& tm_
 }
 
 // Groups of the FP64 chains of a launch, longest tubes first.  pieces: the
-// setting (0 automatic, 1 sweeps, more: parallel in length).
+// setting (plan_states).
 void plan_groups(SweepPart& sp, const TubePass* passes, const negf::TubeDev* tdev, int num_passes, int pieces) {
     std::vector<int> order(num_passes);
     longest_first(passes, num_passes, order.data());
@@ -1006,7 +1020,7 @@ void plan_groups(SweepPart& sp, const TubePass* passes, const negf::TubeDev* tde
         int max_nseg = 1;
         for (negf::GroupDev& g : sp.groups[k]) {
             g.chains_per_unit = iters * (32 / g.lanes);
-            place_pieces(g, k ? 0 : states.sites, sh, sp.tm_doubles);
+            place_pieces(g, k || states.scan ? 0 : states.piece_sites(g.N), sh, sp.tm_doubles);
             g.chain_base = sh.chains;
             g.seg_base = sh.seg_blocks;
             sh.chains += g.nch;
@@ -1414,7 +1428,7 @@ int transport_run(negf_tube& t, const std::vector<Pt>& pts, std::vector<double>&
     sh.scan = states.scan;
     sh.chains = g.nch;
     long long tm_doubles = 0;
-    place_pieces(g, states.sites, sh, tm_doubles);
+    place_pieces(g, states.piece_sites(N), sh, tm_doubles);
     sh.scan_threads = std::min(512, (g.nseg + 31) / 32 * 32);
     if (g.nseg > sh.scan_threads) g.tm_segs = g.nseg;
     NEGF_CUDA(W.ck.reserve(sizeof(double) * group_state_doubles(g)));

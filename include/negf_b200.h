@@ -222,10 +222,11 @@ int negf_last_stats(negf_stats* s);
  *   states, then the pieces' sweeps.  Automatic for FP32 chains: when the
  *   chains fill fewer than 4 warps per SM, enough pieces for about 8 warps
  *   per SM, each of >= 32 segments (256 sites), at most 128.  FP64 chains of
- *   the two-pass schedule are parallel in length by whole 16-site segments
- *   for any P > 1 (one scan per chain), and automatically, by that scan or by
- *   sweeps in pieces of a multiple of 128 sites, when long chains would leave
- *   the sweeps waiting on their steps.  Results agree with
+ *   the two-pass schedule run in pieces of a multiple of 128 sites (so P is an
+ *   upper bound for them), or, where a tube has fewer than 128 sites or P asks
+ *   for shorter pieces and the chains are few, as one scan over the 16-site
+ *   segments of each chain; automatically one of the two when long chains
+ *   would leave the sweeps waiting on their steps.  Results agree with
  *   P = 1 to rounding (relative 1e-10 in the tests, about 1e-12 measured).
  * NEGF_TUNE_SCHEDULE: 0 (default, automatic), NEGF_SCHEDULE_TWO_PASS or
  *   NEGF_SCHEDULE_FUSED.  Two-pass: pass 1 runs both sweeps of every chain
