@@ -170,6 +170,7 @@ struct ChainTable {
     std::vector<negf::SegUnit> units;
     std::vector<int> order;  // fused schedule: FP64 warps, then FP32 warps
     int n64 = 0, n32 = 0;
+    bool fused = false;  // the warps run fused by the estimates (Form::kFused)
     long long partial_doubles = 0, scratch_doubles = 0;
     long long updates = 0, updates_fp32 = 0, contour_updates = 0, realaxis_updates = 0;
     int max_N = 0;
@@ -841,27 +842,103 @@ int make_chain_set(const negf_tube& t, bool rho0_pass, bool fp64_all, cudaStream
     return upload_chain_set(items, codes, stream, set);
 }
 
-// Whether the FP64 chains of a batch run as groups (negf_sweep.cu) beside the
-// FP32 ones.  Not on an explicit fused request, and not when most of the work
-// is FP32: the few FP64 chains left (near the axis or a band edge) then ride
+// Chains of a batch of one precision, for the estimates of its forms.
+struct FormLoad {
+    double C = 0, SC = 0, SP = 0;  // chains, chains x sites, the same with the idle lanes of seg_kernel
+    double W = 0;                  // warps of 32 chains
+    int max_N = 0;
+    bool shorter = false, longer = false;  // tubes of fewer sites than a segment, and of more
+    void add(int N, double chains) {
+        if (chains <= 0) return;
+        const int K = N < negf::kSweepSeg ? 2 : negf::kSweepSeg, nseg = (N + K - 1) / K;
+        int lanes = 1;
+        while (lanes < 32 && lanes < nseg) lanes *= 2;
+        C += chains;
+        SC += chains * N;
+        SP += chains * ((nseg + lanes - 1) / lanes * lanes * K);
+        W += 1 + std::floor(chains / negf::kWarp);
+        max_N = std::max(max_N, N);
+        (K == 2 ? shorter : longer) = true;
+    }
+};
+// Estimated time in us of a charge pass by groups and by the fused schedule,
+// fitted to 255 FP64 batches of (17,0) tubes, of 8 to 1536 sites and 256 to 300 000
+// chains: the form they choose is the slower one in 12 of them, by 3 to 10 % but once
+// (33 %).
+// Groups take three launches or more, whose blocks start one after the other, and
+// tubes of fewer sites than a segment launches of their own; fused, a warp crosses
+// its tube alone, 8 warps per SM make a wave.  Measured, groups / fused: 16 tubes
+// of 8 sites and 65536 chains 231 / 95, 16 sites and 33000 chains 22.6 / 16.6, 64
+// sites and 33000 chains 29 / 23, 256 sites and 33000 chains 47 / 41, and 1024
+// chains 21 / 27, 512 sites and 50000 chains 97 / 99, 1024 sites and 16000 chains
+// 72 / 82, 4000 sites and 33000 chains 400 / 470, 8 tubes of 8 to 68 sites 44 / 25.
+double groups_us(const FormLoad& l) {
+    const double scan = 18.5 + 12e-6 * l.SC;
+    const double sweeps = 18.5 + 0.022 * l.max_N + 0.1e-3 * l.C + 0.8e-6 * l.SC + 1.33e-6 * l.SP;
+    return std::min(scan, sweeps) + (l.shorter && l.longer ? 12.0 : 0.0);
+}
+double fused_us(const FormLoad& l) {
+    if (l.C <= 0) return 0.0;
+    const double alone = 12.5 + 0.061 * l.max_N;  // the longest chain, one warp per scheduler
+    const double waves = l.W / (8 * device_sm_count()), part = waves - std::floor(waves);
+    if (waves <= 0.5) return alone + 0.5e-6 * l.SC;
+    const double mean = l.SC / l.C, tail = part > 0 ? 0.5 + 0.5 * part : 0.0;
+    return std::max(waves > 1.0 ? 15.0 + 0.095 * l.max_N : alone + 2.5 + 0.044 * mean,
+                    11.0 + (std::floor(waves) + tail) * (5.0 + 0.107 * mean));
+}
+
+// Form of a batch's FP64 chains: groups (negf_sweep.cu) beside the FP32 warps;
+// the warp tables of the FP32 ones; or, of FP64 batches alone, the warp tables in
+// the fused schedule.
+enum class Form { kGroups, kWarps, kFused };
+// The warp tables on an explicit fused request, and when most of the work is
+// FP32: the few FP64 chains left (near the axis or a band edge) then ride
 // along in the launches of the FP32 warps (a 16-tube batch with the real axis
-// in FP32: 2.364 ms so, 2.382 ms with groups; a small mixed tube 44 us against
-// 47 us).  Counted by energies; the band-edge rule moves single chains only.
-bool use_groups(negf_tube* const* tubes, int num_tubes, bool fp64_all) {
-    if (settings().schedule == NEGF_SCHEDULE_FUSED) return false;
-    long long all = 0, low = 0;
+// in FP32: 2.364 ms so, 2.382 ms with groups).  Counted by energies; the band-edge
+// rule moves single chains only.  Else, unless a setting asks for other schedules,
+// the faster form by the estimates.  FP64 batches: groups or fused; up to 32 sites
+// fused is ahead at every number of chains.  With FP32 warps, whose schedule is the
+// same in both forms (two-pass below 4 warps per SM, else fused): groups beside
+// them, sharing the GPU, or all chains in the warp tables (half FP32, groups /
+// warp tables: 160 sites and 4096 chains 38 / 35 us, 1024 sites 94 / 89 and 12000
+// chains 106 / 134, 4000 sites and 4096 chains 153 / 205).
+Form choose_form(negf_tube* const* tubes, int num_tubes, bool fp64_all) {
+    const Settings& G = settings();
+    if (G.schedule == NEGF_SCHEDULE_FUSED) return Form::kWarps;
+    FormLoad f64, f32, all;
     for (int i = 0; i < num_tubes; ++i) {
         const negf_tube& t = *tubes[i];
-        const long long w = (long long)t.N * t.d.num_modes;
-        all += w * (long long)(t.eq_pts.size() + t.poles.size() + t.noneq_pts.size());
-        if (t.d.precision != NEGF_PREC_MIXED || fp64_all) continue;
-        const double band = t.d.mixed_fp64_band;
-        for (const Pt& p : t.eq_pts) low += std::fabs(p.E.imag()) >= band ? w : 0;
-        for (const cplx& p : t.poles) low += std::fabs(p.imag()) >= band ? w : 0;
-        if (t.d.mixed_realaxis_fp32)
-            for (const Pt& p : t.noneq_pts) low += std::fabs(p.E.imag()) >= band ? w : 0;
+        const size_t total = t.eq_pts.size() + t.poles.size() + t.noneq_pts.size();
+        size_t low = 0;
+        if (t.d.precision == NEGF_PREC_MIXED && !fp64_all) {
+            const double band = t.d.mixed_fp64_band;
+            for (const Pt& p : t.eq_pts) low += std::fabs(p.E.imag()) >= band;
+            for (const cplx& p : t.poles) low += std::fabs(p.imag()) >= band;
+            if (t.d.mixed_realaxis_fp32)
+                for (const Pt& p : t.noneq_pts) low += std::fabs(p.E.imag()) >= band;
+        }
+        const double per = double(t.d.num_modes) / t.shard_world;
+        f64.add(t.N, per * double(total - low));
+        f32.add(t.N, per * double(low));
+        all.add(t.N, per * double(total));
     }
-    return 2 * low <= all;
+    if (2 * f32.SC > all.SC) return Form::kWarps;
+    if (G.schedule != 0 || G.pass1_pieces != 0) return Form::kGroups;
+    const double groups = groups_us(f64);
+    if (f32.C <= 0) return all.max_N <= 32 || fused_us(all) < groups ? Form::kFused : Form::kGroups;
+    double low, warps, share;  // FP32 warps alone, all chains in the tables
+    if (all.W < 4 * device_sm_count()) {
+        auto latency = [](int N) { return 14.0 + 0.15 * std::min(N, 500); };  // pieces beyond
+        low = latency(f32.max_N);
+        warps = latency(all.max_N);
+        if (all.max_N >= 512) warps = std::max(warps, 60.0 + 7.2e-6 * all.SC);
+        share = 0.25;
+    } else {
+        low = fused_us(f32);
+        warps = fused_us(all);
+        share = 0.5;
+    }
+    return std::max(groups, low) + share * std::min(groups, low) < warps ? Form::kGroups : Form::kWarps;
 }
 
 // The tube's FP64 chains for the current paths, made on first use of a version.
@@ -1214,13 +1291,15 @@ cudaError_t launch_split(bool any64, bool any32, cudaStream_t stream, cudaStream
     return e;
 }
 
+// fused: a new table (rebuild) of warps alone runs fused unless a setting says otherwise.
 int upload_and_launch(Workspace& W, const std::vector<TubePass>& passes, const std::vector<negf::TubeDev>& tdev,
-                      const std::vector<std::shared_ptr<const ChainSet>>& sets, bool rebuild, double* d_Q,
-                      cudaStream_t stream) {
+                      const std::vector<std::shared_ptr<const ChainSet>>& sets, bool fused_form, bool rebuild,
+                      double* d_Q, cudaStream_t stream) {
     Settings& G = settings();
     ChainTable& ct = W.table;
     if (rebuild) {
         build_table(ct, passes, tdev, sets, G.pass1_pieces);
+        ct.fused = fused_form;
         NEGF_CUDA(W.chains.reserve(std::max<size_t>(1, ct.chains.size()) * sizeof(negf::ChainRec)));
         NEGF_CUDA(W.warps.reserve(std::max<size_t>(1, ct.warps.size()) * sizeof(negf::WarpRec)));
         NEGF_CUDA(W.rts.reserve(std::max<size_t>(1, ct.rts.size()) * sizeof(negf::ReduceTube)));
@@ -1284,11 +1363,12 @@ int upload_and_launch(Workspace& W, const std::vector<TubePass>& passes, const s
         NEGF_CUDA(cudaEventRecord(W.ev[0], stream));
     }
     int pieces = G.pass1_pieces;
-    if (pieces == 0 && G.schedule == NEGF_SCHEDULE_FUSED) pieces = 1;  // an explicit fused request wins
+    const int setting = ct.fused ? NEGF_SCHEDULE_FUSED : G.schedule;
+    if (pieces == 0 && setting == NEGF_SCHEDULE_FUSED) pieces = 1;  // an explicit fused request wins
     if (pieces == 0) pieces = auto_pieces(nw_all, ct.max_N);
     pieces = std::max(1, pieces);
     // schedule of the warp tables (the FP32 chains, or every chain of an explicit fused request)
-    const int schedule = nw > 0 ? choose_schedule(G.schedule, nw_all, pieces) : negf::kScheduleTwoPass;
+    const int schedule = nw > 0 ? choose_schedule(setting, nw_all, pieces) : negf::kScheduleTwoPass;
     if (schedule == negf::kScheduleFused) pieces = 1;
     if (nw > 0 && pieces > 1) NEGF_CUDA(W.pieces.reserve(sizeof(double) * (size_t)nw * pieces * 24 * negf::kWarp));
     const bool any64 = ct.fp64.any();
@@ -1371,7 +1451,7 @@ int compute_rho0(negf_tube* t) {
     std::vector<std::shared_ptr<const ChainSet>> sets(1);
     if (int rc = make_chain_set(*t, true, true, nullptr, &sets[0])) return rc;
     W->table_valid = false;
-    int rc = upload_and_launch(*W, passes, tdev, sets, true, t->d_rho0, nullptr);
+    int rc = upload_and_launch(*W, passes, tdev, sets, false, true, t->d_rho0, nullptr);
     W->table_valid = false;
     if (rc != NEGF_OK) return rc;
     NEGF_CUDA(cudaStreamSynchronize(nullptr));
@@ -1855,7 +1935,8 @@ int negf_compute_charge(negf_tube* const* tubes, int num_tubes, double* Q, int q
         if (same && (W.key_serials[i] != t->serial || W.key_versions[i] != t->version)) same = false;
     }
     std::vector<std::shared_ptr<const ChainSet>> sets;  // of a new table; a kept one holds its own
-    if (!same && use_groups(tubes, num_tubes, false)) {
+    const Form form = same ? Form::kGroups : choose_form(tubes, num_tubes, false);
+    if (!same && form == Form::kGroups) {
         sets.resize(num_tubes);
         for (int i = 0; i < num_tubes; ++i)
             if (int rc = chain_set(*tubes[i], s, &sets[i])) return rc;
@@ -1865,7 +1946,7 @@ int negf_compute_charge(negf_tube* const* tubes, int num_tubes, double* Q, int q
         NEGF_CUDA(W.qbuf.reserve(sizeof(double) * off));
         dQ = W.qbuf.as<double>();
     }
-    int rc = upload_and_launch(W, passes, tdev, sets, !same, dQ, s);
+    int rc = upload_and_launch(W, passes, tdev, sets, form == Form::kFused, !same, dQ, s);
     if (rc) {
         W.table_valid = false;
         return rc;
@@ -1889,8 +1970,8 @@ int negf_compute_charge(negf_tube* const* tubes, int num_tubes, double* Q, int q
 
 // ------------------------------------------------------------------ charge plans
 namespace {
-// Tables of a plan for a given number of segments per pass-2 unit.
-int plan_tables(negf_charge_plan& p, int spu, bool upload_all) {
+// Tables of a plan for a form and a number of segments per pass-2 unit.
+int plan_tables(negf_charge_plan& p, Form form, int spu, bool upload_all) {
     const int n = (int)p.tubes.size();
     // an FP64 plan of mixed-precision tubes: their descriptors read as FP64 while the table is built
     std::vector<int> saved(n);
@@ -1911,7 +1992,7 @@ int plan_tables(negf_charge_plan& p, int spu, bool upload_all) {
     ChainTable ct;
     std::vector<std::shared_ptr<const ChainSet>> sets;
     int rc = NEGF_OK;
-    if (use_groups(p.tubes.data(), n, p.force_fp64)) {
+    if (form == Form::kGroups) {
         if (!p.fp64.sets.empty()) {
             sets = p.fp64.sets;
         } else {
@@ -2012,17 +2093,19 @@ int negf_charge_plan_create(negf_tube* const* tubes, int num_tubes, double* d_Q,
     cudaStream_t side0 = nullptr;  // the autotuner's launches run on the legacy default stream
     if (int rc3 = plan_side_stream(0, &side0)) return rc3;
     p->wpb = settings().warps_per_block;
-    rc = plan_tables(*p, negf::kSegsPerUnit, true);
+    Form form = choose_form(tubes, num_tubes, p->force_fp64);  // of the plan's tables
+    rc = plan_tables(*p, form, negf::kSegsPerUnit, true);
     if (rc) return rc;
     {
         // pass-1 pieces as negf_compute_charge chooses them (the setting, else the automatic rule)
+        const int setting = form == Form::kFused ? NEGF_SCHEDULE_FUSED : settings().schedule;
         int pc = settings().pass1_pieces;
-        if (pc == 0 && settings().schedule == NEGF_SCHEDULE_FUSED) pc = 1;
+        if (pc == 0 && setting == NEGF_SCHEDULE_FUSED) pc = 1;
         if (pc == 0) pc = auto_pieces(p->num_warps + p->fp64.warps, p->max_N);
         p->pieces = std::max(1, pc);
+        p->schedule = p->num_warps > 0 ? choose_schedule(setting, p->num_warps + p->fp64.warps, p->pieces)
+                                       : negf::kScheduleTwoPass;
     }
-    p->schedule = p->num_warps > 0 ? choose_schedule(settings().schedule, p->num_warps + p->fp64.warps, p->pieces)
-                                   : negf::kScheduleTwoPass;
     if (p->schedule == negf::kScheduleFused) p->pieces = 1;
     if (p->num_warps == 0 && settings().pass1_pieces == 0) p->pieces = reported_pieces(p->fp64);
     // piece candidates of the autotuner: only when the chains cannot fill the GPU
@@ -2041,62 +2124,90 @@ int negf_charge_plan_create(negf_tube* const* tubes, int num_tubes, double* d_Q,
                                           negf::kWarp));
     }
     if (flags & NEGF_PLAN_AUTOTUNE) {
-        // time the fused schedule (wpb 0 below) and every two-pass shape
-        // (segments per pass-2 unit x pass-2 warps per block x pass-1 pieces) on this batch
+        // Time the forms on this batch: groups, whose shape follows the rules of
+        // plan_groups, and the fused schedule of all chains (unless a setting
+        // asks for one form); with FP32 warps in the tables their schedules, the
+        // fused one (wpb 0 below) and every two-pass shape (segments per pass-2
+        // unit x pass-2 warps per block x pass-1 pieces).
+        struct Shape {
+            Form form;
+            int spu, wpb, schedule, pieces;
+        };
         cudaEvent_t e0, e1;
         NEGF_CUDA(cudaEventCreate(&e0));
         NEGF_CUDA(cudaEventCreate(&e1));
         double best = 1e300;
-        int best_spu = negf::kSegsPerUnit, best_wpb = p->wpb, best_pc = 1;
-        // no warp tables: the FP64 groups have nothing to choose (their shape
-        // follows the rules of plan_groups), one shape is timed
-        const bool choose = p->num_warps > 0;
-        if (!choose) best_pc = p->pieces;
-        for (int spu : {16, 32, 64}) {
-            if (!choose && spu != negf::kSegsPerUnit) continue;
-            rc = plan_tables(*p, spu, false);
-            if (rc) break;
-            for (int wpb : {0, 1, 2, 4}) {
-                if (!choose && wpb != p->wpb) continue;
-                if (wpb == 0 && spu != 16) continue;  // the fused schedule has no segment units
-                for (int pc : piece_cands) {
-                    if (wpb == 0 && pc != 1) continue;  // the fused schedule runs whole chains
-                    if (choose) {
-                        p->wpb = wpb == 0 ? 4 : wpb;
-                        p->schedule = wpb == 0 ? negf::kScheduleFused : negf::kScheduleTwoPass;
-                        p->pieces = pc;
-                    }
-                    cudaError_t e = plan_launch(*p, nullptr, 0, side0);
-                    for (int r = 0; r < 3 && e == cudaSuccess; ++r) {
-                        if (r == 1) e = cudaEventRecord(e0, 0);
-                        if (e == cudaSuccess) e = plan_launch(*p, nullptr, 0, side0);
-                    }
-                    if (e == cudaSuccess) e = cudaEventRecord(e1, 0);
-                    if (e == cudaSuccess) e = cudaEventSynchronize(e1);
-                    float ms = 0.f;
-                    if (e == cudaSuccess) e = cudaEventElapsedTime(&ms, e0, e1);
-                    if (e != cudaSuccess) {
-                        cudaEventDestroy(e0);
-                        cudaEventDestroy(e1);
-                        return fail(NEGF_ERR_CUDA, cudaGetErrorString(e));
-                    }
-                    if (ms / 2 < best) {
-                        best = ms / 2;
-                        best_spu = spu;
-                        best_wpb = wpb;
-                        best_pc = choose ? pc : p->pieces;
+        Shape best_shape{form, negf::kSegsPerUnit, p->wpb, p->schedule, p->pieces};
+        const int wpb0 = p->wpb;
+        auto run = [&](const Shape& s) -> cudaError_t {
+            p->wpb = s.wpb;
+            p->schedule = s.schedule;
+            p->pieces = s.pieces;
+            cudaError_t e = plan_launch(*p, nullptr, 0, side0);
+            for (int r = 0; r < 3 && e == cudaSuccess; ++r) {
+                if (r == 1) e = cudaEventRecord(e0, 0);
+                if (e == cudaSuccess) e = plan_launch(*p, nullptr, 0, side0);
+            }
+            if (e == cudaSuccess) e = cudaEventRecord(e1, 0);
+            if (e == cudaSuccess) e = cudaEventSynchronize(e1);
+            float ms = 0.f;
+            if (e == cudaSuccess) e = cudaEventElapsedTime(&ms, e0, e1);
+            if (e == cudaSuccess && ms / 2 < best) {
+                best = ms / 2;
+                best_shape = s;
+            }
+            return e;
+        };
+        std::vector<Form> forms{form};
+        if (form != Form::kWarps && settings().schedule == 0 && settings().pass1_pieces == 0)
+            forms.push_back(form == Form::kGroups ? Form::kFused : Form::kGroups);
+        cudaError_t e = cudaSuccess;
+        bool current = true;  // the plan's tables are whole ones of `form`
+        for (Form f : forms) {
+            for (int spu : {16, 32, 64}) {
+                const bool one_shape = f == Form::kFused || (f == form && p->num_warps == 0);
+                if (one_shape && spu != negf::kSegsPerUnit) continue;
+                rc = plan_tables(*p, f, spu, f != form);
+                if (rc && f != forms[0]) {  // no room for the second form: the first one stays
+                    cudaGetLastError();
+                    rc = NEGF_OK;
+                    current = false;
+                    break;
+                }
+                if (rc) break;
+                form = f;
+                if (f == Form::kFused || p->num_warps == 0) {
+                    if (spu == negf::kSegsPerUnit)
+                        e = run(f == Form::kFused
+                                    ? Shape{f, spu, wpb0, negf::kScheduleFused, 1}
+                                    : Shape{f, spu, wpb0, negf::kScheduleTwoPass,
+                                            settings().pass1_pieces > 0 ? settings().pass1_pieces
+                                                                        : reported_pieces(p->fp64)});
+                    if (e != cudaSuccess) break;
+                    continue;
+                }
+                for (int wpb : {0, 1, 2, 4}) {
+                    if (wpb == 0 && spu != 16) continue;  // the fused schedule has no segment units
+                    for (int pc : piece_cands) {
+                        if (wpb == 0 && pc != 1) continue;  // the fused schedule runs whole chains
+                        if (e == cudaSuccess)
+                            e = run({f, spu, wpb == 0 ? 4 : wpb,
+                                     wpb == 0 ? negf::kScheduleFused : negf::kScheduleTwoPass, pc});
                     }
                 }
+                if (e != cudaSuccess) break;
             }
+            if (rc || e != cudaSuccess) break;
         }
         cudaEventDestroy(e0);
         cudaEventDestroy(e1);
         if (rc) return rc;
-        p->schedule = best_wpb == 0 ? negf::kScheduleFused : negf::kScheduleTwoPass;
-        p->wpb = best_wpb == 0 ? 4 : best_wpb;
-        p->pieces = best_pc;
+        if (e != cudaSuccess) return fail(NEGF_ERR_CUDA, cudaGetErrorString(e));
+        p->schedule = best_shape.schedule;
+        p->wpb = best_shape.wpb;
+        p->pieces = best_shape.pieces;
         p->tuned_ms = best;
-        rc = plan_tables(*p, best_spu, false);
+        rc = plan_tables(*p, best_shape.form, best_shape.spu, best_shape.form != form || !current);
         if (rc) return rc;
     }
     *out = p.release();

@@ -236,11 +236,12 @@ int negf_last_stats(negf_stats* s);
  *   backward sweep the second, each storing its own checkpoints, then each
  *   continues into the other half and integrates the segments it crosses
  *   (every site crossed twice instead of three times, half the checkpoint
- *   bytes; needs enough chains to fill the GPU).  Automatic: two-pass for
- *   batches whose work is mostly FP64; for mostly FP32 batches (and the FP32
- *   chains of the others) fused when the chains fill at least one warp per
- *   SM sub-partition and the sweeps run as one piece.  Results agree to
- *   rounding. */
+ *   bytes; needs enough chains to fill the GPU).  Automatic: for batches
+ *   whose work is mostly FP64, the faster form by estimated time (fused for
+ *   short tubes, up to about 500 sites where the chains fill the GPU once);
+ *   for mostly FP32 batches (and the FP32 chains of two-pass ones) fused when
+ *   the chains fill at least one warp per SM sub-partition and the sweeps run
+ *   as one piece.  Results agree to rounding. */
 #define NEGF_TUNE_PASS2_WARPS_PER_BLOCK 2
 #define NEGF_TUNE_PASS1_PIECES 4
 #define NEGF_TUNE_SCHEDULE 6
@@ -392,12 +393,14 @@ int negf_write_integrand(negf_tube* t, const char* path, int count, const double
  * contact potentials are read on the device as U[0] and U[N-1] of each
  * tube's potential buffer (U_contact = U at the end sites,
  * Nanostructure.cpp:500-504).  d_Q: device output of sum N doubles (tube
- * order).  With NEGF_PLAN_AUTOTUNE the fused (warp per chain) schedule and
- * every two-pass (segment tile) schedule -- segments per unit 16/32/64 x
- * pass-2 warps per block 1/2/4, and, when the chains fill fewer than 4 warps
- * per SM, pass-1 pieces 1/2/4/8/automatic (parallel in length) -- are timed
- * on the batch and the fastest is kept (results agree to rounding; bitwise
- * within the two-pass shapes of one piece count).  Without it the schedule
+ * order).  With NEGF_PLAN_AUTOTUNE the fused (warp per chain) schedule, the
+ * two-pass form of the FP64 chains (its shape follows from the batch) and, for
+ * FP32 chains and mostly FP32 batches, every two-pass (segment tile) schedule
+ * -- segments per unit 16/32/64 x pass-2 warps per block 1/2/4, and, when the
+ * chains fill fewer than 4 warps per SM, pass-1 pieces 1/2/4/8/automatic
+ * (parallel in length) -- are timed on the batch and the fastest is kept
+ * (results agree to rounding; bitwise within the two-pass shapes of one piece
+ * count).  Without it the schedule
  * and the pieces follow NEGF_TUNE_SCHEDULE's and NEGF_TUNE_PASS1_PIECES's
  * rules, as in negf_compute_charge.
  * negf_charge_plan_info's *pass2_warps_per_block is 0 when the fused

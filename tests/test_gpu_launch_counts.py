@@ -15,7 +15,15 @@ def _call(cells, **kw):
     return last_stats()
 
 
-def test_kernel_launches_of_each_form():
+@pytest.fixture
+def two_pass():
+    from electrostatic_b200.negf import SCHEDULE_AUTO, SCHEDULE_TWO_PASS, TUNE_SCHEDULE, set_tuning
+    set_tuning(TUNE_SCHEDULE, SCHEDULE_TWO_PASS)
+    yield
+    set_tuning(TUNE_SCHEDULE, SCHEDULE_AUTO)
+
+
+def test_kernel_launches_of_each_form(two_pass):
     assert _call(3)["kernel_launches"] == 3      # 12 sites, 2-site segments: states, segments, reduction
     assert _call(100)["kernel_launches"] == 3    # the scan over segments, segments, reduction
     st = _call(4000, type_id=(16, 0), num_modes=8)

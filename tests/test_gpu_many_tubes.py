@@ -18,8 +18,17 @@ def _tubes(n, cells):
     return out
 
 
+@pytest.fixture
+def two_pass():
+    """The form by groups for every length."""
+    from electrostatic_b200.negf import SCHEDULE_AUTO, SCHEDULE_TWO_PASS, TUNE_SCHEDULE, set_tuning
+    set_tuning(TUNE_SCHEDULE, SCHEDULE_TWO_PASS)
+    yield
+    set_tuning(TUNE_SCHEDULE, SCHEDULE_AUTO)
+
+
 @pytest.mark.parametrize("n", [33, 65, 100, 200])
-def test_batch_equals_single_tubes(n):
+def test_batch_equals_single_tubes(two_pass, n):
     """Each tube's charge in the batch is its charge alone (the sums over the
     chains run in another order: rounding), on both sides of one segment."""
     from electrostatic_b200.negf import compute_charge
@@ -38,7 +47,7 @@ def test_batch_equals_single_tubes(n):
     assert np.abs(Q[-len(q):] - q).max() <= 1e-12 * np.abs(q).max()
 
 
-def test_time_of_many_tubes():
+def test_time_of_many_tubes(two_pass):
     """32 times the tubes of a launch that leaves the GPU nearly empty: far from
     32 times the time (a block that walks the table of groups took 24 times)."""
     import torch
