@@ -139,15 +139,64 @@ struct DevBuf {
     }
 };
 
+// Allocations, frees and copies on streams of our own while another thread may be
+// capturing a graph: they are not part of it and do not end it.
+struct RelaxedCapture {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+
+// Device memory of chain lists that no one holds any more.  cudaFree waits for the
+// whole device, so it is put off until more than kKeep bytes are waiting.
+class RetiredLists {
+public:
+    static RetiredLists& get() {
+        static RetiredLists* r = new RetiredLists;  // outlives every tube and workspace
+        return *r;
+    }
+    void add(void* p, size_t bytes) {
+        std::lock_guard<std::mutex> lk(mu_);
+        lists_.push_back(p);
+        bytes_ += bytes;
+        if (bytes_ > kKeep) free_all();
+    }
+    void clear() {
+        std::lock_guard<std::mutex> lk(mu_);
+        free_all();
+    }
+
+private:
+    static constexpr size_t kKeep = size_t(16) << 20;
+    void free_all() {
+        RelaxedCapture relaxed;
+        for (void* p : lists_) cudaFree(p);
+        lists_.clear();
+        bytes_ = 0;
+    }
+    std::mutex mu_;
+    std::vector<void*> lists_;
+    size_t bytes_ = 0;
+};
+
 // FP64 chains of a tube for its current energy paths, on the device: the energy
 // table and the codes (energy, mode) of the contour and pole chains, then of
 // the real-axis ones.  Made once per version of the tube's paths, shared by
-// every call and plan that uses that version and freed with the last of them.
+// every call and plan that uses that version and retired with the last of them.
 struct ChainSet {
     std::vector<negf::EnergyRec> h_items;
     std::vector<int> h_codes;
-    DevBuf items, codes;
+    void* mem = nullptr;  // the energy table, then the codes
+    const negf::EnergyRec* items() const { return static_cast<const negf::EnergyRec*>(mem); }
+    const int* codes() const { return reinterpret_cast<const int*>(items() + h_items.size()); }
+    size_t bytes() const { return h_items.size() * sizeof(negf::EnergyRec) + h_codes.size() * sizeof(int); }
     int contour = 0, realaxis = 0;  // chains of each kind
+    ChainSet() = default;
+    ChainSet(const ChainSet&) = delete;
+    ChainSet& operator=(const ChainSet&) = delete;
+    ~ChainSet() {
+        if (mem) RetiredLists::get().add(mem, bytes());
+    }
 };
 
 // FP64 part of a launch (negf_sweep.cu): groups with K = kSweepSeg and with K = 2.
@@ -782,9 +831,24 @@ void longest_first(const TubePass* passes, int num_passes, int* order) {
     }
 }
 
-// Device copy of an FP64 chain list on `stream`, finished on return (other
-// streams may use it next).  An unchanged list keeps the set it has.
-int upload_chain_set(std::vector<negf::EnergyRec>& items, std::vector<int> (&codes)[2], cudaStream_t stream,
+// Stream of the chain lists' copies, one per device.
+cudaError_t list_stream(cudaStream_t* s) {
+    static std::mutex mu;
+    static std::map<int, cudaStream_t>* streams = new std::map<int, cudaStream_t>;
+    std::lock_guard<std::mutex> lk(mu);
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    cudaStream_t& st = (*streams)[dev];
+    if (!st) e = cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking);
+    *s = st;
+    return e;
+}
+
+// Device copy of an FP64 chain list, finished on return: any stream may use it
+// next, and the host waits for this copy only, not for the work of the call's
+// stream.  An unchanged list keeps the set it has.
+int upload_chain_set(std::vector<negf::EnergyRec>& items, std::vector<int> (&codes)[2],
                      std::shared_ptr<const ChainSet>* set) {
     std::shared_ptr<ChainSet> cs = std::make_shared<ChainSet>();
     cs->contour = (int)codes[negf::kContour].size();
@@ -793,21 +857,22 @@ int upload_chain_set(std::vector<negf::EnergyRec>& items, std::vector<int> (&cod
     cs->h_codes.insert(cs->h_codes.end(), codes[negf::kRealAxis].begin(), codes[negf::kRealAxis].end());
     cs->h_items = std::move(items);
     const size_t ib = cs->h_items.size() * sizeof(negf::EnergyRec), cb = cs->h_codes.size() * sizeof(int);
+    static_assert(sizeof(negf::EnergyRec) % alignof(int) == 0, "codes behind the energies");
     if (*set && (*set)->contour == cs->contour && (*set)->h_codes == cs->h_codes &&
         (*set)->h_items.size() == cs->h_items.size() &&
         (ib == 0 || std::memcmp((*set)->h_items.data(), cs->h_items.data(), ib) == 0))
         return NEGF_OK;
     if (cb) {
-        // another thread may be capturing a graph: these allocations are not part of it
-        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
-        NEGF_CUDA(cudaThreadExchangeStreamCaptureMode(&mode));
-        cudaError_t e = cs->items.reserve(ib);
-        if (e == cudaSuccess) e = cs->codes.reserve(cb);
-        if (e == cudaSuccess) e = cudaMemcpyAsync(cs->items.p, cs->h_items.data(), ib, cudaMemcpyHostToDevice, stream);
-        if (e == cudaSuccess) e = cudaMemcpyAsync(cs->codes.p, cs->h_codes.data(), cb, cudaMemcpyHostToDevice, stream);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
-        cudaThreadExchangeStreamCaptureMode(&mode);
-        NEGF_CUDA(e);
+        std::vector<char> host(ib + cb);
+        std::memcpy(host.data(), cs->h_items.data(), ib);
+        std::memcpy(host.data() + ib, cs->h_codes.data(), cb);
+        RelaxedCapture relaxed;
+        cudaStream_t s = nullptr;
+        NEGF_CUDA(list_stream(&s));
+        NEGF_CUDA(cudaMalloc(&cs->mem, ib + cb));
+        cudaError_t e = cudaMemcpyAsync(cs->mem, host.data(), ib + cb, cudaMemcpyHostToDevice, s);
+        const cudaError_t w = cudaStreamSynchronize(s);  // also after an error: `host` goes
+        NEGF_CUDA(e != cudaSuccess ? e : w);
     }
     *set = std::move(cs);
     return NEGF_OK;
@@ -815,8 +880,7 @@ int upload_chain_set(std::vector<negf::EnergyRec>& items, std::vector<int> (&cod
 
 // FP64 chains of one pass of a tube (see ChainSet); fp64_all: every chain,
 // whatever the tube's precision mode.
-int make_chain_set(const negf_tube& t, bool rho0_pass, bool fp64_all, cudaStream_t stream,
-                   std::shared_ptr<const ChainSet>* set) {
+int make_chain_set(const negf_tube& t, bool rho0_pass, bool fp64_all, std::shared_ptr<const ChainSet>* set) {
     const int M = t.d.num_modes, total = pass_items(t, rho0_pass);
     int lo = 0, hi = total;
     if (!rho0_pass) negf_shard_range(total, t.shard_rank, t.shard_world, &lo, &hi);
@@ -839,7 +903,7 @@ int make_chain_set(const negf_tube& t, bool rho0_pass, bool fp64_all, cudaStream
         if (used) items.push_back({it.E.real(), it.E.imag(), it.c.real(), it.c.imag(), it.b0, it.b1});
     }
     if (items.size() >= (size_t(1) << (31 - negf::kModeBits))) return fail(NEGF_ERR_ARG, "too many energy points");
-    return upload_chain_set(items, codes, stream, set);
+    return upload_chain_set(items, codes, set);
 }
 
 // Chains of a batch of one precision, for the estimates of its forms.
@@ -942,9 +1006,9 @@ Form choose_form(negf_tube* const* tubes, int num_tubes, bool fp64_all) {
 }
 
 // The tube's FP64 chains for the current paths, made on first use of a version.
-int chain_set(negf_tube& t, cudaStream_t stream, std::shared_ptr<const ChainSet>* out) {
+int chain_set(negf_tube& t, std::shared_ptr<const ChainSet>* out) {
     if (!t.set || t.set_version != t.version) {
-        if (int rc = make_chain_set(t, false, false, stream, &t.set)) return rc;
+        if (int rc = make_chain_set(t, false, false, &t.set)) return rc;
         t.set_version = t.version;
     }
     *out = t.set;
@@ -1070,8 +1134,8 @@ void plan_groups(SweepPart& sp, const TubePass* passes, const negf::TubeDev* tde
         for (int kind : {negf::kRealAxis, negf::kContour}) {
             const int nch = kind == negf::kRealAxis ? cs.realaxis : cs.contour;
             if (nch == 0) continue;
-            sp.groups[k].push_back(make_group(tdev[o], cs.items.as<negf::EnergyRec>(),
-                                              cs.codes.as<int>() + (kind == negf::kRealAxis ? cs.contour : 0), kind,
+            sp.groups[k].push_back(make_group(tdev[o], cs.items(),
+                                              cs.codes() + (kind == negf::kRealAxis ? cs.contour : 0), kind,
                                               nch, k ? 2 : negf::kSweepSeg));
             sp.pass_of[k].push_back(o);
             const negf::GroupDev& g = sp.groups[k].back();
@@ -1449,7 +1513,7 @@ int compute_rho0(negf_tube* t) {
     std::vector<TubePass> passes{{t, 0, 0, true}};
     std::vector<negf::TubeDev> tdev{make_tubedev(*t, true)};
     std::vector<std::shared_ptr<const ChainSet>> sets(1);
-    if (int rc = make_chain_set(*t, true, true, nullptr, &sets[0])) return rc;
+    if (int rc = make_chain_set(*t, true, true, &sets[0])) return rc;
     W->table_valid = false;
     int rc = upload_and_launch(*W, passes, tdev, sets, false, true, t->d_rho0, nullptr);
     W->table_valid = false;
@@ -1939,7 +2003,7 @@ int negf_compute_charge(negf_tube* const* tubes, int num_tubes, double* Q, int q
     if (!same && form == Form::kGroups) {
         sets.resize(num_tubes);
         for (int i = 0; i < num_tubes; ++i)
-            if (int rc = chain_set(*tubes[i], s, &sets[i])) return rc;
+            if (int rc = chain_set(*tubes[i], &sets[i])) return rc;
     }
     double* dQ = Q;
     if (!q_on_device) {
@@ -1998,8 +2062,8 @@ int plan_tables(negf_charge_plan& p, Form form, int spu, bool upload_all) {
         } else {
             for (int i = 0; i < n && rc == NEGF_OK; ++i) {
                 sets.emplace_back();
-                rc = p.force_fp64 ? make_chain_set(*p.tubes[i], false, true, nullptr, &sets.back())
-                                  : chain_set(*p.tubes[i], nullptr, &sets.back());
+                rc = p.force_fp64 ? make_chain_set(*p.tubes[i], false, true, &sets.back())
+                                  : chain_set(*p.tubes[i], &sets.back());
             }
         }
     }
@@ -2310,6 +2374,7 @@ int negf_release_scratch(void* stream) {
     std::lock_guard<std::mutex> lk(g_mu);
     int dev = 0;
     NEGF_CUDA(cudaGetDevice(&dev));
+    RetiredLists::get().clear();
     auto& all = workspaces();
     auto it = all.find(WsKey{dev, (cudaStream_t)stream});
     if (it == all.end()) return NEGF_OK;
@@ -2730,7 +2795,7 @@ int ring_modes_charge(negf_tube& t, Workspace& W, bool rho0_pass, double* d_out,
         }
         if (items.size() >= (size_t(1) << (31 - negf::kModeBits))) return fail(NEGF_ERR_ARG, "too many energy points");
         if (!rho0_pass) set = t.ring_set;
-        if (int rc = upload_chain_set(items, codes, s, &set)) return rc;
+        if (int rc = upload_chain_set(items, codes, &set)) return rc;
         if (!rho0_pass) {
             t.ring_set = set;
             t.ring_version = t.version;
@@ -2758,7 +2823,6 @@ int ring_modes_charge(negf_tube& t, Workspace& W, bool rho0_pass, double* d_out,
     NEGF_CUDA(W.tm.reserve(std::max<long long>(1, sp.tm_doubles) * sizeof(double)));
     NEGF_CUDA(launch_fp64(sp, W.groups, W.ck, W.cc, W.tm, W.partial.as<double>(), nullptr, s, nullptr));
     NEGF_CUDA(negf::launch_reduce(rs, 1, t.N, W.partial.as<double>(), d_out, s));
-    // the host lists of a new set are free once the stream has read them (upload_chain_set waits for that)
     NEGF_CUDA(cudaEventRecord(W.done, s));
     W.used = true;
     return NEGF_OK;
