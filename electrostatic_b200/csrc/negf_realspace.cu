@@ -601,6 +601,28 @@ __device__ __forceinline__ bool invert_sym(cplxd (&a)[RowLay<m>::H], cplxd* buf,
     return !__any_sync(0xffffffffu, bad && r < m);
 }
 
+// S^-1 of a complex symmetric matrix in the row layout, build() forming a = -S: by
+// invert_sym, or, after a large multiplier, with partial pivoting (a second
+// build(), in `tile`; col_buf: pivot column).  Returns false on a zero pivot.
+template <int m, class F>
+__device__ __forceinline__ bool invert_rows(cplxd (&a)[RowLay<m>::H], F&& build, Mat<m, double> tile, cplxd* sym_buf,
+                                            cplxd* col_buf, int lane) {
+    build();
+    if (invert_sym<m>(a, sym_buf, lane)) return true;
+    const int r = lane >> 1, h = lane & 1;
+    build();
+#pragma unroll
+    for (int j = 0; j < RowLay<m>::H; ++j)
+        if (r < m && RowLay<m>::col(h, j) < m) tile.at(r, RowLay<m>::col(h, j)) = a[j];
+    __syncwarp();
+    const bool ok = invert_pivoted<m, double>(tile, tile, col_buf, lane);
+#pragma unroll
+    for (int j = 0; j < RowLay<m>::H; ++j)
+        a[j] = cscale(tile.at(min(r, m - 1), min(RowLay<m>::col(h, j), m - 1)), -1.0);
+    __syncwarp();  // every lane has read the tile
+    return ok;
+}
+
 // Asynchronous global -> shared copy of one complex value (cp.async, 8 or 16
 // bytes, both addresses aligned to the size) and the wait for all of them.
 template <typename T>
@@ -922,8 +944,8 @@ __host__ __device__ constexpr int pair_complex() {
 // circulants, so both sides run the same code; only the potentials' addresses,
 // the rows and the contacts' roles differ.  Each side
 //   sweeps forward over its KS blocks (X_k kept in myX),
-//   takes the other side's end corner g[b][b], reflected, as its right lead:
-//     G' = G_K[a][a] = (I - gamma^2 s g_L[b][b])^-1 s of the other side's last ring,
+//   takes the other side's end corner s = g[b][b], reflected, as its right lead:
+//     G' = G_K[a][a] = (s^-1 - gamma^2 g_L[b][b])^-1 of the other side's last ring,
 //   and runs the backward recursion over its blocks, with V = X Y, Y = C D^-1:
 //     M = V G'                            gamma^2 M = G_{k,k+1}[a][a]
 //     G_kk[a][a] = X + gamma^4 M V^T      (symmetric: three of four tiles)
@@ -943,8 +965,11 @@ __host__ __device__ constexpr int pair_complex() {
 // the other one (T_k):
 //   forward   P_k = gamma X_k Q_{k-1}, Q_k = gamma Y^T P_k, Q_{-1} = L / gamma
 //             (Q_k = g_L[k]_{b_k, a_0} L; P_k kept in myP);
-//   middle    S_K = gamma G' Q_{KS-1}; T_K = (I + gamma^2 G' g_L[b][b]) Q', Q' the
-//             other side's last Q, reflected;
+//   middle    S_K = gamma G' Q_{KS-1}; T_K = G' s^-1 Q', Q' the other side's last Q,
+//             reflected (not (I + gamma^2 G' g_L[b][b]) Q': where E passes the potential
+//             of whole rings, s and g_L[b][b] are as large as 1 / Im E in some modes and
+//             G' = -1 / (gamma^2 g_L[b][b]) there to the last digit; a (13,0) tube of 10
+//             blocks at that energy and Im E = 1e-8 came out 1e9 times too large);
 //   backward  S_k = P_k + gamma^2 V S_{k+1}, T_k = gamma^2 V T_{k+1}, and on ring b
 //             the rows of (E - H) G = 1: D^-1 gamma (C^T S_k + S_{k+1}), the same for T.
 // Three products per block; no G_jj sums (the real-axis energies carry no
@@ -982,6 +1007,7 @@ __device__ __forceinline__ bool rs_side(int side, int K, int KS, double gamma, c
     // are clamped, so that no load is conditional and the loads of a pass overlap.
     const int rr = min(lane >> 1, m - 1), hr = lane & 1;
     const bool rv = (lane >> 1) < m;
+    auto col = [&](int j) { return min(RowLay<m>::col(hr, j), m - 1); };
     const int pc = min(lane & 15, m - 1), pr = (lane >> 4) * H;
     const bool pv = (lane & 15) < m;
     // potentials of atom rr (of the reflected ring on side 1) on rings a and b of the next block
@@ -1027,7 +1053,6 @@ __device__ __forceinline__ bool rs_side(int side, int K, int KS, double gamma, c
         // -S, S = diag(E - U_a) - gamma^2 g_L[b][b]_{k-1} - gamma^2 C D^-1 C^T, in the row layout straight
         // from X_{k-1} (the lead's corner at k = 0): no pass over a tile between two inversions
         C a[HR];
-        auto col = [&](int j) { return min(RowLay<m>::col(hr, j), m - 1); };
         auto build = [&]() {
             const int r0 = wrap<m>(rr - 1), r1 = wrap<m>(rr + 1);
             const C lo = cscale(db, g2), hi = cscale(dv[r1], g2);
@@ -1059,18 +1084,7 @@ __device__ __forceinline__ bool rs_side(int side, int K, int KS, double gamma, c
                 if (r1 == c) a[j] = cadd(a[j], hi);   // column r + 1
             }
         };
-        build();
-        if (!invert_sym<m>(a, inv_buf, lane)) {
-            // a large multiplier: -S again as a tile (in V, free here), inverted with partial pivoting
-            build();
-#pragma unroll
-            for (int j = 0; j < HR; ++j)
-                if (rv && RowLay<m>::col(hr, j) < m) V.at(rr, RowLay<m>::col(hr, j)) = a[j];
-            __syncwarp();
-            ok = invert_pivoted<m, double>(V, V, buf, lane) && ok;
-#pragma unroll
-            for (int j = 0; j < HR; ++j) a[j] = cscale(V.at(rr, col(j)), -1.0);
-        }
+        ok = invert_rows<m>(a, build, V, inv_buf, buf, lane) && ok;
         __syncwarp();  // every lane is done with X_{k-1} and dp
         C* dst = myX + (size_t)k * mm2;
 #pragma unroll
@@ -1121,11 +1135,12 @@ __device__ __forceinline__ bool rs_side(int side, int K, int KS, double gamma, c
         if constexpr (NEQ) T.a[i] = other[4 * mm2 + r1 * m + c];
     }
     __syncthreads();  // both have read: B and Q may change
-    // G_K[a][a] of the other side's last ring: (I - gamma^2 s g_L[b][b])^-1 s
-    mm<m, false, false, false>(Gn, X, B, Gn, -g2, lane);
-    if (lane < m) Gn.at(lane, lane) = cadd(Gn.at(lane, lane), cmk(1.0, 0.0));
+    // s^-1 in place of s, then G' = (s^-1 - gamma^2 g_L[b][b])^-1: on checked pivots, as s can be as near to
+    // singular as Im E (invert_sym's multipliers of up to 256 cost the charge 1e-7 at Im E = 1e-8)
+    ok = invert<m>(X, X, buf, lane) && ok;
+    if constexpr (NEQ) mm<m, false, false, false>(P, X, T, P, 1.0, lane);  // s^-1 Q'
+    for (int i = lane; i < mm2; i += 32) Gn.a[i] = csub(X.a[i], cscale(B.a[i], g2));
     ok = invert<m>(Gn, Gn, buf, lane) && ok;
-    mm<m, false, false, false>(Gn, Gn, X, Gn, 1.0, lane);
     fetch_u(KS - 1);
     if constexpr (!NEQ) {
         // X_{k-1} is copied into the other of two tiles while step k runs
@@ -1206,8 +1221,7 @@ __device__ __forceinline__ bool rs_side(int side, int K, int KS, double gamma, c
     } else {
         // S_K and T_K; then S and T alternate between two tiles each
         Tile Sc = Q, So = B, Tc = T, To = Gn;
-        mm<m, false, false, false>(V, B, T, V, 1.0, lane);
-        mm<m, false, false, true>(T, Gn, V, T, g2, lane);
+        mm<m, false, false, false>(T, Gn, P, T, 1.0, lane);
         mm<m, false, false, false>(Q, Gn, Q, Q, gamma, lane);
         auto fetch = [&](Tile to, const C* src) {
             for (int i = lane; i < mm2; i += 32) cp_async(to.a + i, src + i);
