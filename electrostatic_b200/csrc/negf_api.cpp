@@ -2617,7 +2617,7 @@ int negf_broyden_input_device_ptr(negf_broyden* b, double** p) {
 }
 
 int negf_device_selftest(int which, int n, const double* in, double* out) {
-    if (!in || !out || n <= 0 || which < 0 || which > 5) return fail(NEGF_ERR_ARG, "bad self-test arguments");
+    if (!in || !out || n <= 0 || which < 0 || which > 6) return fail(NEGF_ERR_ARG, "bad self-test arguments");
     int rc = require_device();
     if (rc) return rc;
     DevBuf a, b;
@@ -2629,8 +2629,10 @@ int negf_device_selftest(int which, int n, const double* in, double* out) {
     } else {
         // in = [m, count, matrices...]; out = [m, count, results...]
         const int m = (int)in[0], count = (int)in[1];
-        const long long per = (long long)(which >= 4 ? 4 : 2) * m * m;
-        if (m != 4 && m != 13 && m != 16) return fail(NEGF_ERR_ARG, "self-test tiles: m must be 4, 13 or 16");
+        const long long per = (long long)(which == 4 || which == 5 ? 4 : 2) * m * m;
+        if (which == 6 ? m < 1 || m > 16 : m != 4 && m != 13 && m != 16)
+            return fail(NEGF_ERR_ARG, which == 6 ? "self-test tiles: m must be 1 to 16"
+                                                 : "self-test tiles: m must be 4, 13 or 16");
         if (count < 1 || 2 + per * count > n || 2 + 2LL * m * m * count > n)
             return fail(NEGF_ERR_ARG, "self-test tiles: n too small for count matrices");
         NEGF_CUDA(cudaMemset(b.p, 0, sizeof(double) * n));

@@ -1328,11 +1328,12 @@ __global__ void __launch_bounds__(64, 4) rs_pair_kernel(int K, double gamma, con
     if (!ok && lane == 0) atomicExch(status, 1);
 }
 
-// Self-test of the tile primitives: warp w takes matrix w (inversion) or the
-// pair (A, B) w (product) from in (complex, re/im interleaved, row-major
-// m x m, FP64), computes in precision R and writes the m x m result to out.
+// Self-test of the tile primitives: warp w takes matrix w (inversion: mode 0;
+// symmetric, as the FP64 chains do: mode 2) or the pair (A, B) w (product: mode 1)
+// from in (complex, re/im interleaved, row-major m x m, FP64), computes in
+// precision R and writes the m x m result to out.
 template <int m, typename R>
-__global__ void __launch_bounds__(32) rs_selftest_kernel(int product, int count, const double* __restrict__ in,
+__global__ void __launch_bounds__(32) rs_selftest_kernel(int mode, int count, const double* __restrict__ in,
                                                          double* __restrict__ out) {
     __shared__ __align__(16) cplx<R> sh[3 * m * m + kMaxM + 2];
     const int lane = threadIdx.x, w = blockIdx.x;
@@ -1340,6 +1341,7 @@ __global__ void __launch_bounds__(32) rs_selftest_kernel(int product, int count,
     constexpr int mm2 = m * m;
     cplx<R>* buf = sh;
     const Mat<m, R> A{sh + kMaxM + 2}, B{A.a + mm2}, C{B.a + mm2};
+    const bool product = mode == 1;
     const double* src = in + (size_t)w * (product ? 2 : 1) * 2 * mm2;
     for (int i = lane; i < mm2; i += 32) {
         A.a[i] = cmk((R)src[2 * i], (R)src[2 * i + 1]);
@@ -1349,8 +1351,26 @@ __global__ void __launch_bounds__(32) rs_selftest_kernel(int product, int count,
     bool ok = true;
     if (product)
         mm<m, false, false, false>(C, A, B, C, R(1), lane);
-    else
+    else if (mode == 0)
         ok = invert<m>(C, A, buf, lane);
+    else if constexpr (sizeof(R) == 8) {
+        __shared__ cplxd sym_buf[RowLay<m>::kBuf];
+        constexpr int H = RowLay<m>::H;
+        const int r = lane >> 1, h = lane & 1;
+        cplxd a[H];
+        auto col = [&](int j) { return min(RowLay<m>::col(h, j), m - 1); };
+        ok = invert_rows<m>(
+            a,
+            [&]() {
+#pragma unroll
+                for (int j = 0; j < H; ++j) a[j] = cscale(A.at(min(r, m - 1), col(j)), -1.0);
+            },
+            B, sym_buf, buf, lane);
+#pragma unroll
+        for (int j = 0; j < H; ++j)
+            if (r < m && RowLay<m>::col(h, j) < m) C.at(r, RowLay<m>::col(h, j)) = a[j];
+        __syncwarp();
+    }
     double* dst = out + (size_t)w * 2 * mm2;
     for (int i = lane; i < mm2; i += 32) {
         dst[2 * i] = ok ? (double)C.a[i].x : NAN;
@@ -1412,7 +1432,7 @@ int rs_max_atoms_per_block() { return 2 * kMaxM; }
 
 cudaError_t rs_selftest(int which, int m, int count, const double* d_in, double* d_out, cudaStream_t stream) {
     if (count <= 0) return cudaSuccess;
-    const int product = which >= 4;
+    const int product = which == 6 ? 2 : which >= 4;  // the kernel's mode
     const bool fp32 = which == 3 || which == 5;
 #define RS_ST(M)                                                                                                   \
     case M:                                                                                                        \
@@ -1422,7 +1442,8 @@ cudaError_t rs_selftest(int which, int m, int count, const double* d_in, double*
             rs_selftest_kernel<M, double><<<count, 32, 0, stream>>>(product, count, d_in, d_out);                  \
         break;
     switch (m) {
-        RS_ST(4) RS_ST(13) RS_ST(16)
+        RS_ST(1) RS_ST(2) RS_ST(3) RS_ST(4) RS_ST(5) RS_ST(6) RS_ST(7) RS_ST(8)
+        RS_ST(9) RS_ST(10) RS_ST(11) RS_ST(12) RS_ST(13) RS_ST(14) RS_ST(15) RS_ST(16)
         default:
             return cudaErrorInvalidValue;
     }

@@ -508,7 +508,8 @@ int negf_broyden_input_device_ptr(negf_broyden* b, double** d_n_in);
  * 13 or 16; in = [m, count, data], out = [m, count, results], complex values
  * re/im interleaved, row-major): 2 / 3 inverse in FP64 / FP32 (data: count
  * matrices; a NaN result marks a zero pivot), 4 / 5 product A B on the FP64
- * cores / FP32 tensor cores (data: count pairs A, B). */
+ * cores / FP32 tensor cores (data: count pairs A, B), 6 inverse of complex
+ * symmetric matrices in FP64, as the chains form it (any m from 1 to 16). */
 int negf_device_selftest(int which, int n, const double* in, double* out);
 
 /* Affine electrostatics stand-in used by the SCF harness:
