@@ -236,9 +236,12 @@ __global__ void step_kernel(BroydenDev b, double max_norm, double switch_norm, i
 // finish, dots, row, dots, input, step) are bound by their launches and by chains
 // of one block each; a cluster moves V and W at 8 SMs' rate.  us a step, general /
 // here, at 30 rows: 2800 sites 35 / 13, 16384 sites 63 / 25, 65536 sites 163 / 74;
-// at 60 rows 38 / 15, 69 / 36, 172 / 171: the line kMixSites keeps the general
-// path where a long history (200 rows) makes it the faster one.
+// at 60 rows 38 / 15, 69 / 36, 172 / 171; 12000 sites at 100, 200 and 500 rows 66 /
+// 49, 78 / 80, 149 / 287, 4000 sites at 500 and 1000 rows 102 / 82, 166 / 177: the
+// general path beyond kMixSites sites or kMixWork sites x rows, which a long history
+// reaches.
 constexpr int kMixBlocks = 8, kMixThreads = 512, kMixSites = 16384;
+constexpr long long kMixWork = 200LL * kMixSites;
 namespace cg = cooperative_groups;
 __global__ void __cluster_dims__(kMixBlocks, 1, 1) __launch_bounds__(kMixThreads)
     mix_kernel(BroydenDev b, const double* __restrict__ n_out, double max_norm, double switch_norm, int* flags,
@@ -471,12 +474,13 @@ cudaError_t affine_toeplitz(const double* tab, int ntab, const int* idx, const d
 }
 
 namespace {
-// One cluster while it is the faster form (see mix_kernel) and the rows' sums fit its shared memory.
+// One cluster while it is the faster form (see mix_kernel) and the rows' sums fit its shared memory; rows: the
+// most that the launch may find.
 constexpr int kMixShared = 200 * 1024;
-bool mix_fits(const BroydenDev& b, int& chunk, size_t& smem) {
+bool mix_fits(const BroydenDev& b, int rows, int& chunk, size_t& smem) {
     chunk = (b.S + kMixBlocks - 1) / kMixBlocks;
     smem = sizeof(double) * (2 * (4 + 2 * (size_t)b.max_step) + 2 * (size_t)chunk);
-    return b.nseg == 1 && b.S <= kMixSites && smem <= kMixShared;
+    return b.nseg == 1 && b.S <= kMixSites && (long long)b.S * rows <= kMixWork && smem <= kMixShared;
 }
 cudaError_t mix(const BroydenDev& b, const double* n_out, double max_norm, double switch_norm, int* flags, int m_host,
                 int chunk, size_t smem, cudaStream_t s) {
@@ -495,7 +499,7 @@ void norm(const BroydenDev& b, const double* n_out, const int* flags, cudaStream
 cudaError_t broyden_step(const BroydenDev& b, const double* n_out, int m, cudaStream_t s) {
     int chunk;
     size_t smem;
-    if (mix_fits(b, chunk, smem)) return mix(b, n_out, 0.0, 0.0, nullptr, m, chunk, smem, s);
+    if (mix_fits(b, b.base + m, chunk, smem)) return mix(b, n_out, 0.0, 0.0, nullptr, m, chunk, smem, s);
     norm(b, n_out, nullptr, s);
     if (m > 0) {
         if (b.base + m - 1 >= 1) dots_kernel<<<dim3(b.base + m - 1, b.nseg), kThreads, 0, s>>>(b, b.dF, m, 0, nullptr);
@@ -511,7 +515,7 @@ cudaError_t broyden_step_device(const BroydenDev& b, const double* n_out, double
                                 cudaStream_t s) {
     int chunk;
     size_t smem;
-    if (mix_fits(b, chunk, smem)) return mix(b, n_out, max_norm, switch_norm, flags, 0, chunk, smem, s);
+    if (mix_fits(b, b.max_step, chunk, smem)) return mix(b, n_out, max_norm, switch_norm, flags, 0, chunk, smem, s);
     norm(b, n_out, flags, s);
     // shapes cover every m up to max_step, rows above m return
     const dim3 g(b.max_step > 1 ? b.max_step : 1, b.nseg);
