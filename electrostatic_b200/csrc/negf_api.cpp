@@ -947,7 +947,7 @@ double fused_us(const FormLoad& l) {
     const double waves = l.W / (8 * device_sm_count()), part = waves - std::floor(waves);
     if (waves <= 0.5) return alone + 0.5e-6 * l.SC;
     const double mean = l.SC / l.C, tail = part > 0 ? 0.5 + 0.5 * part : 0.0;
-    return std::max(waves > 1.0 ? 15.0 + 0.095 * l.max_N : alone + 2.5 + 0.044 * mean,
+    return std::max(waves > 1.0 ? 15.0 + 0.095 * l.max_N : alone + 2.5 + 0.05 * mean,
                     11.0 + (std::floor(waves) + tail) * (5.0 + 0.107 * mean));
 }
 
@@ -965,7 +965,8 @@ enum class Form { kGroups, kWarps, kFused };
 // same in both forms (two-pass below 4 warps per SM, else fused): groups beside
 // them, sharing the GPU, or all chains in the warp tables (half FP32, groups /
 // warp tables: 160 sites and 4096 chains 38 / 35 us, 1024 sites 94 / 89 and 12000
-// chains 106 / 134, 4000 sites and 4096 chains 153 / 205).
+// chains 106 / 134, 4000 sites and 4096 chains 153 / 205 and, a quarter FP32, 33000
+// chains 421 / 471).
 Form choose_form(negf_tube* const* tubes, int num_tubes, bool fp64_all) {
     const Settings& G = settings();
     if (G.schedule == NEGF_SCHEDULE_FUSED) return Form::kWarps;
@@ -1000,7 +1001,7 @@ Form choose_form(negf_tube* const* tubes, int num_tubes, bool fp64_all) {
     } else {
         low = fused_us(f32);
         warps = fused_us(all);
-        share = 0.5;
+        share = 0.4;
     }
     return std::max(groups, low) + share * std::min(groups, low) < warps ? Form::kGroups : Form::kWarps;
 }
