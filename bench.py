@@ -438,10 +438,9 @@ def config3_measure(torch, passes=2, small=False):
     E = len(t.energy_points(1)[0]) + len(t.energy_points(2)[0])
     E0 = len(t.energy_points(0)[0])
     K, m = t.num_field_sites // 2, 13
-    # ring-corner algorithm: one m x m inverse (8m^3) and three m x m complex
-    # products (8m^3 each) per block update; the lead decimation (stopped at
-    # convergence, data-dependent) is not counted
-    flops = E * K * 32 * m ** 3  # timed passes: the tube's Rho0 comes from the warm-up call
+    # ring-corner algorithm: one m x m inverse (8m^3) and two m x m complex
+    # products (8m^3 each) per block update; the leads are not counted
+    flops = E * K * 24 * m ** 3  # timed passes: the tube's Rho0 comes from the warm-up call
     Qr = Q.cpu().numpy()
     return {"workload": "(13,0) CNT, %d blocks of 2 rings (26 atoms), %d contour+pole energies per pass (the "
                         "%d-energy Rho0 pass at U = 0 runs once per tube, in the warm-up call, as the mode-space "
@@ -450,15 +449,15 @@ def config3_measure(torch, passes=2, small=False):
                         "seeded config-2 ring potential" % (K, E, E0),
             "seconds_per_pass": sec, "block_updates_per_s": E * K / sec,
             "achieved_tflops": flops / sec / 1e12, "flops_per_pass": flops,
-            "flop_convention": "ring corners m=13: inverse 8m^3 + three complex products 8m^3 per block update "
+            "flop_convention": "ring corners m=13: inverse 8m^3 + two complex products 8m^3 per block update "
                                "(leads not counted)",
             "dense_convention": {"flops_per_pass": E * K * 56 * (2 * m) ** 3,
                                  "effective_tflops": E * K * 56 * (2 * m) ** 3 / sec / 1e12,
                                  "note": "the dense 2m x 2m block algorithm's count (56 n^3 per block update, n = 26: "
                                          "forward inverse + 2 GEMM, backward the same, G_nn inverse), which the "
-                                         "ring-corner algebra replaces with 1/14 of the operations (32 m^3 per update)"},
-            "path": "negf_rs_compute_charge with per-atom potentials (FP64, one warp per energy, Schur complements "
-                    "on ring corners)",
+                                         "ring-corner algebra replaces with 1/19 of the operations (24 m^3 per update)"},
+            "path": "negf_rs_compute_charge with per-atom potentials (FP64, two warps per energy from the tube's "
+                    "ends, Schur complements on ring corners)",
             "ring_uniform": {"seconds_per_pass": sec_uniform,
                              "path": "the same call without per-atom potentials: the ring's Fourier modes decouple "
                                      "the blocks exactly (FP64)",
@@ -946,7 +945,7 @@ def main():
     k_ms = float(np.mean(rgf_ms))
     achieved_tf = flops / (k_ms * 1e-3) / 1e12
     peak_tf = measured_fp64_peak(torch) if rank == 0 else None
-    prof = load_profile_traffic("rgf_kernel_config2_ncu.json") or {}
+    prof = load_profile_traffic("fp64_config2_pass_ncu.json") or {}
     peaks = json.load(open(os.path.join(ROOT, "MEASURED_PEAKS.json"))) if os.path.exists(
         os.path.join(ROOT, "MEASURED_PEAKS.json")) else {}
     hbm_peak = peaks.get("hbm_gbs", 6650.0)

@@ -756,7 +756,7 @@ __host__ __device__ constexpr int chain_complex() {
 // every other pair of waves of 148 blocks swaps the roles, so that the inverting
 // warps, with twice the work, do not share two schedulers.  Charge of a 57-cell
 // (13,0) tube, us, one warp per energy / here: 526 FP32 energies 1200 / 653, with
-// 128 real-axis points 1428 / 1054; 2062 with 512: 2302 / 2433 (start 3900).  The
+// 128 real-axis points 1428 / 1045; 2062 with 512: 2302 / 2391 (start 3900).  The
 // arithmetic of every FP32 value is that of the one-warp form.
 constexpr int kFlip = 2 * 148;
 template <int m>
@@ -979,13 +979,13 @@ __host__ __device__ constexpr int pair_complex() {
 // (8000 cycles at m = 13: inversion 2640, products 2000, passes over tiles the
 // rest), by FP64 issue and shared memory beyond.  Charge of a 75-cell tube, us,
 // with one warp per energy, three products and single pivots / here:
-//   m = 13, 64 + 64 + 128 contour points   1428 / 379
-//   m = 13, 128 + 128 + 256                1524 / 549
-//   m = 13, 512 + 512 + 1024               3365 / 1850
-//   m = 16, 128 + 128 + 256                1905 / 770
-//   m = 7,  128 + 128 + 256                 600 / 277
-//   m = 13, 64 real-axis points            3535 / 771
-//   m = 13, 2048 real-axis points          7920 / 2815
+//   m = 13, 64 + 64 + 128 contour points   1425 / 377
+//   m = 13, 128 + 128 + 256                1514 / 548
+//   m = 13, 512 + 512 + 1024               3366 / 1826
+//   m = 16, 128 + 128 + 256                1912 / 759
+//   m = 7,  128 + 128 + 256                 600 / 272
+//   m = 13, 64 real-axis points            3529 / 758
+//   m = 13, 2048 real-axis points          7920 / 2774
 template <int m, bool NEQ>
 __device__ __forceinline__ bool rs_side(int side, int K, int KS, double gamma, cplxd E, cplxd cc,
                                         const double* __restrict__ Ua, const cplxd* __restrict__ sL,

@@ -907,9 +907,9 @@ __device__ __forceinline__ void seg_loop(const GroupDev& g, SegStage* __restrict
 // steps, 7 for the real axis or 2 for the contour, 1 per site of the segment's
 // D and weights).  168 registers hold the half states and the site sums; the
 // potentials sit in shared memory (in registers they spill: 218 us against
-// 196 us).  4000 sites, 33 488 chains: 196 us, 0.66 of the pipe; the sweeps
-// 195 us, 0.60 of the pipe (14 warps per SM; 0.67 at full occupancy).  The
-// fused schedule's single kernel took 467 us for the same pass.
+// 196 us).  4000 sites, 33 488 chains: 197 us, 0.63 of the pipe; the sweeps
+// 202 us, 0.57 of the pipe (14 warps per SM).  The fused schedule's single
+// kernel took 467 us for the same pass.
 template <int K>
 __global__ void __launch_bounds__(32, 11) seg_kernel(const __grid_constant__ GroupSet gs,
                                                      const double* __restrict__ ck, const double* __restrict__ cc,

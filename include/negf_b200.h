@@ -187,7 +187,8 @@ int negf_compute_charge_noalloc(negf_tube* const* tubes, int num_tubes, double* 
  * the scratch belongs to the (device, stream) pair, not to a tube, is kept
  * between calls (a self-consistent loop reuses it every iteration), and this
  * call hands it back, e.g. before destroying `stream` or after the last
- * solve of a sweep.  A stream with no scratch is a no-op.
+ * solve of a sweep.  A stream with no scratch is a no-op.  Replaced chain
+ * lists that wait to be freed (16 MB at most) go too, on every device.
  * It waits on the host, so it is not for a stream that is being captured.
  * Charge plans and the allocation-free entry point are not affected. */
 int negf_release_scratch(void* stream);
