@@ -190,35 +190,41 @@ __device__ __forceinline__ double pow2d(int e) { return __longlong_as_double((lo
 __device__ __forceinline__ double inv_root2(double x) {
     return __hiloint2double((int)((0xbfd00000u - (unsigned)__double2hiint(x)) >> 1 & 0x7ff00000u), 0);
 }
-__device__ __forceinline__ void tm_normalise(Tm& m) {
+// Returns the exponent taken out (0: none).
+__device__ __forceinline__ int tm_normalise(Tm& m) {
     const double s = fmax(fmax(fabs(m.A.x) + fabs(m.A.y), fabs(m.B.x) + fabs(m.B.y)),
                           fmax(fabs(m.C.x) + fabs(m.C.y), fabs(m.D.x) + fabs(m.D.y)));
     const int be = (int)((__double_as_longlong(s) >> 52) & 0x7ff);
-    if (be == 0 || be >= 0x7fe) return;  // zero, subnormal, inf or NaN: leave as is
+    if (be == 0 || be >= 0x7fe) return 0;  // zero, subnormal, inf or NaN: leave as is
     const double f = pow2d(1023 - be);
     m.A = cscale(f, m.A);
     m.B = cscale(f, m.B);
     m.C = cscale(f, m.C);
     m.D = cscale(f, m.D);
     m.e += be - 1023;
+    return be - 1023;
 }
-// later o earlier: [[-D2, C2], [-B2, A2]] [[-D1, C1], [-B1, A1]]
-__device__ __forceinline__ Tm tm_mul(const Tm& m2, const Tm& m1) {
+// later o earlier: [[-D2, C2], [-B2, A2]] [[-D1, C1], [-B1, A1]].  drop: the least
+// exponent of a result of normalised operands so far; a small one is what is left
+// of larger terms.
+__device__ __forceinline__ Tm tm_mul(const Tm& m2, const Tm& m1, int& drop) {
     Tm o;
     o.D = cms(m2.C, m1.B, cmul(m2.D, m1.D));
     o.C = cms(m2.C, m1.A, cmul(m2.D, m1.C));
     o.B = cms(m2.A, m1.B, cmul(m2.B, m1.D));
     o.A = cms(m2.A, m1.A, cmul(m2.B, m1.C));
     o.e = m1.e + m2.e;
-    tm_normalise(o);
+    drop = min(drop, tm_normalise(o));
     return o;
 }
 __device__ __forceinline__ Tm tm_identity() { return Tm{{1.0, 0.0}, {0.0, 0.0}, {0.0, 0.0}, {-1.0, 0.0}, 0}; }
 // State (Z, 1) with lambda through m: Z = (-D Z + K1) / (-K2 Z + A), (K1, K2) = (C, B) forward, (B, C) backward
-__device__ __forceinline__ void tm_apply(const Tm& m, bool back, cd& Z, double& lam) {
+__device__ __forceinline__ void tm_apply(const Tm& m, bool back, cd& Z, double& lam, int& drop) {
     const cd k1 = back ? m.B : m.C, k2 = back ? m.C : m.B;
     const cd num = {fma(-m.D.x, Z.x, fma(m.D.y, Z.y, k1.x)), fma(-m.D.x, Z.y, fma(-m.D.y, Z.x, k1.y))};
     const cd den = {fma(-k2.x, Z.x, fma(k2.y, Z.y, m.A.x)), fma(-k2.x, Z.y, fma(-k2.y, Z.x, m.A.y))};
+    auto hi = [](cd z) { return max(__double2hiint(z.x) & 0x7fffffff, __double2hiint(z.y) & 0x7fffffff) >> 20; };
+    drop = min(drop, max(hi(num), hi(den)) - max(hi(Z), 1023));
     const double iq = rcp(fma(den.x, den.x, den.y * den.y));
     Z = {fma(num.x, den.x, num.y * den.y) * iq, fma(num.y, den.x, -num.x * den.y) * iq};
     lam *= iq;
@@ -644,10 +650,63 @@ __device__ __forceinline__ Tm seg_matrix(const double* __restrict__ U, int n0, i
     return m;
 }
 
+// One chain's boundary states by sweeps, for the chains whose scan loses digits:
+// lane 0 forward, lane 1 backward (the same steps), potentials staged by the block.
+// 30 ns a site.
+constexpr int kStage = 256;
+template <int K>
+__device__ __noinline__ void sweep_states(const GroupDev& g, int c, double* __restrict__ ck, const cd* sig, double Eg,
+                                          double ei, double ig, double r, double (*stage)[kStage]) {
+    const bool ra = g.kind == kRealAxis, back = threadIdx.x == 1;
+    const int N = g.N, nseg = g.nseg;
+    Lin s{sig[back].x, sig[back].y, 1.0, 0.0};
+    double mu = 1.0, h = 1.0;  // mu = lambda |q|^2, h: product of rho since the last boundary
+    for (int m0 = 0; m0 < N; m0 += kStage) {
+        const int len = min(kStage, N - m0);
+        __syncthreads();
+        for (int i = threadIdx.x; i < len; i += blockDim.x) {
+            stage[0][i] = g.U[m0 + i];
+            stage[1][i] = g.U[N - 1 - m0 - i];
+        }
+        __syncthreads();
+        if (threadIdx.x > 1) continue;
+        for (int i = 0; i < len; ++i) {
+            const int m = m0 + i, n = back ? N - 1 - m : m;
+            // boundaries: the first site of a segment forward, its last one backward
+            int seg = -1;
+            if (back)
+                seg = n == N - 1 ? nseg - 1 : (n + 1) % K == 0 && n / K < nseg - 1 ? n / K : -1;
+            else
+                seg = n == N - K ? nseg - 1 : n % K == 0 && n < N - K ? n / K : -1;
+            if (seg >= 0) {
+                const double q2 = fma(s.qr, s.qr, s.qi * s.qi), q1 = rcp(q2), f = inv_root2(q2);
+                double* o = ck + (ra ? state_at<6>(g, c, seg) : state_at<4>(g, c, seg)) +
+                            (back ? (ra ? 3 : 2) : 0) * kBlk;
+                mu *= h;
+                h = 1.0;
+                o[0] = fma(s.pr, s.qr, s.pi * s.qi) * q1;
+                o[kBlk] = fma(s.pi, s.qr, -s.pr * s.qi) * q1;
+                if (ra) o[2 * kBlk] = mu * q1;
+                mu = mu * f * f;
+                s = {s.pr * f, s.pi * f, s.qr * f, s.qi * f};
+            }
+            const bool odd = m & 1;
+            lin_step(s, fma(-stage[back][i], ig, Eg), ei, r, odd);
+            if (!odd) h *= r;
+        }
+    }
+}
+
 // One block per chain.  Thread t owns segments [t gper, (t + 1) gper): their
 // matrices (kept in `tm` when gper > 1), their product, an inclusive scan over
 // the warp in both directions by shuffles, the warps' totals through shared
-// memory, then the boundary states of its own segments.
+// memory, then the boundary states of its own segments.  A product of
+// matrices, or one with a state, that comes out small against its factors (2^kDrop:
+// an evanescent wave that decays, a resonance) has lost as many digits; its chain
+// is swept instead, at 30 ns a site.  (Periodic potentials at Im E = 2e-6: charges off
+// by 1e-7 of their largest value without this, by 1e-11 with it.  Chains of the
+// benchmark's potentials come down to 2^-6.)
+constexpr int kDrop = -8;
 template <int K>
 __global__ void __launch_bounds__(kScanMaxThreads) scan_kernel(const __grid_constant__ GroupSet gs,
                                                                double* __restrict__ ck, double* __restrict__ cc,
@@ -656,6 +715,7 @@ __global__ void __launch_bounds__(kScanMaxThreads) scan_kernel(const __grid_cons
     if (skip && *skip) return;
     __shared__ Tm tot[kScanMaxThreads / 32];
     __shared__ cd sh_sig[2];
+    __shared__ double stage[2][kStage];
     const GroupDev& g = group(gs, find_group<&GroupDev::chain_base>(gs, gs.chain_base, blockIdx.x));
     const int c = blockIdx.x - g.chain_base;
     const int t = threadIdx.x, lane = t & 31, wid = t >> 5, W = blockDim.x >> 5;
@@ -673,6 +733,7 @@ __global__ void __launch_bounds__(kScanMaxThreads) scan_kernel(const __grid_cons
     const double* __restrict__ U = g.U;
     const int s0 = min(t * gper, nseg), s1 = min(s0 + gper, nseg);
     double* __restrict__ mine = tm + ((long long)blockIdx.x * g.tm_segs) * 9;
+    int drop = 0;
     Tm own = tm_identity(), first = own;
     for (int s = s0; s < s1; ++s) {
         const Tm m = seg_matrix<K>(U, s * K, min(K, N - s * K), ig, Eg, ei, r, hs);
@@ -683,14 +744,14 @@ __global__ void __launch_bounds__(kScanMaxThreads) scan_kernel(const __grid_cons
         } else {
             first = m;
         }
-        own = s == s0 ? m : tm_mul(m, own);
+        own = s == s0 ? m : tm_mul(m, own, drop);
     }
     Tm pre = own, suf = own;  // inclusive products: pre over lanes <= mine, suf over lanes >= mine
 #pragma unroll
     for (int d = 1; d < 32; d <<= 1) {
         const Tm a = tm_shfl(pre, max(lane - d, 0)), b = tm_shfl(suf, min(lane + d, 31));
-        if (lane >= d) pre = tm_mul(pre, a);
-        if (lane + d < 32) suf = tm_mul(b, suf);
+        if (lane >= d) pre = tm_mul(pre, a, drop);
+        if (lane + d < 32) suf = tm_mul(b, suf, drop);
     }
     if (lane == 31) tot[wid] = pre;
     Tm ex = tm_shfl(pre, max(lane - 1, 0)), sx = tm_shfl(suf, min(lane + 1, 31));
@@ -699,10 +760,10 @@ __global__ void __launch_bounds__(kScanMaxThreads) scan_kernel(const __grid_cons
     __syncthreads();
     cd Y = sh_sig[0], X = sh_sig[1];
     double lam = 1.0, rho = 1.0;
-    for (int w = 0; w < wid; ++w) tm_apply(tot[w], false, Y, lam);
-    for (int w = W - 1; w > wid; --w) tm_apply(tot[w], true, X, rho);
-    tm_apply(ex, false, Y, lam);
-    tm_apply(sx, true, X, rho);
+    for (int w = 0; w < wid; ++w) tm_apply(tot[w], false, Y, lam, drop);
+    for (int w = W - 1; w > wid; --w) tm_apply(tot[w], true, X, rho, drop);
+    tm_apply(ex, false, Y, lam, drop);
+    tm_apply(sx, true, X, rho, drop);
     auto load = [&](int s) {
         if (gper == 1) return first;
         const double* q = mine + s;
@@ -729,12 +790,13 @@ __global__ void __launch_bounds__(kScanMaxThreads) scan_kernel(const __grid_cons
             const double rq = rcp(fma(q.qr, q.qr, q.qi * q.qi));
             put_y(nseg - 1, {fma(q.pr, q.qr, q.pi * q.qi) * rq, fma(q.pi, q.qr, -q.pr * q.qi) * rq}, lam * rp * rq);
         }
-        if (s + 1 < s1) tm_apply(load(s), false, Y, lam);
+        if (s + 1 < s1) tm_apply(load(s), false, Y, lam, drop);
     }
     for (int s = s1 - 1; s >= s0; --s) {
         put(s, ra ? 3 : 2, X, rho);
-        if (s > s0) tm_apply(load(s), true, X, rho);
+        if (s > s0) tm_apply(load(s), true, X, rho, drop);
     }
+    if (__syncthreads_or(drop < kDrop)) sweep_states<K>(g, c, ck, sh_sig, Eg, ei, ig, r, stage);
 }
 
 // ------------------------------------------------------------------ segments
