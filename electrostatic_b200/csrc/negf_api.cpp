@@ -217,6 +217,7 @@ struct ChainTable {
     std::vector<negf::WarpRec> warps;
     std::vector<negf::ReduceTube> rts;
     std::vector<negf::SegUnit> units;
+    std::vector<negf::TubeDev> tdev;  // tubes of the warp tables, as last uploaded
     std::vector<int> order;  // fused schedule: FP64 warps, then FP32 warps
     int n64 = 0, n32 = 0;
     bool fused = false;  // the warps run fused by the estimates (Form::kFused)
@@ -960,8 +961,8 @@ enum class Form { kGroups, kWarps, kFused };
 // along in the launches of the FP32 warps (a 16-tube batch with the real axis
 // in FP32: 2.364 ms so, 2.382 ms with groups).  Counted by energies; the band-edge
 // rule moves single chains only.  Else, unless a setting asks for other schedules,
-// the faster form by the estimates.  FP64 batches: groups or fused; up to 32 sites
-// fused is ahead at every number of chains.  With FP32 warps, whose schedule is the
+// the faster form by the estimates.  FP64 batches: groups or, where it is ahead by
+// more than the estimates' error, fused; below 32 sites at every number of chains.  With FP32 warps, whose schedule is the
 // same in both forms (two-pass below 4 warps per SM, else fused): groups beside
 // them, sharing the GPU, or all chains in the warp tables (half FP32, groups /
 // warp tables: 160 sites and 4096 chains 38 / 35 us, 1024 sites 94 / 89 and 12000
@@ -990,7 +991,7 @@ Form choose_form(negf_tube* const* tubes, int num_tubes, bool fp64_all) {
     if (2 * f32.SC > all.SC) return Form::kWarps;
     if (G.schedule != 0 || G.pass1_pieces != 0) return Form::kGroups;
     const double groups = groups_us(f64);
-    if (f32.C <= 0) return all.max_N <= 32 || fused_us(all) < groups ? Form::kFused : Form::kGroups;
+    if (f32.C <= 0) return all.max_N < 32 || fused_us(all) < 0.95 * groups ? Form::kFused : Form::kGroups;
     double low, warps, share;  // FP32 warps alone, all chains in the tables
     if (all.W < 4 * device_sm_count()) {
         auto latency = [](int N) { return 14.0 + 0.15 * std::min(N, 500); };  // pieces beyond
@@ -1406,9 +1407,12 @@ int upload_and_launch(Workspace& W, const std::vector<TubePass>& passes, const s
     }
     const int nw = (int)ct.warps.size(), nw_all = nw + ct.fp64.warps;
     if (nw > 0) {
-        NEGF_CUDA(W.tubes.reserve(tdev.size() * sizeof(negf::TubeDev)));
-        NEGF_CUDA(cudaMemcpyAsync(W.tubes.p, tdev.data(), tdev.size() * sizeof(negf::TubeDev), cudaMemcpyHostToDevice,
-                                  stream));
+        const size_t bytes = tdev.size() * sizeof(negf::TubeDev);
+        NEGF_CUDA(W.tubes.reserve(bytes));
+        if (rebuild || ct.tdev.size() != tdev.size() || std::memcmp(ct.tdev.data(), tdev.data(), bytes) != 0) {
+            ct.tdev = tdev;
+            NEGF_CUDA(cudaMemcpyAsync(W.tubes.p, ct.tdev.data(), bytes, cudaMemcpyHostToDevice, stream));
+        }
     }
     // potentials and contacts of this call
     for (int k = 0; k < 2; ++k)
